@@ -357,6 +357,7 @@ cudaError_t batched_exclusive_scan_u32(const ScanSeg* segs, const unsigned* tile
                                        cudaStream_t s);
 
 // pcg.cu
+struct PcgPacket;
 struct GridSync {
     unsigned count;  // arrivals at the current barrier (top bit: barriers passed, mod 2)
 };
@@ -371,6 +372,7 @@ struct PcgWork {
     double* part = nullptr;
     float* partMaxF = nullptr;
     double* partMaxD = nullptr;
+    PcgPacket* packets = nullptr;  // partials of the chunk-resident solve
     int4* rec = nullptr;  // packed grid rows
     float4* coefRow = nullptr;  // packed rows' off-diagonal values (2 per row)
     // single-reduction solve: row records {r, w, s, 1/diag} (double-buffered; FP32 as
@@ -386,13 +388,20 @@ struct PcgOutcome {
     double residual = 0;
     float kernelMs = 0.f;  // device time of the persistent launches (all inner solves)
 };
-// gridRows: the x neighbours of every row are rows r-1 / r+1 (or none) and the y
-// neighbours lie within 65535 rows (rows of a grid in cell order, at most 65535 cells
-// along x); the solve then reads the packed 16-byte row records.
+// How a system's rows are numbered.  kRowsGrid: the x neighbours of every row are rows
+// r-1 / r+1 (or none), its y neighbours lie within 65535 rows and on their side, its z
+// neighbours on theirs (rows of a grid in cell order, at most 65535 cells along x); the solve
+// then reads the packed 16-byte row records.  kRowsCompact: also y within kCompactDy rows and
+// z within kCompactDz (the chunk-resident solve's 8-byte records).
+enum RowLayout { kRowsAny, kRowsGrid, kRowsCompact };
+constexpr int kCompactDy = 512, kCompactDz = (1 << 18) - 1;
+inline RowLayout row_layout(long long maxDy, long long maxDz) {
+    return maxDy <= kCompactDy && maxDz <= kCompactDz ? kRowsCompact : kRowsGrid;
+}
 // coef (optional): six planes of off-diagonal values in the order of nbr (face weights
 // != 1); without it every off-diagonal is -dt.
 int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const float* invd, const int32_t* nbr,
-              const float* coef, bool gridRows, float dt, int mode, float tol, unsigned maxIter, float innerTol,
+              const float* coef, RowLayout layout, float dt, int mode, float tol, unsigned maxIter, float innerTol,
               float outerTol, float* pressure, double* x64out, DevState* dst, DevState* hst, cudaStream_t s,
               PcgOutcome& out);
 int pcg_reserve(PcgWork& w, int n, bool fp64);

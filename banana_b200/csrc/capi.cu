@@ -3,6 +3,7 @@
 // FLIP_Solver::advanceVelocity, FLIP_Solver.cpp:42-53).
 #include "bnn_internal.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -305,7 +306,7 @@ static uint64_t device_bytes(const bnn_flip* h) {
     const bool affine = h->P.solver_kind == BNN_SOLVER_APIC || h->P.solver_kind == BNN_SOLVER_AFLIP;
     b += (uint64_t)h->cap * (172u + (affine ? 72u : 0u) + (h->moved ? 12u : 0u));  // particle arrays
     b += (uint64_t)h->rowCap * 44u;                                                // rows
-    b += (uint64_t)h->pcg.cap * (48u + (h->pcg.x64 ? 56u : 0u)) + (uint64_t)h->pcg.nchCap * 40u;
+    b += (uint64_t)h->pcg.cap * (48u + (h->pcg.x64 ? 56u : 0u)) + (uint64_t)h->pcg.nchCap * 296u;
     return b;
 }
 
@@ -682,7 +683,7 @@ static int run_substep(bnn_flip* h, bnn_step_stats* st, const HostIo* io = nullp
     cudaEventRecord(h->ev[6], s);
     PcgOutcome po;
     rc = pcg_solve(h->pcg, (int)nrows, h->rhs, h->diag, h->invd, h->nbr, h->gridBoundary ? h->coef : nullptr,
-                   true, substep, h->P.pcg_mode,
+                   row_layout(g.G[0], (long long)g.G[0] * g.G[1]), substep, h->P.pcg_mode,
                    h->P.cg_relative_tolerance, h->P.max_cg_iteration, h->P.refine_inner_tolerance,
                    h->P.refine_tolerance, h->pressure, nullptr, h->dst, h->hst, s, po);
     if(rc != BNN_OK) return rc;
@@ -955,6 +956,7 @@ extern "C" int bnn_pcg_solve_7pt(uint32_t n, const float* diag, const int32_t* n
     // rows of a grid in cell order (x neighbours r-1 / r+1, y neighbours within 65535 rows,
     // z neighbours on their side) take the packed-record solve
     bool gridRows = true;
+    int64_t maxDy = 0, maxDz = 0;
     for(uint32_t r = 0; r < n; ++r) {
         inv[r] = diag[r] != 0.f ? 1.0f / diag[r] : 0.f;
         for(int q = 0; q < 6; ++q) {
@@ -976,6 +978,10 @@ extern "C" int bnn_pcg_solve_7pt(uint32_t n, const float* diag, const int32_t* n
         if(nb[4] >= 0 && !(nb[4] > R && nb[4] - R <= 65535)) gridRows = false;
         if(nb[0] >= 0 && !(nb[0] < R)) gridRows = false;
         if(nb[5] >= 0 && !(nb[5] > R)) gridRows = false;
+        if(nb[1] >= 0) maxDy = std::max(maxDy, R - nb[1]);
+        if(nb[4] >= 0) maxDy = std::max(maxDy, nb[4] - R);
+        if(nb[0] >= 0) maxDz = std::max(maxDz, R - nb[0]);
+        if(nb[5] >= 0) maxDz = std::max(maxDz, nb[5] - R);
     }
     // the system stores -dt as the off-diagonal; recover dt so the kernels form -(1*dt)
     const float dt = -offdiag;
@@ -996,7 +1002,7 @@ extern "C" int bnn_pcg_solve_7pt(uint32_t n, const float* diag, const int32_t* n
     if(rc == BNN_OK) rc = pcg_reserve(w, (int)n, (mode & BNN_PCG_MODE_MASK) != BNN_PCG_FP32);  // outside the timed region
     if(rc == BNN_OK) {
         cudaEventRecord(e0, s);
-        rc = pcg_solve(w, (int)n, dRhs, dDiag, dInv, dNbr, nullptr, gridRows, dt, mode, tol, max_iter, inner_tol, tol, dP, dX,
+        rc = pcg_solve(w, (int)n, dRhs, dDiag, dInv, dNbr, nullptr, gridRows ? row_layout(maxDy, maxDz) : kRowsAny, dt, mode, tol, max_iter, inner_tol, tol, dP, dX,
                        dst, hst, s, po);
         cudaEventRecord(e1, s);
     }

@@ -575,6 +575,579 @@ __global__ void __launch_bounds__(kLanes, pcg_min_blocks<VT, COEF>()) k_pcg_pers
     }
 }
 
+// The 16-byte record of row r (layout at the top of this file).  The caller guarantees the
+// x neighbours are rows r-1 / r+1 and the y distances fit 16 bits.
+__device__ __forceinline__ int4 pack_row(int r, const int32_t nb[6], float diag) {
+    const unsigned dyM = nb[1] >= 0 ? (unsigned)(r - nb[1]) : 0u, dyP = nb[4] >= 0 ? (unsigned)(nb[4] - r) : 0u;
+    const unsigned dzM = nb[0] >= 0 ? (unsigned)(r - nb[0]) : 0u, dzP = nb[5] >= 0 ? (unsigned)(nb[5] - r) : 0u;
+    int4 v;
+    v.x = (int)(dyM | (dyP << 16));
+    v.y = (int)(dzM | (nb[2] >= 0 ? 0x80000000u : 0u));
+    v.z = (int)(dzP | (nb[3] >= 0 ? 0x80000000u : 0u));
+    v.w = __float_as_int(diag);
+    return v;
+}
+
+// ---------------------------------------------------------------------------------
+// Chunk-resident PCG: the same iteration for systems whose 2048-row chunks are all on the
+// chip at once.  One block per SM, of G groups of 256 threads; a group owns K chunks for the
+// whole solve and keeps what its own rows need on the chip: r and z / q in registers, s and
+// the row records in shared memory.  Only what other blocks read crosses L2 on the critical
+// path: a pair {z, s} per row, written once per iteration (phase B) and read by its z
+// neighbours and across chunk ends (phase A).  One buffer is enough: all reads lie between
+// the second exchange and the next first one, all writes between the first and the second.
+// The x and y neighbours inside a chunk are read from shared memory.
+//
+// The grid barriers are merged with the reductions: a group publishes a chunk's partial sum
+// and max as one 16-byte packet, and every block polls the packets of all chunks and adds them
+// in the canonical order; a block has passed when it has seen all of them.  A packet's max
+// carries the parity of its exchange in the top bit (a block is at most one exchange ahead of
+// the slowest, so one bit tells old from new; the packets start zeroed).  Packets lie 128
+// bytes apart so that the polls of all blocks spread over the L2 slices.  The x update
+// overlaps the second wait.
+//
+// What bounds it: up to a chunk per SM the latency of the two exchanges (about 1.5 us each:
+// the release of the pairs, a packet's way through L2, the FP64 tree) and of one round of
+// neighbour loads; at six chunks per SM the instructions of phase A, the pair stores of phase
+// B and the FP32-to-FP64 conversions of the products (16 a clock and SM).  One block per SM
+// instead of three: one poller per SM, and a group's registers can hold a whole chunk's loads.
+// Measured, us per iteration with everything around it (k_pcg_persistent before): FP32 26,652
+// rows 4.96 (9.41), 161,057 rows 5.51 (9.63), 315,698 6.66 (10.96), 705,846 9.05 (13.81),
+// 1,283,026 14.7 (22.1), 1,736,304 16.9 (22.9); FP64 26,652 rows 5.88 (12.8), 315,698 8.10
+// (15.2), 705,846 14.3 (19.8).
+// ---------------------------------------------------------------------------------
+template<class VT> struct alignas(2 * sizeof(VT)) RowPair {
+    VT z, s;
+};
+template<class VT> __device__ __forceinline__ RowPair<VT> ld_pair(const RowPair<VT>* p) {
+    if constexpr(sizeof(VT) == 4) {
+        const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+        return {v.x, v.y};
+    } else {
+        const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+        return {v.x, v.y};
+    }
+}
+// ld_pair where `on`, zeros elsewhere, as one predicated load (a branch around each of a
+// row's loads costs more than the load)
+template<class VT> __device__ __forceinline__ RowPair<VT> ld_pair_if(const RowPair<VT>* p, bool on) {
+    RowPair<VT> v{VT(0), VT(0)};
+    if constexpr(sizeof(VT) == 4)
+        asm volatile("{ .reg .pred p; setp.ne.s32 p, %3, 0; @p ld.global.cg.v2.f32 {%0, %1}, [%2]; }"
+                     : "+f"(v.z), "+f"(v.s) : "l"(p), "r"((int)on) : "memory");
+    else
+        asm volatile("{ .reg .pred p; setp.ne.s32 p, %3, 0; @p ld.global.cg.v2.f64 {%0, %1}, [%2]; }"
+                     : "+d"(v.z), "+d"(v.s) : "l"(p), "r"((int)on) : "memory");
+    return v;
+}
+// volatile: issued where it stands, ahead of a wait
+__device__ __forceinline__ float ld_const_if(const float* p, bool on) {
+    float v = 0.f;
+    asm volatile("{ .reg .pred p; setp.ne.s32 p, %2, 0; @p ld.global.nc.f32 %0, [%1]; }" : "+f"(v) : "l"(p), "r"((int)on));
+    return v;
+}
+__device__ __forceinline__ double ld_const_if(const double* p, bool on) {
+    double v = 0.0;
+    asm volatile("{ .reg .pred p; setp.ne.s32 p, %2, 0; @p ld.global.nc.f64 %0, [%1]; }" : "+d"(v) : "l"(p), "r"((int)on));
+    return v;
+}
+// A chunk's partial of one exchange: the bits of the FP64 sum, and of the max in its vector
+// type, the exchange's parity in the top bit
+struct alignas(16) PcgPacket {
+    unsigned long long sum, max;
+};
+constexpr int kPacketStride = 8;  // packets apart
+__device__ __forceinline__ unsigned long long max_bits(float m) { return __float_as_uint(m) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned long long max_bits(double m) {
+    return (unsigned long long)__double_as_longlong(m) & 0x7fffffffffffffffull;
+}
+template<class VT> __device__ __forceinline__ VT max_of(unsigned long long b) {
+    if constexpr(sizeof(VT) == 4) return __uint_as_float((unsigned)b);
+    else return __longlong_as_double((long long)(b & 0x7fffffffffffffffull));
+}
+// 16-byte accesses are single (PTX .b128), so a packet is never seen half written
+__device__ __forceinline__ void st_relaxed_packet(PcgPacket* p, PcgPacket v) {
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
+                 : : "l"(p), "l"(v.sum), "l"(v.max) : "memory");
+}
+__device__ __forceinline__ PcgPacket ld_relaxed_packet(const PcgPacket* p) {
+    PcgPacket v;
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(v.sum), "=l"(v.max) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_packet(PcgPacket* p, PcgPacket v) {
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.release.gpu.global.b128 [%0], t; }"
+                 : : "l"(p), "l"(v.sum), "l"(v.max) : "memory");
+}
+__device__ __forceinline__ PcgPacket ld_acquire_packet(const PcgPacket* p) {
+    PcgPacket v;
+    asm volatile("{ .reg .b128 t; ld.acquire.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(v.sum), "=l"(v.max) : "l"(p) : "memory");
+    return v;
+}
+
+struct Yes { static constexpr bool value = true; };
+struct No { static constexpr bool value = false; };
+
+// Barrier over one group of 256 threads (hardware barriers 1 .. G; 0 is the whole block's)
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 256;" : : "r"(g + 1) : "memory"); }
+
+// One warp: sum and max (MAX) of 256 lanes' values in the canonical order (as
+// block_sum_max_256); valid in lane 0
+template<class VT, bool MAX>
+__device__ __forceinline__ void lane_tree(const double* smd, const VT* smv, double& sum, VT& mx) {
+    const int t = threadIdx.x & 31;
+    const double a0 = smd[t] + smd[t + 128];
+    const double a1 = smd[t + 64] + smd[t + 192];
+    const double a2 = smd[t + 32] + smd[t + 160];
+    const double a3 = smd[t + 96] + smd[t + 224];
+    double c = (a0 + a1) + (a2 + a3);
+    VT x = VT(0);
+    if(MAX) {
+        x = smv[t];
+#pragma unroll
+        for(int q = 1; q < 8; ++q) { const VT o = smv[t + 32 * q]; x = x > o ? x : o; }
+    }
+#pragma unroll
+    for(int off = 16; off > 0; off >>= 1) {
+        c = c + __shfl_down_sync(0xffffffffu, c, off);
+        if(MAX) { const VT o = __shfl_down_sync(0xffffffffu, x, off); x = x > o ? x : o; }
+    }
+    sum = c;
+    mx = x;
+}
+
+// One warp: a chunk's sum and max from its 256 lanes' values out to its packet.  RELEASE:
+// everything the group wrote before its last barrier is visible to whoever acquires the packet.
+template<class VT, bool MAX, bool RELEASE>
+__device__ __forceinline__ void packet_publish(const double* smd, const VT* smv, PcgPacket* slot, unsigned parity) {
+    double c;
+    VT x;
+    lane_tree<VT, MAX>(smd, smv, c, x);
+    if((threadIdx.x & 31) == 0) {
+        PcgPacket v;
+        v.sum = (unsigned long long)__double_as_longlong(c);
+        v.max = max_bits(x) | ((unsigned long long)parity << 63);
+        if(RELEASE) st_release_packet(slot, v);
+        else st_relaxed_packet(slot, v);
+    }
+}
+
+// Polls one packet per lane (where `on`) until all of the warp's carry `parity`; false when
+// the bounded wait gave up.
+template<bool ACQUIRE>
+__device__ __forceinline__ bool packet_poll(const PcgPacket* slot, bool on, unsigned parity, PcgPacket& pk) {
+    const BarrierLimit lim = solve_barrier_limit();
+    unsigned spins = 0;
+    unsigned long long t0 = 0;
+    while(true) {
+        if(on) {
+            pk = ACQUIRE ? ld_acquire_packet(slot) : ld_relaxed_packet(slot);
+            on = (unsigned)(pk.max >> 63) != parity;
+        }
+        if(!__any_sync(0xffffffffu, on)) return true;
+        ++spins;
+        if(spins == lim.minSpins) t0 = global_ns();
+        const bool late = spins >= lim.maxSpins ||
+                          (spins > lim.minSpins && (spins & 255u) == 0u && global_ns() - t0 >= lim.ns);
+        if(__any_sync(0xffffffffu, late)) return false;
+    }
+}
+
+// Second half of an exchange: waits for every chunk's packet of this parity and gives the
+// canonical sum and max (as reduce_partials_bcast) to every thread of the block.  Up to 32
+// chunks are polled by warp 0, which then needs no shared memory for their sum; more by all
+// threads, through the W's arrays.  ACQUIRE: what the other blocks released is visible.  False
+// when the bounded wait gave up (the timeout flag is set).
+constexpr int kWarpPackets = 32;
+constexpr int kMostSM = 160;  // SMs a chunk-resident solve is spread over at most
+template<class VT, int CH> struct WaitSmem {
+    double part[CH * kMostSM];  // the chunks' sums and maxima as polled
+    VT partMax[CH * kMostSM];
+    double lanes[kLanes];       // ... of the 256 lanes of the canonical tree
+    VT lanesMax[kLanes];
+    double sum;                 // the result
+    VT max;
+    int bad;                    // a wait gave up
+};
+template<class VT, bool MAX, bool ACQUIRE, int CH>
+__device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
+                                            WaitSmem<VT, CH>& W, double& sum, VT& mx) {
+    const int t = threadIdx.x;
+    if(nch > kWarpPackets) {
+        // whole warps stay in the loop (the poll votes)
+        for(int c = t; c < ((nch + 31) & ~31); c += (int)blockDim.x) {
+            PcgPacket pk;
+            if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad = 1; break; }
+            if(c < nch) {
+                W.part[c] = __longlong_as_double((long long)pk.sum);
+                if(MAX) W.partMax[c] = max_of<VT>(pk.max);
+            }
+        }
+        __syncthreads();
+        if(t < kLanes) {
+            double acc = 0.0;
+            VT m = VT(0);
+            for(int c = t; c < nch; c += kLanes) {
+                acc = acc + W.part[c];
+                if(MAX) { const VT o = W.partMax[c]; m = m > o ? m : o; }
+            }
+            W.lanes[t] = acc;
+            if(MAX) W.lanesMax[t] = m;
+            group_sync(0);
+        }
+        if(t < 32) {
+            double c;
+            VT x;
+            lane_tree<VT, MAX>(W.lanes, W.lanesMax, c, x);
+            if(t == 0) { W.sum = c; W.max = x; }
+        }
+    } else if(t < 32) {
+        PcgPacket pk;
+        if(!packet_poll<ACQUIRE>(slots + (size_t)t * kPacketStride, t < nch, parity, pk)) W.bad = 1;
+        double c = 0.0;
+        VT m = VT(0);
+        if(t < nch) {
+            c = c + __longlong_as_double((long long)pk.sum);
+            if(MAX) { const VT o = max_of<VT>(pk.max); m = m > o ? m : o; }
+        }
+#pragma unroll
+        for(int off = 16; off > 0; off >>= 1) {
+            if(off >= nch) continue;  // the tree's other half holds no chunk: +0
+            c = c + __shfl_down_sync(0xffffffffu, c, off);
+            if(MAX) { const VT o = __shfl_down_sync(0xffffffffu, m, off); m = m > o ? m : o; }
+        }
+        if(t == 0) { W.sum = c; W.max = m; }
+    }
+    __syncthreads();
+    sum = W.sum;
+    mx = W.max;
+    if(W.bad == 0) return true;
+    if(t == 0) atomicOr(flags, BNN_FLAG_TIMEOUT);
+    return false;
+}
+
+template<class VT> struct ChunkArgs {
+    int n;
+    int nch;
+    const float* rhsF;
+    const float* diag;
+    const VT* invd;
+    const int32_t* nbr;
+    const float* coef;  // off-diagonal planes (COEF)
+    VT negoff;
+    VT tolFactor;
+    unsigned maxIter;
+    VT* x;
+    RowPair<VT>* pair;
+    PcgPacket *pkA, *pkB;  // nch packets each, zeroed
+    DevState* st;
+};
+// A row's neighbours in 8 bytes: .x = dz- | y- << 18 | (has -x) << 31, .y = dz+ | y+ << 18 |
+// (has +x) << 31.  dz is a row distance (0 = none); y is the neighbour's place in the chunk,
+// kNoRow for none, kNoRow + 1 + its distance when it lies in another chunk.  Grids of up to
+// kCompactDy cells along x and kCompactDz cells per z plane fit (kRowsCompact).  With y
+// neighbours within two of the chunk's eight 256-row strips, only its first and last two
+// strips reach across its ends.
+constexpr unsigned kNoRow = kChunk;
+static_assert(kCompactDy <= 2 * kLanes && kNoRow + 1 + kCompactDy < (1 << 12) && kCompactDz < (1 << 18),
+              "the records' fields");
+__device__ __forceinline__ unsigned row_code(int dz, int l, int dy, int sign, bool x) {
+    const int to = l + sign * dy;
+    const unsigned y = dy == 0 ? kNoRow : ((unsigned)to < (unsigned)kChunk ? (unsigned)to : kNoRow + 1u + (unsigned)dy);
+    return (unsigned)dz | y << 18 | (x ? 0x80000000u : 0u);
+}
+// Shared memory of a block: CH chunks.  x and 1/diag are kept there too where they fit (else
+// x stays in global memory and 1/diag is loaded ahead of every iteration's first exchange).
+template<class VT> constexpr int kRoomy = sizeof(VT) == 4 ? 3 : 2;
+template<class VT, bool COEF, int CH> struct ChunkSmem {
+    static constexpr int kX = CH <= kRoomy<VT> ? CH : 1, kXRows = CH <= kRoomy<VT> ? kChunk : 1;
+    VT s[CH][kChunk + 16 / sizeof(VT)];  // s[kNoRow] = 0: what a missing neighbour adds
+    uint2 nb[CH][kChunk];
+    float diag[CH][kChunk];
+    VT inv[kX][kXRows], x[kX][kXRows];
+    float co[COEF ? CH : 1][COEF ? 6 : 1][COEF ? kChunk : 1];
+    double sum[CH][kLanes];
+    VT max[CH][kLanes];
+    WaitSmem<VT, CH> wait;
+};
+
+template<class VT, bool COEF, int G, int K>
+__global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
+    // rows whose neighbour loads are in flight together
+    constexpr int kGroup = sizeof(VT) == 4 ? (G == 1 ? 8 : 4) : (G == 1 ? 4 : 2);
+    constexpr int R = K * kPerLane;
+    constexpr bool kHere = G * K <= kRoomy<VT>;  // x and 1/diag in shared memory
+    extern __shared__ __align__(16) unsigned char dynSm[];
+    ChunkSmem<VT, COEF, G * K>& S = *reinterpret_cast<ChunkSmem<VT, COEF, G * K>*>(dynSm);
+    const int n = a.n, nch = a.nch, grp = (int)threadIdx.x / kLanes, t = (int)threadIdx.x % kLanes;
+    unsigned* flags = &a.st->flags;
+    RowPair<VT>* __restrict__ pair = a.pair;
+    const VT negoff = a.negoff;
+    // this group's chunks: slots grp * K + k of the block, striped over the grid so that the
+    // blocks' counts differ by one at most
+    auto chunk_of = [&](int k) { return (int)blockIdx.x + (grp * K + k) * (int)gridDim.x; };
+    auto rows_of = [&](int k) { return max(min(n - chunk_of(k) * kChunk, kChunk), 0); };
+
+    // ---- init: r = rhs, x = 0, z = D^-1 r; partial z.r and max|r| (PCGSolver.cpp:151-168)
+    if(threadIdx.x == 0) S.wait.bad = 0;
+    VT r[R], q[R];  // q holds z from phase B to the next phase A
+#pragma unroll
+    for(int k = 0; k < K; ++k) {
+        const int slot = grp * K + k, base = chunk_of(k) * kChunk, rows = rows_of(k);
+        double acc = 0.0;
+        VT m = VT(0);
+#pragma unroll
+        for(int j = 0; j < kPerLane; ++j) {
+            const int l = t + j * kLanes;
+            uint2 nbv = make_uint2(kNoRow << 18, kNoRow << 18);
+            float dg = 0.f;
+            VT rv = VT(0), zv = VT(0), iv = VT(0);
+            asm volatile("" : : : "memory");  // a row's loads at a time: registers
+            if(l < rows) {
+                const int e = base + l;
+                int32_t nb[6];
+#pragma unroll
+                for(int p = 0; p < 6; ++p) nb[p] = __ldg(a.nbr + (size_t)p * n + e);
+                nbv.x = row_code(nb[0] >= 0 ? e - nb[0] : 0, l, nb[1] >= 0 ? e - nb[1] : 0, -1, nb[2] >= 0);
+                nbv.y = row_code(nb[5] >= 0 ? nb[5] - e : 0, l, nb[4] >= 0 ? nb[4] - e : 0, 1, nb[3] >= 0);
+                dg = __ldg(a.diag + e);
+                if constexpr(COEF)
+#pragma unroll
+                    for(int p = 0; p < 6; ++p) S.co[slot][p][l] = __ldg(a.coef + (size_t)p * n + e);
+                rv = (VT)__ldg(a.rhsF + e);
+                const VT ab = vabs(rv);
+                m = m > ab ? m : ab;
+                iv = __ldg(a.invd + e);
+                zv = iv * rv;
+                pair[e] = {zv, VT(0)};
+                acc = acc + (double)zv * (double)rv;
+            }
+            if constexpr(kHere) {
+                S.inv[slot][l] = iv;
+                S.x[slot][l] = VT(0);
+            } else if(rows > 0) a.x[base + l] = VT(0);
+            S.nb[slot][l] = nbv;
+            S.diag[slot][l] = dg;
+            S.s[slot][l] = VT(0);
+            r[k * kPerLane + j] = rv;
+            q[k * kPerLane + j] = zv;
+        }
+        if(t == 0) S.s[slot][kNoRow] = VT(0);
+        if constexpr(COEF) if(rows < kChunk)
+            for(int l = rows + t; l < kChunk; l += kLanes)
+#pragma unroll
+                for(int p = 0; p < 6; ++p) S.co[slot][p][l] = 0.f;
+        S.sum[slot][t] = acc;
+        S.max[slot][t] = m;
+    }
+    __syncthreads();
+    double rho;
+    VT resid;
+    unsigned parity = 1;  // of this iteration's exchanges
+    auto publish = [&](auto withMax, auto release, PcgPacket* slots) {
+        // a warp of the group for each of its chunks
+        if(t < 32 * K) {
+            const int k = t >> 5, slot = grp * K + k, c = chunk_of(k);
+            if(c < nch)
+                packet_publish<VT, decltype(withMax)::value, decltype(release)::value>(
+                    S.sum[slot], S.max[slot], slots + (size_t)c * kPacketStride, parity);
+        }
+    };
+    publish(Yes(), Yes(), a.pkB);
+    if(!packet_wait<VT, true, true>(a.pkB, nch, parity, flags, S.wait, rho, resid)) return;
+    const VT tolFactor = fmax(a.tolFactor, VT(1e-30));
+    unsigned iter = 0, success = 0;
+    bool done = false;
+    VT tol = VT(0);
+    if(resid < (VT)FLT_MIN) {
+        done = true;
+        success = 1;
+    } else {
+        tol = tolFactor * resid;
+        if(rho < (double)FLT_MIN || isnan(rho)) done = true;
+    }
+    if(a.maxIter == 0) done = true;
+
+    // beta and every s are 0 in the first iteration, where s = z: z + 0 * 0 differs from z in
+    // the sign of a zero at most, which no sum or product keeps
+    VT beta = VT(0);
+    while(!done) {
+        // ---- phase A: s = z + beta s_old, q = A s, partial s.q (PCGSolver.cpp:173-174,192-193)
+        RowPair<VT> zn[kGroup][2], ye[kGroup];
+        uint2 nb[kGroup];
+        // what rows g0 .. of chunk k read from the pairs: their z neighbours, and the y
+        // neighbours across the chunk's ends
+        auto load_pairs = [&](int k, int g0) {
+            const RowPair<VT>* own = pair + (size_t)chunk_of(k) * kChunk;
+#pragma unroll
+            for(int u = 0; u < kGroup; ++u) {
+                const int j = g0 + u, l = t + j * kLanes;
+                nb[u] = S.nb[grp * K + k][l];
+                const int dM = (int)(nb[u].x & 0x3ffffu), dP = (int)(nb[u].y & 0x3ffffu);
+                zn[u][0] = ld_pair_if(own + (l - dM), dM != 0);
+                zn[u][1] = ld_pair_if(own + (l + dP), dP != 0);
+                if(j < 2) {
+                    const unsigned y = nb[u].x >> 18 & 0xfffu;
+                    ye[u] = ld_pair_if(own + (l - (int)(y - kNoRow - 1u)), y > kNoRow);
+                }
+                if(j >= kPerLane - 2) {
+                    const unsigned y = nb[u].y >> 18 & 0xfffu;
+                    ye[u] = ld_pair_if(own + (l + (int)(y - kNoRow - 1u)), y > kNoRow);
+                }
+            }
+        };
+        // the x neighbours across the chunk's ends: of its first and its last row
+        RowPair<VT> xe[K];
+#pragma unroll
+        for(int k = 0; k < K; ++k) {
+            const uint2 e = S.nb[grp * K + k][t == 0 ? 0 : kChunk - 1];
+            xe[k] = ld_pair_if(pair + (t == 0 ? chunk_of(k) * kChunk - 1 : (chunk_of(k) + 1) * kChunk),
+                               (t == 0 && (int)e.x < 0) || (t == kLanes - 1 && (int)e.y < 0));
+        }
+        load_pairs(0, 0);
+#pragma unroll
+        for(int k = 0; k < K; ++k)
+#pragma unroll
+            for(int j = 0; j < kPerLane; ++j) {
+                VT* ps = &S.s[grp * K + k][t + j * kLanes];
+                *ps = q[k * kPerLane + j] + beta * *ps;
+            }
+        group_sync(grp);
+        auto s_of = [&](const RowPair<VT>& p) { return p.z + beta * p.s; };
+#pragma unroll
+        for(int k = 0; k < K; ++k) {
+            const int slot = grp * K + k;
+            const VT* __restrict__ sS = S.s[slot];
+            double acc = 0.0;
+#pragma unroll
+            for(int g0 = 0; g0 < kPerLane; g0 += kGroup) {
+                if(k + g0 > 0) load_pairs(k, g0);
+#pragma unroll
+                for(int u = 0; u < kGroup; ++u) {
+                    const int j = g0 + u, l = t + j * kLanes;
+                    const unsigned yM = nb[u].x >> 18 & 0xfffu, yP = nb[u].y >> 18 & 0xfffu;
+                    // a missing neighbour's value is 0: its term -0 (or 0) changes no sum
+                    VT vyM = sS[j < 2 ? min(yM, kNoRow) : yM], vyP = sS[j >= kPerLane - 2 ? min(yP, kNoRow) : yP];
+                    if(j < 2) vyM = yM > kNoRow ? s_of(ye[u]) : vyM;
+                    if(j >= kPerLane - 2) vyP = yP > kNoRow ? s_of(ye[u]) : vyP;
+                    VT vxM = sS[j == 0 ? max(l - 1, 0) : l - 1], vxP = sS[l + 1];
+                    if(j == 0) vxM = t == 0 ? s_of(xe[k]) : vxM;
+                    if(j == kPerLane - 1) vxP = t == kLanes - 1 ? s_of(xe[k]) : vxP;
+                    vxM = (int)nb[u].x < 0 ? vxM : VT(0);
+                    vxP = (int)nb[u].y < 0 ? vxP : VT(0);
+                    auto cf = [&](int p) { return COEF ? (VT)S.co[slot][p][l] : negoff; };
+                    const VT sv = sS[l];
+                    VT tq = VT(0) + cf(0) * s_of(zn[u][0]);
+                    tq = tq + cf(1) * vyM;
+                    tq = tq + cf(2) * vxM;
+                    tq = tq + (VT)S.diag[slot][l] * sv;
+                    tq = tq + cf(3) * vxP;
+                    tq = tq + cf(4) * vyP;
+                    tq = tq + cf(5) * s_of(zn[u][1]);
+                    q[k * kPerLane + j] = tq;
+                    acc = acc + (double)sv * (double)tq;
+                }
+            }
+            S.sum[slot][t] = acc;
+        }
+        group_sync(grp);
+        // relaxed: phase A writes nothing that other blocks read, and its reads of the pairs
+        // are over when the sum formed from them is out
+        publish(No(), No(), a.pkA);
+        VT inv[kHere ? 1 : R];
+        if constexpr(!kHere)
+#pragma unroll
+            for(int k = 0; k < K; ++k)
+#pragma unroll
+                for(int j = 0; j < kPerLane; ++j) {
+                    const int l = t + j * kLanes;
+                    inv[k * kPerLane + j] = ld_const_if(a.invd + (size_t)chunk_of(k) * kChunk + l, l < rows_of(k));
+                }
+        double tmp;
+        VT unused;
+        if(!packet_wait<VT, false, false>(a.pkA, nch, parity, flags, S.wait, tmp, unused)) return;
+        if(tmp < (double)FLT_MIN) {
+            ++iter;
+            success = 1;
+            break;
+        }
+        const VT alpha = (VT)(rho / tmp);
+        parity ^= 1u;
+        // ---- phase B: r -= alpha q, max|r|, z = D^-1 r, partial z.r; then x += alpha s
+#pragma unroll
+        for(int k = 0; k < K; ++k) {
+            const int slot = grp * K + k, base = chunk_of(k) * kChunk;
+            const bool live = chunk_of(k) < nch;
+            double acc = 0.0;
+            VT m = VT(0);
+#pragma unroll
+            for(int j = 0; j < kPerLane; ++j) {
+                const int l = t + j * kLanes, i = k * kPerLane + j;
+                const VT rv = r[i] + (-alpha) * q[i];
+                r[i] = rv;
+                const VT ab = vabs(rv);
+                m = m > ab ? m : ab;
+                VT iv;
+                if constexpr(kHere) iv = S.inv[slot][l];
+                else iv = inv[i];
+                const VT zv = iv * rv;
+                q[i] = zv;
+                if(live) pair[base + l] = {zv, S.s[slot][l]};
+                acc = acc + (double)zv * (double)rv;
+            }
+            S.sum[slot][t] = acc;
+            S.max[slot][t] = m;
+        }
+        group_sync(grp);
+        publish(Yes(), Yes(), a.pkB);
+#pragma unroll
+        for(int k = 0; k < K; ++k) {
+            const int slot = grp * K + k;
+            if constexpr(kHere) {
+#pragma unroll
+                for(int j = 0; j < kPerLane; ++j)
+                    S.x[slot][t + j * kLanes] = S.x[slot][t + j * kLanes] + alpha * S.s[slot][t + j * kLanes];
+            } else if(chunk_of(k) < nch) {
+                VT* xp = a.x + (size_t)chunk_of(k) * kChunk + t;
+                VT xv[kPerLane];
+#pragma unroll
+                for(int j = 0; j < kPerLane; ++j) xv[j] = __ldcg(xp + j * kLanes);
+#pragma unroll
+                for(int j = 0; j < kPerLane; ++j) xp[j * kLanes] = xv[j] + alpha * S.s[slot][t + j * kLanes];
+            }
+        }
+        double rhoNew;
+        if(!packet_wait<VT, true, true>(a.pkB, nch, parity, flags, S.wait, rhoNew, resid)) return;
+        ++iter;
+        if(resid < tol) {
+            success = 1;
+            break;
+        }
+        beta = (VT)(rhoNew / rho);
+        rho = rhoNew;
+        if(iter >= a.maxIter) {
+            if(blockIdx.x == 0 && threadIdx.x == 0) atomicOr(flags, BNN_FLAG_PCG_MAXITER);
+            break;
+        }
+    }
+    if constexpr(kHere)
+#pragma unroll
+        for(int k = 0; k < K; ++k)
+#pragma unroll
+            for(int j = 0; j < kPerLane; ++j) {
+                const int l = t + j * kLanes;
+                if(l < rows_of(k)) a.x[(size_t)chunk_of(k) * kChunk + l] = S.x[grp * K + k][l];
+            }
+    if(blockIdx.x == 0 && threadIdx.x == 0) {
+        a.st->iter = iter;
+        a.st->success = success;
+        a.st->done = 1;
+        Sc<VT>::set_resid(a.st, resid);
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // Single-reduction PCG (Chronopoulos & Gear, 1989): the same Krylov iterates as
 // PCGSolver::solve_precond (PCGSolver.cpp:143-199) in exact arithmetic, with both inner
@@ -1496,8 +2069,7 @@ __global__ void k_d64_to_f32(int n, const double* __restrict__ a, float* __restr
     if(e < (size_t)n) b[e] = (float)a[e];
 }
 
-// Packs rows of a grid into the 16-byte records (layout at the top of this file).  The
-// caller guarantees the x neighbours are rows r-1 / r+1 and the y distances fit 16 bits.
+// Packs rows of a grid into the 16-byte records
 __global__ void k_pack_rows(int n, const float* __restrict__ diag, const int32_t* __restrict__ nbr,
                             int4* __restrict__ rec) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1505,14 +2077,7 @@ __global__ void k_pack_rows(int n, const float* __restrict__ diag, const int32_t
     int32_t nb[6];
 #pragma unroll
     for(int q = 0; q < 6; ++q) nb[q] = nbr[(size_t)q * n + r];
-    const unsigned dyM = nb[1] >= 0 ? (unsigned)(r - nb[1]) : 0u, dyP = nb[4] >= 0 ? (unsigned)(nb[4] - r) : 0u;
-    const unsigned dzM = nb[0] >= 0 ? (unsigned)(r - nb[0]) : 0u, dzP = nb[5] >= 0 ? (unsigned)(nb[5] - r) : 0u;
-    int4 v;
-    v.x = (int)(dyM | (dyP << 16));
-    v.y = (int)(dzM | (nb[2] >= 0 ? 0x80000000u : 0u));
-    v.z = (int)(dzP | (nb[3] >= 0 ? 0x80000000u : 0u));
-    v.w = __float_as_int(diag[r]);
-    rec[r] = v;
+    rec[r] = pack_row(r, nb, diag[r]);
 }
 // The off-diagonal planes of the rows as 2 float4 per row (6 values, plane order)
 __global__ void k_pack_coef(int n, const float* __restrict__ coef, float4* __restrict__ out) {
@@ -1542,6 +2107,17 @@ struct CoopState {
 };
 static CoopState g_coop;
 
+static int coop_sm_count(int& numSM) {
+    std::lock_guard<std::mutex> lk(g_coop.mu);
+    if(!g_coop.numSM) {
+        int dev = 0;
+        BNN_CUDA_CHECK(cudaGetDevice(&dev));
+        BNN_CUDA_CHECK(cudaDeviceGetAttribute(&g_coop.numSM, cudaDevAttrMultiProcessorCount, dev));
+    }
+    numSM = g_coop.numSM;
+    return BNN_OK;
+}
+
 // Holds `units` of the GPU for the lifetime of the object; waits while other solves hold
 // so much that this grid would not fit beside them.
 struct CoopShare {
@@ -1564,7 +2140,8 @@ int pcg_reserve(PcgWork& w, int n, bool fp64) {
     if(n <= w.cap && (!fp64 || w.x64)) return BNN_OK;
     if(n > w.cap) {
         pcg_release(w);
-        const int cap = (int)(n * 1.25) + 4096;
+        // whole chunks: the chunk-resident solve writes its last chunk's rows past n too
+        const int cap = ((int)(n * 1.25) + 4096 + kChunk - 1) / kChunk * kChunk;
         const size_t nch = ((size_t)cap + kChunk - 1) / kChunk + 1;
         w.nchCap = (int)nch;
         BNN_CUDA_CHECK(dev_alloc(&w.x, cap * sizeof(float)));
@@ -1577,6 +2154,7 @@ int pcg_reserve(PcgWork& w, int n, bool fp64) {
         BNN_CUDA_CHECK(dev_alloc(&w.r32, cap * sizeof(float)));
         BNN_CUDA_CHECK(dev_alloc(&w.rec, cap * sizeof(int4)));
         BNN_CUDA_CHECK(dev_alloc(&w.part, 3 * nch * sizeof(double)));
+        BNN_CUDA_CHECK(dev_alloc(&w.packets, 2 * nch * kPacketStride * sizeof(PcgPacket)));
         BNN_CUDA_CHECK(dev_alloc(&w.gs, sizeof(GridSync)));
         BNN_CUDA_CHECK(cudaMemset(w.gs, 0, sizeof(GridSync)));
         BNN_CUDA_CHECK(dev_alloc(&w.partMaxF, nch * sizeof(float)));
@@ -1610,20 +2188,104 @@ void pcg_release(PcgWork& w) {
         if(e) cudaEventDestroy(e);
     for(void* p : {(void*)w.rec, (void*)w.coefRow, (void*)w.x, (void*)w.r, (void*)w.z, (void*)w.s0, (void*)w.s1, (void*)w.q, (void*)w.d32, (void*)w.r32,
                    (void*)w.part, (void*)w.partMaxF, (void*)w.partMaxD, (void*)w.x64, (void*)w.r64, (void*)w.z64,
-                   (void*)w.s064, (void*)w.s164, (void*)w.q64, (void*)w.inv64, (void*)w.gs, (void*)w.st32[0],
+                   (void*)w.s064, (void*)w.s164, (void*)w.q64, (void*)w.inv64, (void*)w.gs, (void*)w.packets, (void*)w.st32[0],
                    (void*)w.st32[1], (void*)w.st64[0], (void*)w.st64[1], (void*)w.cgPart, (void*)w.cgMax})
         if(p) dev_free(p);
     w = PcgWork();
 }
 
+// The shape of a chunk-resident solve of n rows: groups per block and chunks per group (0:
+// more chunks than it holds, they take turns in k_pcg_persistent).  One block per SM; as few
+// groups as hold the chunks (more registers and loads in flight for each), then two chunks per
+// group.  The line lies where registers and shared memory end: 6 FP32 chunks per SM are 210 KB
+// of records, s and partials (1.82 M rows on 148 SMs), 4 FP64 chunks 186 KB; with off-diagonal
+// values 2 and 1.  Up to that line it is faster than k_pcg_persistent at every size (figures
+// above).
+struct ChunkShape {
+    int G = 0, K = 0;
+};
+template<class VT> static ChunkShape chunk_shape(int n, bool coef, int numSM) {
+    const int nch = (n + kChunk - 1) / kChunk;
+    const int per = (nch + numSM - 1) / numSM;
+    if(coef) return per <= (sizeof(VT) == 4 ? 2 : 1) ? ChunkShape{per, 1} : ChunkShape{};
+    const int most = sizeof(VT) == 4 ? 3 : 2;
+    if(per <= most) return {per, 1};
+    return per <= 2 * most ? ChunkShape{most, 2} : ChunkShape{};
+}
+struct ChunkKernel {
+    const void* fn = nullptr;
+    size_t smem = 0;
+};
+template<class VT, bool COEF, int G, int K> static ChunkKernel chunk_kernel_of() {
+    return {(const void*)k_pcg_chunk<VT, COEF, G, K>, sizeof(ChunkSmem<VT, COEF, G * K>)};
+}
+template<class VT> static ChunkKernel chunk_kernel(bool coef, ChunkShape c) {
+    if(coef) {
+        if constexpr(sizeof(VT) == 4) if(c.G == 2) return chunk_kernel_of<VT, true, 2, 1>();
+        return chunk_kernel_of<VT, true, 1, 1>();
+    }
+    if(c.G == 1) return chunk_kernel_of<VT, false, 1, 1>();
+    if constexpr(sizeof(VT) == 4) {
+        if(c.G == 2) return chunk_kernel_of<VT, false, 2, 1>();
+        return c.K == 1 ? chunk_kernel_of<VT, false, 3, 1>() : chunk_kernel_of<VT, false, 3, 2>();
+    } else {
+        return c.K == 1 ? chunk_kernel_of<VT, false, 2, 1>() : chunk_kernel_of<VT, false, 2, 2>();
+    }
+}
+
+// What the host waits for after a solve's launch: the state record, and the launch's time
+template<class VT> static int pcg_read_outcome(PcgWork& w, DevState* dst, DevState* hst, cudaStream_t s, PcgOutcome& out) {
+    BNN_CUDA_CHECK(cudaMemcpyAsync(hst, dst, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+    BNN_CUDA_CHECK(cudaStreamSynchronize(s));
+    if(w.ev[0] && w.ev[1]) {
+        float ms = 0.f;
+        if(cudaEventElapsedTime(&ms, w.ev[0], w.ev[1]) == cudaSuccess) out.kernelMs = ms;
+    }
+    if(hst->flags & BNN_FLAG_TIMEOUT) { bnn_set_error("PCG grid barrier timed out"); return BNN_ERR_TIMEOUT; }
+    out.iterations = hst->iter;
+    out.success = hst->success;
+    out.residual = sizeof(VT) == 8 ? hst->resid64 : (double)hst->resid;
+    return BNN_OK;
+}
+
+// One PCG solve by k_pcg_chunk in the shape chunk_shape gave
+template<class VT>
+static int pcg_solve_chunk(PcgWork& w, int n, ChunkShape shape, int numSM, const float* rhsF, const float* diag,
+                           const VT* invd, const int32_t* nbr, const float* coef, VT negoff, VT tolFactor,
+                           unsigned maxIter, VT* x, DevState* dst, DevState* hst, cudaStream_t s, PcgOutcome& out) {
+    out = PcgOutcome();
+    const ChunkKernel kern = chunk_kernel<VT>(coef != nullptr, shape);
+    BNN_CUDA_CHECK(cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kern.smem));
+    ChunkArgs<VT> a;
+    a.n = n; a.nch = (n + kChunk - 1) / kChunk;
+    a.rhsF = rhsF; a.diag = diag; a.invd = invd; a.nbr = nbr; a.coef = coef; a.negoff = negoff;
+    a.tolFactor = tolFactor; a.maxIter = maxIter; a.x = x;
+    a.pair = sizeof(VT) == 8 ? (RowPair<VT>*)(void*)w.st64[0] : (RowPair<VT>*)(void*)w.st32[0];
+    a.pkA = w.packets;
+    a.pkB = a.pkA + (size_t)w.nchCap * kPacketStride;
+    a.st = dst;
+    BNN_CUDA_CHECK(cudaMemsetAsync(w.packets, 0, 2 * (size_t)w.nchCap * kPacketStride * sizeof(PcgPacket), s));
+    void* args[] = {(void*)&a};
+    const int most = numSM < kMostSM ? numSM : kMostSM, grid = a.nch < most ? a.nch : most;
+    CoopShare share((long long)grid * kShareUnits, (long long)numSM * kShareUnits);
+    if(w.ev[0]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[0], s));
+    BNN_CUDA_CHECK(cudaLaunchCooperativeKernel(kern.fn, dim3(grid), dim3(shape.G * kLanes), args, kern.smem, s));
+    bnn_note_launch();
+    if(w.ev[1]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[1], s));
+    return pcg_read_outcome<VT>(w, dst, hst, s, out);
+}
+
 // Runs one PCG solve (VT vectors) as a single cooperative launch.  Returns BNN status;
 // the solution is left in x.
 template<class VT>
-static int pcg_solve_t(PcgWork& w, int n, const float* rhsF, const float* diag, const VT* invd, const int32_t* nbr,
+static int pcg_solve_t(PcgWork& w, int n, ChunkShape shape, int numSM, const float* rhsF, const float* diag, const VT* invd, const int32_t* nbr,
                        const int4* rec, const float* coef, const float4* coefRow, VT negoff, VT tolFactor, unsigned maxIter, VT* x, VT* r, VT* z, VT* s0, VT* s1, VT* q,
                        VT* partMax, bool twoReductions, DevState* dst, DevState* hst, cudaStream_t s, PcgOutcome& out) {
     out = PcgOutcome();
     if(n == 0) { out.success = 1; return BNN_OK; }
+    if(shape.G > 0)
+        return pcg_solve_chunk<VT>(w, n, shape, numSM, rhsF, diag, invd, nbr, coef, negoff, tolFactor, maxIter, x, dst, hst,
+                                   s, out);
     const int nch = (n + kChunk - 1) / kChunk;
     const bool packedCoef = rec && coefRow;
     // kernel variant: bit 0 FP64, bit 1 packed rows, bit 2 coefficients, bit 3 single reduction
@@ -1636,19 +2298,13 @@ static int pcg_solve_t(PcgWork& w, int n, const float* rhsF, const float* diag, 
         kern = coefRow ? (const void*)k_pcg_cg1<VT, true, true> : (const void*)k_pcg_cg1<VT, true, false>;
     else
         kern = coef ? (const void*)k_pcg_cg1<VT, false, true> : (const void*)k_pcg_cg1<VT, false, false>;
-    int numSM = 0, perSMv = 0;
+    int perSMv = 0;
     {
         std::lock_guard<std::mutex> lk(g_coop.mu);
-        if(!g_coop.numSM) {
-            int dev = 0;
-            BNN_CUDA_CHECK(cudaGetDevice(&dev));
-            BNN_CUDA_CHECK(cudaDeviceGetAttribute(&g_coop.numSM, cudaDevAttrMultiProcessorCount, dev));
-        }
         if(!g_coop.perSM[ti]) {
             BNN_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_coop.perSM[ti], kern, kLanes, 0));
             if(g_coop.perSM[ti] < 1) { bnn_set_error("persistent PCG kernel cannot be resident"); return BNN_ERR_CUDA; }
         }
-        numSM = g_coop.numSM;
         perSMv = g_coop.perSM[ti];
     }
     const int cap = numSM * perSMv;
@@ -1674,23 +2330,13 @@ static int pcg_solve_t(PcgWork& w, int n, const float* rhsF, const float* diag, 
     BNN_CUDA_CHECK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kLanes), args, 0, s));
     bnn_note_launch();
     if(w.ev[1]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[1], s));
-    BNN_CUDA_CHECK(cudaMemcpyAsync(hst, dst, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-    BNN_CUDA_CHECK(cudaStreamSynchronize(s));
-    if(w.ev[0] && w.ev[1]) {
-        float ms = 0.f;
-        if(cudaEventElapsedTime(&ms, w.ev[0], w.ev[1]) == cudaSuccess) out.kernelMs = ms;
-    }
-    if(hst->flags & BNN_FLAG_TIMEOUT) { bnn_set_error("PCG grid barrier timed out"); return BNN_ERR_TIMEOUT; }
-    out.iterations = hst->iter;
-    out.success = hst->success;
-    out.residual = sizeof(VT) == 8 ? hst->resid64 : (double)hst->resid;
-    return BNN_OK;
+    return pcg_read_outcome<VT>(w, dst, hst, s, out);
 }
 
 // mode: BNN_PCG_FP32 / FP64 / REFINED, optionally with BNN_PCG_SINGLE_REDUCTION.  Pressure
 // written to `pressure` (float, n).
 int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const float* invd, const int32_t* nbr,
-              const float* coef, bool gridRows, float dt, int modeFlags, float tol, unsigned maxIter, float innerTol,
+              const float* coef, RowLayout layout, float dt, int modeFlags, float tol, unsigned maxIter, float innerTol,
               float outerTol, float* pressure, double* x64out, DevState* dst, DevState* hst, cudaStream_t s,
               PcgOutcome& out) {
     const int mode = modeFlags & BNN_PCG_MODE_MASK;
@@ -1702,7 +2348,16 @@ int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const floa
     out = PcgOutcome();
     const int4* rec = nullptr;
     const float4* coefRow = nullptr;
-    if(gridRows && n > 0) {
+    int numSM = 0;
+    rc = coop_sm_count(numSM);
+    if(rc != BNN_OK) return rc;
+    const int chunkSM = numSM < kMostSM ? numSM : kMostSM;
+    const bool gridRows = layout != kRowsAny;
+    ChunkShape shape;
+    if(layout == kRowsCompact && two && n > 0)
+        shape = mode == BNN_PCG_FP64 ? chunk_shape<double>(n, coef != nullptr, chunkSM)
+                                     : chunk_shape<float>(n, coef != nullptr, chunkSM);
+    if(gridRows && n > 0 && shape.G == 0) {
         { k_pack_rows<<<nb, 256, 0, s>>>(n, diag, nbr, w.rec); bnn_note_launch(); }
         rec = w.rec;
         if(coef) {
@@ -1713,7 +2368,7 @@ int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const floa
         }
     }
     if(mode == BNN_PCG_FP32) {
-        rc = pcg_solve_t<float>(w, n, rhs, diag, invd, nbr, rec, coef, coefRow, -(1.0f * dt), tol, maxIter, w.x, w.r, w.z, w.s0, w.s1,
+        rc = pcg_solve_t<float>(w, n, shape, numSM, rhs, diag, invd, nbr, rec, coef, coefRow, -(1.0f * dt), tol, maxIter, w.x, w.r, w.z, w.s0, w.s1,
                                 w.q, w.partMaxF, two, dst, hst, s, out);
         if(rc != BNN_OK) return rc;
         if(n > 0) BNN_CUDA_CHECK(cudaMemcpyAsync(pressure, w.x, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -1722,7 +2377,7 @@ int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const floa
     }
     if(mode == BNN_PCG_FP64) {
         if(n > 0) { k_inv_diag64<<<nb, 256, 0, s>>>(n, diag, w.inv64); bnn_note_launch(); }
-        rc = pcg_solve_t<double>(w, n, rhs, diag, w.inv64, nbr, rec, coef, coefRow, -(double)(1.0f * dt), (double)tol, maxIter, w.x64,
+        rc = pcg_solve_t<double>(w, n, shape, numSM, rhs, diag, w.inv64, nbr, rec, coef, coefRow, -(double)(1.0f * dt), (double)tol, maxIter, w.x64,
                                  w.r64, w.z64, w.s064, w.s164, w.q64, w.partMaxD, two, dst, hst, s, out);
         if(rc != BNN_OK) return rc;
         if(n > 0) { k_d64_to_f32<<<nb, 256, 0, s>>>(n, w.x64, pressure); bnn_note_launch(); }
@@ -1745,7 +2400,7 @@ int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const floa
         if(res < (double)outerTol * bmax) { ok = true; break; }
         { k_ir_to_f32<<<nb, 256, 0, s>>>(n, w.r64, w.r32); bnn_note_launch(); }
         PcgOutcome inner;
-        rc = pcg_solve_t<float>(w, n, w.r32, diag, invd, nbr, rec, coef, coefRow, -(1.0f * dt), innerTol, maxIter, w.d32, w.r, w.z, w.s0,
+        rc = pcg_solve_t<float>(w, n, shape, numSM, w.r32, diag, invd, nbr, rec, coef, coefRow, -(1.0f * dt), innerTol, maxIter, w.d32, w.r, w.z, w.s0,
                                 w.s1, w.q, w.partMaxF, two, dst, hst, s, inner);
         if(rc != BNN_OK) return rc;
         total += inner.iterations;
@@ -1811,14 +2466,7 @@ __global__ void kb_pack_rows(const IrScene* __restrict__ S, const unsigned* __re
     int32_t nb[6];
 #pragma unroll
     for(int k = 0; k < 6; ++k) nb[k] = c.nbr[(size_t)k * n + r];
-    const unsigned dyM = nb[1] >= 0 ? (unsigned)(r - nb[1]) : 0u, dyP = nb[4] >= 0 ? (unsigned)(nb[4] - r) : 0u;
-    const unsigned dzM = nb[0] >= 0 ? (unsigned)(r - nb[0]) : 0u, dzP = nb[5] >= 0 ? (unsigned)(nb[5] - r) : 0u;
-    int4 v;
-    v.x = (int)(dyM | (dyP << 16));
-    v.y = (int)(dzM | (nb[2] >= 0 ? 0x80000000u : 0u));
-    v.z = (int)(dzP | (nb[3] >= 0 ? 0x80000000u : 0u));
-    v.w = __float_as_int(c.diag[r]);
-    c.rec[r] = v;
+    c.rec[r] = pack_row(r, nb, c.diag[r]);
 }
 __global__ void __launch_bounds__(kLanes) kb_ir_init(const IrScene* __restrict__ S, const unsigned* __restrict__ P,
                                                      int ns) {
@@ -1991,18 +2639,14 @@ int pcg_solve_batch_refined(BatchPcgCtx& ctx, BatchSolveItem* items, int count, 
 
     // cooperative grid of the inner solves
     int numSM = 0, perSMv = 0;
+    rc = coop_sm_count(numSM);
+    if(rc != BNN_OK) return rc;
     {
         std::lock_guard<std::mutex> lk(g_coop.mu);
-        if(!g_coop.numSM) {
-            int dev = 0;
-            BNN_CUDA_CHECK(cudaGetDevice(&dev));
-            BNN_CUDA_CHECK(cudaDeviceGetAttribute(&g_coop.numSM, cudaDevAttrMultiProcessorCount, dev));
-        }
         if(!g_coop.perSM[15]) {
             BNN_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_coop.perSM[15], k_pcg_batch, kLanes, 0));
             if(g_coop.perSM[15] < 1) { bnn_set_error("batched PCG kernel cannot be resident"); return BNN_ERR_CUDA; }
         }
-        numSM = g_coop.numSM;
         perSMv = g_coop.perSM[15];
     }
 

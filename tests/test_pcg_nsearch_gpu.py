@@ -220,6 +220,57 @@ def test_pcg_grid_row_layouts_match_oracle(bnn, oracle_mod, kind, mode, omode):
         assert np.array_equal(x, xo)
 
 
+def _first_cells(nx, ny, n, seed):
+    """The first n cells, in cell order, of a grid of nx by ny cells a plane: neighbour
+    table (-z, -y, -x, +x, +y, +z), diagonal with 1/theta terms, right-hand side."""
+    r = np.arange(n, dtype=np.int64)
+    x, y = r % nx, r // nx % ny
+    cand = [r - nx * ny, r - nx, r - 1, r + 1, r + nx, r + nx * ny]
+    ok = [r >= nx * ny, y > 0, x > 0, x < nx - 1, y < ny - 1, np.ones(n, bool)]
+    nbr = np.stack([np.where(o & (c >= 0) & (c < n), c, -1) for c, o in zip(cand, ok)], 1).astype(np.int32)
+    rng = np.random.default_rng(seed)
+    theta = (0.05 + 0.95 * rng.random((n, 6))).astype(np.float32)
+    one = np.float32(1.0)
+    diag = (np.where(nbr >= 0, one, one / theta).sum(1) * np.float32(0.004)).astype(np.float32)
+    return nbr, diag, rng.standard_normal(n).astype(np.float32)
+
+
+def _csr_of(nbr, diag, off):
+    """The same rows for the oracle: entries in column order, the diagonal in its place."""
+    n = len(diag)
+    cols = np.concatenate([nbr[:, :3], np.arange(n, dtype=np.int32)[:, None], nbr[:, 3:]], 1)
+    vals = np.full(cols.shape, off, np.float32)
+    vals[:, 3] = diag
+    keep = cols >= 0
+    start = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.uint32)
+    return start, cols[keep].astype(np.uint32), vals[keep]
+
+
+# Edges of the chunk-resident solve on 148 SMs: of a 2048-row chunk; of one, two, three and six
+# chunks per SM (FP32) and of one, two and four (FP64); of the rows its 8-byte records hold (512
+# cells along x, 2^18 - 1 a plane), past which the other kernels take over.
+_SM = 148 * 2048
+
+
+@pytest.mark.parametrize("nx,ny,n", [
+    (1, 1, 1), (7, 5, 2047), (7, 5, 2048), (7, 5, 2049), (512, 3, 4 * 2048 + 1), (513, 3, 4 * 2048 + 1),
+    (31, 29, 32 * 2048), (31, 29, 33 * 2048 + 5), (64, 80, _SM), (64, 80, _SM + 1), (101, 90, 2 * _SM), (101, 90, 2 * _SM + 1),
+    (102, 154, 3 * _SM + 1), (102, 154, 4 * _SM), (102, 154, 4 * _SM + 1), (260, 260, 6 * _SM), (260, 260, 6 * _SM + 1),
+    (512, 511, 600_000), (512, 512, 600_000)])
+@pytest.mark.parametrize("mode,omode", [("fp32", 0), ("fp64", 1)])
+def test_pcg_chunk_edges_match_oracle(bnn, oracle_mod, nx, ny, n, mode, omode):
+    nbr, diag, rhs = _first_cells(nx, ny, n, seed=nx + n)
+    off = -float(np.float32(0.004))
+    # a handful of iterations: what differs would differ in the first ones already
+    x, st = bnn.pcg_solve_7pt(diag, nbr, off, rhs, 1e-6, 5, mode=mode)
+    xo, so = oracle_mod.pcg(*_csr_of(nbr, diag, off), rhs, 1e-6, 5, omode)
+    assert st["iterations"] == so["iterations"]
+    if mode == "fp32":
+        assert np.array_equal(x.astype(np.float32), xo.astype(np.float32))
+    else:
+        assert np.array_equal(x, xo)
+
+
 def test_barrier_wait_gives_up_and_device_stays_usable(bnn, oracle_mod):
     """A block waiting at a barrier that nothing completes (sized for two blocks, one
     launched) gives up after its limit and reports a timeout; the device then solves a
