@@ -209,102 +209,144 @@ __global__ void k_gather_pos(const float* __restrict__ pos, const uint32_t* __re
     out[i] = make_float4(pos[3 * (size_t)p], pos[3 * (size_t)p + 1], pos[3 * (size_t)p + 2], __uint_as_float(p));
 }
 
-// NeighborSearch::query3D (NeighborSearch.cpp:530-692) per point: every other point of the
-// 27 hash cells with (dx*dx + dy*dy) + dz*dz < r^2.  One thread per point in cell-sorted
-// order, so a warp shares its candidate cells.  This pass counts each point's neighbours;
-// k_ns_query_write then writes them, visiting the candidates in the same order.
-__global__ void __launch_bounds__(256) k_ns_count(const float4* __restrict__ sp, const uint32_t* __restrict__ scid,
-                                                  uint32_t n, const uint32_t* __restrict__ cellStart, int d0, int d1,
-                                                  float r2, uint32_t* __restrict__ counts) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= n) return;
-    const float4 a = sp[i];
-    const uint32_t self = __float_as_uint(a.w);
-    const uint32_t c = scid[i];
-    const size_t plane = (size_t)d0 * d1;
-    uint32_t cnt = 0;
-    for(int dz = -1; dz <= 1; ++dz)
-        for(int dy = -1; dy <= 1; ++dy) {
-            const size_t row = (size_t)((long long)c + dz * (long long)plane + dy * (long long)d0);
-            const uint32_t b = cellStart[row - 1], e = cellStart[row + 2];
-            for(uint32_t j = b; j < e; ++j) {
-                const float4 q = sp[j];
-                const uint32_t other = __float_as_uint(q.w);
-                if(other == self) continue;
-                const float t0 = a.x - q.x, t1 = a.y - q.y, t2 = a.z - q.z;
-                const float l2 = t0 * t0 + t1 * t1 + t2 * t2;
-                if(l2 < r2) ++cnt;
-            }
-        }
-    counts[self] = cnt;
+// Packed FP32: two lanes of a 64-bit register, each operation rounded as the scalar one
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    return (unsigned long long)__float_as_uint(lo) | (unsigned long long)__float_as_uint(hi) << 32;
 }
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// a * b as a * b + (-0), which rounds to the product.  The -0 pair comes in as a kernel
+// argument: of a plain packed product and sum the assembler makes one fused operation, which
+// rounds once (20 of 4M points' lists changed).
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b, unsigned long long minus0) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(minus0));
+    return d;
+}
+constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
 
-// The writing pass, its stores gathered per warp: each lane appends its
-// neighbours to its own row of a shared-memory buffer, and as soon as one lane's row is
-// full the warp writes every lane's buffered entries out, one lane's entries at a time
-// (lanes k write entry k: consecutive addresses), instead of 32 lanes storing into 32
-// different lists at every candidate.  The lanes walk their candidate ranges in step (the
-// warp's longest range; shorter ones idle), so the warp's votes see every lane.  Each list
-// holds exactly the entries k_ns_count counted, in its visiting order.
-constexpr int kNsBuf = 32;   // entries a lane's buffer row holds
-constexpr int kNsGroup = 4;  // candidates tested between two checks of the rows
-__global__ void __launch_bounds__(256) k_ns_query_write(const float4* __restrict__ sp, const uint32_t* __restrict__ scid,
-                                                        uint32_t n, const uint32_t* __restrict__ cellStart, int d0,
-                                                        int d1, float r2, const unsigned long long* __restrict__ offsets,
-                                                        uint32_t* __restrict__ idx) {
-    __shared__ uint32_t buf[256 / 32][32][kNsBuf + 1];  // +1: a lane's row starts in its own bank
+// NeighborSearch::query3D (NeighborSearch.cpp:530-692): every other point of the 27 hash cells
+// around a point with (dx*dx + dy*dy) + dz*dz < r^2, in the order of the cells (z, y, x major)
+// and of the sorted points inside them.
+//
+// A warp owns P consecutive sorted points.  Points of one cell share their candidates, the 9
+// rows of 3 cells around it laid end to end: a lane holds one candidate of a group of 32 and
+// tests it against the cell's points one pair at a time (packed FP32, the points broadcast from
+// shared memory), a vote makes each point's hits in the group one word, kept by the point's
+// lane.  Counting is then one population count per lane and group; in the writing pass
+// (WRITE) the warp writes each point's hits as consecutive entries.  A point is tested against
+// itself too; that bit is cleared in its word.
+//
+// Bound by instruction issue: about 9 per point and 32 candidates, 20 when writing, against 15
+// per point and candidate (and its store through a shared buffer) with a thread per point that
+// walks the candidates alone.  Measured, whole bnn_neighbors call: 4M points and 933 M entries
+// 8.70 ms (11.5 with a thread per point), 20,011 points 0.335 ms (0.617).
+constexpr int kNsWarps = 4;  // warps per block: they end at different times
+template<int P, bool WRITE>
+__global__ void __launch_bounds__(kNsWarps * 32) k_ns_pairs(const float4* __restrict__ sp, const uint32_t* __restrict__ scid,
+                                                            uint32_t n, const uint32_t* __restrict__ cellStart, int d0,
+                                                            int d1, float r2, unsigned long long minus0,
+                                                            uint32_t* __restrict__ counts,
+                                                            const unsigned long long* __restrict__ offsets,
+                                                            uint32_t* __restrict__ idx) {
+    constexpr unsigned full = 0xffffffffu;
+    __shared__ __align__(16) float2 sXY[kNsWarps][P], sZ[kNsWarps][P / 2];  // {x pair, y pair} per pair, {z pair}
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned full = 0xffffffffu;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i < n;
-    const float4 a = live ? sp[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t first = (blockIdx.x * kNsWarps + warp) * (uint32_t)P;
+    if(first >= n) return;
+    const int mine = (int)min((uint32_t)P, n - first);  // points of this warp
+    const bool live = lane < mine;
+    const float4 a = live ? sp[first + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
     const uint32_t self = __float_as_uint(a.w);
-    const uint32_t c = live ? scid[i] : 0u;
-    const size_t plane = (size_t)d0 * d1;
-    const unsigned long long o = live ? offsets[self] : 0ull;
-    unsigned long long written = 0;  // entries of this lane's list already in idx
-    uint32_t held = 0;               // entries in this lane's buffer row
-    uint32_t* row = buf[warp][lane];
-    auto flush = [&]() {
-        __syncwarp();
-        for(int L = 0; L < 32; ++L) {
-            const uint32_t cntL = __shfl_sync(full, held, L);
-            const unsigned long long dst = __shfl_sync(full, o + written, L);
-            if((uint32_t)lane < cntL) idx[dst + lane] = buf[warp][L][lane];
+    const uint32_t cell = live ? scid[first + lane] : full;
+    if(lane < P) {
+        float* xy = reinterpret_cast<float*>(&sXY[warp][lane & ~1]);
+        xy[lane & 1] = a.x;
+        xy[2 + (lane & 1)] = a.y;
+        reinterpret_cast<float*>(sZ[warp])[lane] = a.z;
+    }
+    __syncwarp();
+    unsigned long long o = WRITE && live ? offsets[self] : 0ull;
+    uint32_t cnt = 0;
+    for(int s0 = 0; s0 < mine;) {
+        // the points s0 .. s1 - 1 of one cell
+        const uint32_t c = __shfl_sync(full, cell, s0);
+        const int s1 = s0 + __popc(__ballot_sync(full, cell == c && live));
+        // its candidate rows: lane q the q-th one, at places before .. before + len - 1 of the list
+        uint32_t b = 0, len = 0;
+        if(lane < 9) {
+            const long long row = (long long)c + (lane / 3 - 1) * ((long long)d0 * d1) + (lane % 3 - 1) * (long long)d0;
+            b = cellStart[row - 1];
+            len = cellStart[row + 2] - b;
         }
-        __syncwarp();
-        written += held;
-        held = 0;
-    };
-    for(int dz = -1; dz <= 1; ++dz)
-        for(int dy = -1; dy <= 1; ++dy) {
-            uint32_t b = 0, e = 0;
-            if(live) {
-                const size_t r = (size_t)((long long)c + dz * (long long)plane + dy * (long long)d0);
-                b = cellStart[r - 1];
-                e = cellStart[r + 2];
+        uint32_t before = len;
+#pragma unroll
+        for(int off = 1; off < 16; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(full, before, off);
+            if(lane >= off) before += v;
+        }
+        const uint32_t total = __shfl_sync(full, before, 8);
+        before -= len;
+        const uint32_t shift = b - before;  // place in the list + shift = sorted index
+        uint32_t rowAt[9], rowShift[9];
+#pragma unroll
+        for(int q = 0; q < 9; ++q) {
+            rowAt[q] = __shfl_sync(full, before, q);
+            rowShift[q] = __shfl_sync(full, shift, q);
+        }
+        // this lane's point stands at this place of the list (the middle row holds its cell)
+        const uint32_t selfAt = first + lane - rowShift[4];
+        for(uint32_t g = 0; g < total; g += 32) {
+            const uint32_t at = g + lane;
+            uint32_t sh = rowShift[0];
+#pragma unroll
+            for(int q = 1; q < 9; ++q) sh = at >= rowAt[q] ? rowShift[q] : sh;
+            const float4 q = at < total ? sp[at + sh] : make_float4(INFINITY, 0.f, 0.f, 0.f);
+            const unsigned long long nx = pack2(-q.x, -q.x), ny = pack2(-q.y, -q.y), nz = pack2(-q.z, -q.z);
+            unsigned hits = 0;
+            for(int k = s0 & ~1; k < s1; k += 2) {
+                const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(&sXY[warp][k]);
+                const unsigned long long z = *reinterpret_cast<const unsigned long long*>(&sZ[warp][k >> 1]);
+                const unsigned long long t0 = add2(xy.x, nx), t1 = add2(xy.y, ny), t2 = add2(z, nz);
+                const unsigned long long l2 = add2(add2(mul2(t0, t0, minus0), mul2(t1, t1, minus0)), mul2(t2, t2, minus0));
+                const unsigned h0 = __ballot_sync(full, __uint_as_float((unsigned)l2) < r2);
+                const unsigned h1 = __ballot_sync(full, __uint_as_float((unsigned)(l2 >> 32)) < r2);
+                if(lane == k) hits = h0;
+                if(lane == k + 1) hits = h1;
             }
-            const uint32_t len = e - b;
-            uint32_t most = len;
-#pragma unroll
-            for(int off = 16; off > 0; off >>= 1) most = max(most, __shfl_xor_sync(full, most, off));
-            // candidates four at a time (their loads in flight together); a group adds at
-            // most four entries, so the warp writes out before any row could overflow
-            for(uint32_t t = 0; t < most; t += kNsGroup) {
-                float4 q[kNsGroup];
-#pragma unroll
-                for(int u = 0; u < kNsGroup; ++u) q[u] = t + u < len ? sp[b + t + u] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for(int u = 0; u < kNsGroup; ++u) {
-                    const uint32_t other = __float_as_uint(q[u].w);
-                    const float t0 = a.x - q[u].x, t1 = a.y - q[u].y, t2 = a.z - q[u].z;
-                    const float l2 = t0 * t0 + t1 * t1 + t2 * t2;
-                    if(t + u < len && other != self && l2 < r2) row[held++] = other;
+            if(lane < s0 || lane >= s1) hits = 0;
+            if(selfAt - g < 32u) hits &= ~(1u << (selfAt - g));
+            if constexpr(!WRITE) cnt += __popc(hits);
+            else {
+                const uint32_t other = __float_as_uint(q.w);
+                const unsigned lt = (1u << lane) - 1u;
+                for(unsigned todo = __ballot_sync(full, hits != 0u); todo; todo &= todo - 1) {
+                    const int k = __ffs(todo) - 1;
+                    const unsigned h = __shfl_sync(full, hits, k);
+                    const unsigned long long to = __shfl_sync(full, o, k);
+                    if(h >> lane & 1u) idx[to + __popc(h & lt)] = other;
                 }
-                if(__any_sync(full, held > (uint32_t)(kNsBuf - kNsGroup))) flush();
+                o += __popc(hits);
             }
         }
-    if(__any_sync(full, held != 0u)) flush();
+        s0 = s1;
+    }
+    if(!WRITE && live) counts[self] = cnt;
+}
+// Points per warp: 32 share their candidates' loads best; below kNsFew points, 8 give the GPU
+// four times the warps
+constexpr uint32_t kNsFew = 150000;
+template<bool WRITE>
+void launch_ns_pairs(const float4* sp, const uint32_t* scid, uint32_t n, const uint32_t* cellStart, int d0, int d1, float r2,
+                     uint32_t* counts, const unsigned long long* offsets, uint32_t* idx, cudaStream_t s) {
+    const uint32_t per = (n < kNsFew ? 8u : 32u) * kNsWarps;
+    const unsigned blocks = (n + per - 1) / per;
+    if(n < kNsFew) k_ns_pairs<8, WRITE><<<blocks, kNsWarps * 32, 0, s>>>(sp, scid, n, cellStart, d0, d1, r2, kMinusZero2, counts, offsets, idx);
+    else k_ns_pairs<32, WRITE><<<blocks, kNsWarps * 32, 0, s>>>(sp, scid, n, cellStart, d0, d1, r2, kMinusZero2, counts, offsets, idx);
+    bnn_note_launch();
 }
 } // namespace
 
@@ -472,8 +514,8 @@ extern "C" int bnn_neighbors(const float* pos_dev, uint32_t n, float radius, uin
     if(wsb) BNN_CUDA_CHECK(ws.alloc(wsb, s));
     BNN_CUDA_CHECK(exclusive_scan_u32(cnt.as<uint32_t>(), start.as<uint32_t>(), (size_t)V, ws.p, s));
     BNN_CUDA_CHECK(counts.alloc((size_t)n * sizeof(uint32_t), s));
-    { k_ns_count<<<(n + 255) / 256, 256, 0, s>>>(sp.as<float4>(), cidSorted.as<uint32_t>(), n, start.as<uint32_t>(),
-                                                 (int)d0, (int)d1, r2, counts.as<uint32_t>()); bnn_note_launch(); }
+    launch_ns_pairs<false>(sp.as<float4>(), cidSorted.as<uint32_t>(), n, start.as<uint32_t>(), (int)d0, (int)d1, r2,
+                           counts.as<uint32_t>(), nullptr, nullptr, s);
     size_t wsb64 = scan_workspace_bytes_u64(n);
     if(wsb64) BNN_CUDA_CHECK(ws64.alloc(wsb64, s));
     BNN_CUDA_CHECK(exclusive_scan_u32_to_u64(counts.as<uint32_t>(), (unsigned long long*)offsets_dev, n, ws64.p, s));
@@ -483,9 +525,8 @@ extern "C" int bnn_neighbors(const float* pos_dev, uint32_t n, float radius, uin
     if(total) *total = tot;
     if(tot > capacity) return BNN_ERR_CAPACITY;
     if(tot && !idx_dev) return BNN_ERR_INVALID_ARGUMENT;
-    { k_ns_query_write<<<(n + 255) / 256, 256, 0, s>>>(sp.as<float4>(), cidSorted.as<uint32_t>(), n, start.as<uint32_t>(),
-                                                      (int)d0, (int)d1, r2, (const unsigned long long*)offsets_dev,
-                                                      idx_dev); bnn_note_launch(); }
+    launch_ns_pairs<true>(sp.as<float4>(), cidSorted.as<uint32_t>(), n, start.as<uint32_t>(), (int)d0, (int)d1, r2, nullptr,
+                          (const unsigned long long*)offsets_dev, idx_dev, s);
     BNN_CUDA_CHECK(cudaGetLastError());
     BNN_CUDA_CHECK(cudaStreamSynchronize(s));
     return BNN_OK;

@@ -390,6 +390,46 @@ def test_neighbors_set_equal(bnn, oracle_mod, n, seed):
     assert np.array_equal(gi[a], idx_o)
 
 
+@pytest.mark.parametrize("n,seed,r", [(1, 3, 0.1), (2, 3, 2.0), (31, 3, 0.4), (33, 3, 0.4), (2_049, 3, 0.2), (149_999, 5, 0.012),
+                                      (150_001, 5, 0.012)])
+def test_neighbors_order_and_edges(bnn, n, seed, r):
+    """Lists in their order (27 cells z, y, x major, a cell's points by index), around the sizes
+    where a warp's points end and where the points per warp change, with coincident points and a
+    cell of one point beside crowded ones; the reference is the same test in numpy float32."""
+    rng = np.random.default_rng(seed)
+    p = rng.random((n, 3)).astype(np.float32)
+    p[: n // 3] = np.float32(0.5) + np.float32(0.02) * rng.standard_normal((n // 3, 3)).astype(np.float32)
+    if n > 40:
+        p[5:9] = p[4]
+    pos = _dev(p)
+    off = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    idx = torch.zeros(max(1, min(n * n, 60_000_000)), dtype=torch.int32, device="cuda")
+    tot = C.c_uint64()
+    bnn.capi.check(bnn.load().bnn_neighbors(pos.data_ptr(), n, r, off.data_ptr(), idx.data_ptr(), idx.numel(),
+                                            C.byref(tot), None), "bnn_neighbors")
+    off = off.cpu().numpy()
+    assert off[0] == 0 and off[-1] == tot.value
+    idx = idx[: tot.value].cpu().numpy()
+    rf = np.float32(r)
+    inv = np.float32(1.0 / float(rf))
+    t = p - np.float32(1.2345)
+    key = np.where(t >= 0, (inv * t).astype(np.int32), (inv * t).astype(np.int32) - 1)
+    d = key.max(0) - key.min(0) + 3
+    cell = key - key.min(0) + 1
+    lin = (cell[:, 2].astype(np.int64) * d[1] + cell[:, 1]) * d[0] + cell[:, 0]
+    order = np.argsort(lin, kind="stable")
+    slin = lin[order]
+    for i in np.unique(np.concatenate([np.arange(min(n, 40)), rng.integers(0, n, 300)])):
+        cand = [order[np.searchsorted(slin, lin[i] + dz * d[0] * d[1] + dy * d[0] - 1):
+                      np.searchsorted(slin, lin[i] + dz * d[0] * d[1] + dy * d[0] + 1, "right")]
+                for dz in (-1, 0, 1) for dy in (-1, 0, 1)]
+        cand = np.concatenate(cand)
+        cand = cand[cand != i]
+        e = p[i] - p[cand]
+        l2 = (e[:, 0] * e[:, 0] + e[:, 1] * e[:, 1]) + e[:, 2] * e[:, 2]
+        assert np.array_equal(idx[off[i]:off[i + 1]], cand[l2 < rf * rf]), i
+
+
 def test_neighbors_capacity_error(bnn):
     pts = scenes.point_cloud(5_000, seed=2)
     L = bnn.load()
