@@ -26,11 +26,21 @@
 // inside the few tiles that hold the floor.  A block has one thread per cell of its tile
 // and the tile's 1-cell halo (warps are rows of 32 cells along x: 30 interior columns and a
 // halo cell each side).  For each cell layer it needs, every thread forms its cell's
-// partials into shared memory, one component at a time, then the interior threads add the
-// partials their faces need to register accumulators for the three face layers the cell
-// layer reaches.  Each particle record is therefore read once per block (plus the halo)
-// instead of once per candidate face, the weight of a particle is formed once per reached
-// slot, and no thread forms two cells' partials while the rest of the block waits.
+// partials into shared memory, then the interior threads add the partials their faces need to
+// register accumulators for the three face layers the cell layer reaches.  Each particle
+// record is therefore read once per block (plus the halo) instead of once per candidate face,
+// the weight of a particle is formed once per reached slot, and no thread forms two cells'
+// partials while the rest of the block waits.
+//
+// The four passes (u, v, w, fluid SDF) are blocks of their own: each reads its own record
+// plane, so nothing but the cell offsets is read again, and a tile's passes run side by side
+// instead of one after another.  A pass is bound by the latency of its cells' record loads
+// and, where cells are crowded, by the serial sum over a cell's particles; one after another in
+// a block they took, with a small scene's few tiles leaving most of the GPU idle, ms per
+// sub-step: 64^3 FLIP 0.128 (now 0.055), 121 x 77 x 95 APIC 0.415 (0.148), 96^3 AFLIP 0.509
+// (0.19), 160 x 192 x 128 FLIP 0.384 (0.275), 256^3 FLIP 0.974 (0.773); a batch of 24 scenes, 30
+// steps, 206 -> 169.
+//
 //
 // Input: one 16-byte record per particle and component, written by the sort's gather
 // (flip_kernels.cu, k_gather_particles): plane D < 3 holds {e_x, e_y, e_z, v_D}, e_a the
@@ -64,7 +74,10 @@ struct Shape {
     static constexpr int kYC = YC;             // face layers per block along y (the walk)
     static constexpr int kNH = kHX * kHZ;      // cells of one layer whose partials the tile needs
     static constexpr int kThreads = kNH;
-    static constexpr int kMinBlocks = 768 / kThreads > 0 ? 768 / kThreads : 1;
+    // resident threads per SM: 1024 of 64 registers (256^3 0.81 ms against 0.84 at 768 of 80,
+    // 80^3 0.068 against 0.079); the affine term and the batch's scene lookup want 80 (121 x 77 x
+    // 95 APIC 0.15 ms against 0.27 with the spills of 64)
+    static constexpr int min_blocks(int threads) { return threads / kThreads > 0 ? threads / kThreads : 1; }
     static constexpr size_t kSmemBytes = sizeof(float) * kPartials * kNH;
 };
 // The shapes the tuner chooses from (index = bnn tile-shape id); 0 is the default
@@ -342,27 +355,35 @@ __device__ __forceinline__ void write_phi(const TileArgs& a, int fx, int fy, int
 }
 } // namespace
 
-// P2G: the three face components and the fluid SDF (FLIP); otherwise the fluid SDF alone.
-// Which tile a block works on: its own launch's block index, or one given to it (a scene's
-// tile in a batched launch).  Reading blockIdx keeps the indices out of registers.
-struct OwnTile {
-    __device__ __forceinline__ unsigned x() const { return blockIdx.x; }
+// P2G: the three face components and the fluid SDF; otherwise the fluid SDF alone.
+// Which tile and pass (0 u, 1 v, 2 w, 3 SDF) a block works on: its own launch's block index,
+// or one given to it (a scene's tile in a batched launch).  Reading blockIdx keeps the indices
+// out of registers.
+constexpr int kPasses = 4;
+template<bool P2G> struct OwnTile {
+    __device__ __forceinline__ unsigned pass() const { return P2G ? blockIdx.x % kPasses : 3u; }
+    __device__ __forceinline__ unsigned x() const { return P2G ? blockIdx.x / kPasses : blockIdx.x; }
     __device__ __forceinline__ unsigned z() const { return blockIdx.y; }
     __device__ __forceinline__ unsigned y() const { return blockIdx.z; }
 };
 struct GivenTile {
-    unsigned bx, bz, by;
+    unsigned bp, bx, bz, by;
+    __device__ __forceinline__ unsigned pass() const { return bp; }
     __device__ __forceinline__ unsigned x() const { return bx; }
     __device__ __forceinline__ unsigned z() const { return bz; }
     __device__ __forceinline__ unsigned y() const { return by; }
 };
 
-// One block of the pass: tile (x, z) of face columns, y-chunk y.  EXACT: some particle
+// One block of the pass PASS: tile (x, z) of face columns, y-chunk y.  EXACT: some particle
 // left the grid (the same for the whole launch; see sdf_partials).  AFF: APIC / AFLIP
 // momentum (cell_partials).
-template<bool P2G, class SH, bool EXACT, bool AFF = false, class Tile>
-__device__ __forceinline__ void tile_body(const TileArgs& a, const Tile tile) {
+template<int PASS, class SH, bool EXACT, bool AFF, class Tile>
+__device__ __forceinline__ void pass_body(const TileArgs& a, const Tile tile) {
     constexpr int kTZ = SH::kTZ, kYC = SH::kYC;
+    constexpr bool SDF = PASS == 3;
+    // the cell layer that completes face / cell layer y: y + 1, but y itself for v, whose faces
+    // have the walk's axis
+    constexpr int kLag = PASS == 1 ? 0 : 1;
     extern __shared__ float sm[];
     const GridDesc& g = a.g;
     const int t = threadIdx.y * kHX + threadIdx.x;        // this thread's halo cell
@@ -371,71 +392,63 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const Tile tile) {
     const int x0 = (int)tile.x() * kTX, z0 = (int)tile.z() * kTZ;
     const int yA = (int)tile.y() * kYC, yB = min(yA + kYC, g.G[1] + 1);  // face layers [yA, yB)
     const int fx = owner ? x0 + tx : INT_MAX, fz = owner ? z0 + tz : INT_MAX;
+    const float inf = __int_as_float(0x7f800000);
     {
         const int lo[3] = {x0 - 1, yA - 1, z0 - 1}, hi[3] = {x0 + kTX, yB, z0 + kTZ};
         if(!meets_particles(a.st, lo, hi)) {
             // no particle reaches the tile: empty faces and cells
             for(int fy = yA; fy < yB; ++fy) {
-                if constexpr(P2G) {
-                    write_face<0>(a, fx, fy, fz, 0.0f, 0.0f);
-                    write_face<1>(a, fx, fy, fz, 0.0f, 0.0f);
-                    write_face<2>(a, fx, fy, fz, 0.0f, 0.0f);
-                }
-                write_phi(a, fx, fy, fz, __int_as_float(0x7f800000));
+                if constexpr(SDF) write_phi(a, fx, fy, fz, inf);
+                else write_face<PASS>(a, fx, fy, fz, 0.0f, 0.0f);
             }
             return;
         }
     }
-    const float inf = __int_as_float(0x7f800000);
-    // accumulators of face layers cy - 1 + j (v, whose own axis is the walk, uses j = 1, 2)
-    float uS[3] = {0.f, 0.f, 0.f}, uW[3] = {0.f, 0.f, 0.f};
-    float vS[3] = {0.f, 0.f, 0.f}, vW[3] = {0.f, 0.f, 0.f};
-    float wS[3] = {0.f, 0.f, 0.f}, wW[3] = {0.f, 0.f, 0.f};
-    float aM[3] = {inf, inf, inf};
-    for(int cy = yA - 1; cy <= yB; ++cy) {
+    // accumulators of layers cy - 1 + j (v uses j = 1, 2): momentum and weight, or the minimum
+    const float none = SDF ? inf : 0.0f;
+    float aS[3] = {none, none, none}, aW[3] = {0.f, 0.f, 0.f};
+    const int cEnd = min(yB - 1 + kLag, g.G[1] - 1);
+    uint32_t pb = 0u, pe = 0u;
+    if(yA > 0) cell_range(a, x0, z0, yA - 1, t, pb, pe);
+    for(int cy = yA - 1; cy <= yB - 1 + kLag; ++cy) {
+        // the next layer's particle range, on its way while this layer is summed
+        uint32_t nb = 0u, ne = 0u;
+        if(cy + 1 <= cEnd) cell_range(a, x0, z0, cy + 1, t, nb, ne);
         if(cy >= 0 && cy < g.G[1]) {
-            uint32_t pb, pe;
-            cell_range(a, x0, z0, cy, t, pb, pe);
-            if constexpr(P2G) {
-                cell_partials<0, SH, AFF>(a, t, pb, pe, sm, x0, z0, cy);
-                __syncthreads();
-                if(owner) pull_partials<0, SH>(sm, tx, tz, uS, uW);
-                __syncthreads();
-                if(cy < yB) {
-                    cell_partials<1, SH, AFF>(a, t, pb, pe, sm, x0, z0, cy);
-                    __syncthreads();
-                    if(owner) pull_partials<1, SH>(sm, tx, tz, vS, vW);
-                    __syncthreads();
-                }
-                cell_partials<2, SH, AFF>(a, t, pb, pe, sm, x0, z0, cy);
-                __syncthreads();
-                if(owner) pull_partials<2, SH>(sm, tx, tz, wS, wW);
-                __syncthreads();
-            }
-            sdf_partials<SH, EXACT>(a, x0, z0, cy, t, pb, pe, sm);
+            if constexpr(SDF) sdf_partials<SH, EXACT>(a, x0, z0, cy, t, pb, pe, sm);
+            else cell_partials<PASS, SH, AFF>(a, t, pb, pe, sm, x0, z0, cy);
+            // the first line of the next layer's records: the one load the serial sum cannot
+            // issue ahead (256^3 0.81 -> 0.77 ms)
+            if(nb < ne) asm volatile("prefetch.global.L1 [%0];" : : "l"(a.rec + (size_t)PASS * a.stride + nb));
             __syncthreads();
-            if(owner) pull_sdf<SH>(sm, tx, tz, aM);
+            if(owner) {
+                if constexpr(SDF) pull_sdf<SH>(sm, tx, tz, aS);
+                else pull_partials<PASS, SH>(sm, tx, tz, aS, aW);
+            }
             __syncthreads();
         }
-        // face / cell layer cy - 1 is complete for u, w and the SDF, face layer cy for v
-        if(cy - 1 >= yA && cy - 1 < yB) {
-            if constexpr(P2G) {
-                write_face<0>(a, fx, cy - 1, fz, uS[0], uW[0]);
-                write_face<2>(a, fx, cy - 1, fz, wS[0], wW[0]);
-            }
-            write_phi(a, fx, cy - 1, fz, aM[0]);
+        pb = nb;
+        pe = ne;
+        const int fy = cy - kLag;
+        if(fy >= yA) {
+            if constexpr(SDF) write_phi(a, fx, fy, fz, aS[0]);
+            else write_face<PASS>(a, fx, fy, fz, aS[1 - kLag], aW[1 - kLag]);
         }
-        if constexpr(P2G) {
-            if(cy >= yA && cy < yB) write_face<1>(a, fx, cy, fz, vS[1], vW[1]);
-        }
-        uS[0] = uS[1]; uS[1] = uS[2]; uS[2] = 0.f;
-        uW[0] = uW[1]; uW[1] = uW[2]; uW[2] = 0.f;
-        wS[0] = wS[1]; wS[1] = wS[2]; wS[2] = 0.f;
-        wW[0] = wW[1]; wW[1] = wW[2]; wW[2] = 0.f;
-        vS[1] = vS[2]; vS[2] = 0.f;
-        vW[1] = vW[2]; vW[2] = 0.f;
-        aM[0] = aM[1]; aM[1] = aM[2]; aM[2] = inf;
+        aS[0] = aS[1]; aS[1] = aS[2]; aS[2] = none;
+        aW[0] = aW[1]; aW[1] = aW[2]; aW[2] = 0.f;
     }
+}
+template<bool P2G, class SH, bool EXACT, bool AFF = false, class Tile>
+__device__ __forceinline__ void tile_body(const TileArgs& a, const Tile tile) {
+    if constexpr(P2G) {
+        switch(tile.pass()) {
+        case 0: pass_body<0, SH, EXACT, AFF>(a, tile); return;
+        case 1: pass_body<1, SH, EXACT, AFF>(a, tile); return;
+        case 2: pass_body<2, SH, EXACT, AFF>(a, tile); return;
+        default: break;
+        }
+    }
+    pass_body<3, SH, EXACT, AFF>(a, tile);
 }
 // The rare launch in which some particle left the grid, kept out of line so that its
 // per-slot tests do not weigh on the registers of the common path
@@ -444,29 +457,30 @@ __device__ __noinline__ void tile_body_exact(const TileArgs& a, const Tile tile)
     tile_body<P2G, SH, true, AFF>(a, tile);
 }
 template<bool P2G, class SH, bool AFF = false>
-__global__ void __launch_bounds__(SH::kThreads, SH::kMinBlocks) k_p2g_sdf_tile(const __grid_constant__ TileArgs a) {
-    if((a.st->flags & BNN_FLAG_OUT_OF_GRID) != 0u) tile_body_exact<P2G, SH, AFF>(a, OwnTile{});
-    else tile_body<P2G, SH, false, AFF>(a, OwnTile{});
+__global__ void __launch_bounds__(SH::kThreads, SH::min_blocks(AFF ? 768 : 1024)) k_p2g_sdf_tile(const __grid_constant__ TileArgs a) {
+    if((a.st->flags & BNN_FLAG_OUT_OF_GRID) != 0u) tile_body_exact<P2G, SH, AFF>(a, OwnTile<P2G>{});
+    else tile_body<P2G, SH, false, AFF>(a, OwnTile<P2G>{});
 }
 
 // Batched: the tiles of all scenes of a batch in one launch (P: per-scene tile prefix);
-// a block's flat tile index within its scene maps to (x, z, y) as in tile_grid
+// a block's flat index within its scene maps to (pass, x, z, y) as in tile_grid
 template<class SH>
-__global__ void __launch_bounds__(SH::kThreads, SH::kMinBlocks) kb_p2g_sdf_tile(const TileArgs* __restrict__ A,
+__global__ void __launch_bounds__(SH::kThreads, SH::min_blocks(768)) kb_p2g_sdf_tile(const TileArgs* __restrict__ A,
                                                                             const unsigned* __restrict__ P, int ns) {
     int q;
     const Blk b = seg_blk(P, ns, q);
     const TileArgs& a = A[q];
     const unsigned gx = (unsigned)((a.g.G[0] + 1 + kTX - 1) / kTX);
     const unsigned gz = (unsigned)((a.g.G[2] + 1 + SH::kTZ - 1) / SH::kTZ);
-    const GivenTile tile{b.x % gx, (b.x / gx) % gz, b.x / (gx * gz)};
+    const unsigned f = b.x / kPasses;
+    const GivenTile tile{b.x % kPasses, f % gx, (f / gx) % gz, f / (gx * gz)};
     if((a.st->flags & BNN_FLAG_OUT_OF_GRID) != 0u) tile_body_exact<true, SH, false>(a, tile);  // the scene's flag
     else tile_body<true, SH, false, false>(a, tile);
 }
 static_assert(kHX == 32, "a warp is one row of halo cells");
 
-template<class SH> static dim3 tile_grid_of(const GridDesc& g) {
-    return dim3((unsigned)((g.G[0] + 1 + kTX - 1) / kTX), (unsigned)((g.G[2] + 1 + SH::kTZ - 1) / SH::kTZ),
+template<class SH, bool P2G = true> static dim3 tile_grid_of(const GridDesc& g) {
+    return dim3((unsigned)((g.G[0] + 1 + kTX - 1) / kTX) * (P2G ? kPasses : 1), (unsigned)((g.G[2] + 1 + SH::kTZ - 1) / SH::kTZ),
                 (unsigned)((g.G[1] + 1 + SH::kYC - 1) / SH::kYC));
 }
 
@@ -483,7 +497,7 @@ template<class K> static void opt_in_smem(K* kern, size_t bytes, std::atomic<uin
 template<bool P2G, class SH> static void launch_tile_sh(const TileArgs& a, cudaStream_t s) {
     static std::atomic<uint64_t> configured{0};
     opt_in_smem(k_p2g_sdf_tile<P2G, SH>, SH::kSmemBytes, configured);
-    k_p2g_sdf_tile<P2G, SH><<<tile_grid_of<SH>(a.g), dim3(kHX, SH::kHZ), SH::kSmemBytes, s>>>(a);
+    k_p2g_sdf_tile<P2G, SH><<<tile_grid_of<SH, P2G>(a.g), dim3(kHX, SH::kHZ), SH::kSmemBytes, s>>>(a);
     bnn_note_launch();
 }
 template<class SH>
