@@ -350,8 +350,10 @@ int batch_substep(BatchStepWork& w, bnn_flip* const* hs, int nsIn, int* rc, bnn_
         it.innerTol = h->P.refine_inner_tolerance;
         it.outerTol = h->P.refine_tolerance;
         it.maxIter = h->P.max_cg_iteration;
+        it.layout = row_layout(h->g.G[0], (long long)h->g.G[0] * h->g.G[1]);
         it.pressure = h->pressure;
         it.dst = h->dst;
+        it.hst = h->hst;
     }
     BNN_CUDA_CHECK(cudaMemcpyAsync(D, H, L.up, cudaMemcpyHostToDevice, s));
     launch_batch_stage(BatchStage::ActiveRows, dS, dP(PCells), ns, tot(PCells), s);

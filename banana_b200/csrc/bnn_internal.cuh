@@ -414,15 +414,15 @@ struct BatchSolveItem {
     const int32_t* nbr;
     float dt, innerTol, outerTol;
     unsigned maxIter;
+    RowLayout layout;
     float* pressure;
-    DevState* dst;
+    DevState *dst, *hst;
     PcgOutcome out;
 };
 // Device tables of the batched solve, kept between calls (grown on demand)
 struct BatchPcgCtx {
-    int cap = 0;
-    size_t upBytes = 0, blobBytes = 0;
-    void* dev = nullptr;       // device tables, reports, barrier
+    int cap = 0, capGroups = 0;
+    void* dev = nullptr;       // device tables and reports
     void* host = nullptr;      // pinned mirror of the uploaded part, then the reports
     cudaEvent_t ev[2] = {nullptr, nullptr};
 };

@@ -23,6 +23,7 @@
 //   grid barrier; every block reduces to the same rho, max|r| and beta.
 #include "bnn_internal.cuh"
 
+#include <algorithm>
 #include <condition_variable>
 #include <cstdio>
 #include <cstring>
@@ -755,6 +756,30 @@ __device__ __forceinline__ bool packet_poll(const PcgPacket* slot, bool on, unsi
     }
 }
 
+// One warp: the packets of up to 32 chunks, their canonical sum and max (valid in lane 0);
+// false when the wait gave up
+template<class VT, bool MAX, bool ACQUIRE>
+__device__ __forceinline__ bool warp_packets(const PcgPacket* slots, int nch, unsigned parity, double& sum, VT& mx) {
+    const int t = threadIdx.x & 31;
+    PcgPacket pk;
+    const bool ok = packet_poll<ACQUIRE>(slots + (size_t)t * kPacketStride, t < nch, parity, pk);
+    double c = 0.0;
+    VT m = VT(0);
+    if(t < nch) {
+        c = c + __longlong_as_double((long long)pk.sum);
+        if(MAX) { const VT o = max_of<VT>(pk.max); m = m > o ? m : o; }
+    }
+#pragma unroll
+    for(int off = 16; off > 0; off >>= 1) {
+        if(off >= nch) continue;  // the tree's other half holds no chunk: +0
+        c = c + __shfl_down_sync(0xffffffffu, c, off);
+        if(MAX) { const VT o = __shfl_down_sync(0xffffffffu, m, off); m = m > o ? m : o; }
+    }
+    sum = c;
+    mx = m;
+    return ok;
+}
+
 // Second half of an exchange: waits for every chunk's packet of this parity and gives the
 // canonical sum and max (as reduce_partials_bcast) to every thread of the block.  Up to 32
 // chunks are polled by warp 0, which then needs no shared memory for their sum; more by all
@@ -804,23 +829,58 @@ __device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, uns
             if(t == 0) { W.sum = c; W.max = x; }
         }
     } else if(t < 32) {
-        PcgPacket pk;
-        if(!packet_poll<ACQUIRE>(slots + (size_t)t * kPacketStride, t < nch, parity, pk)) W.bad = 1;
-        double c = 0.0;
-        VT m = VT(0);
-        if(t < nch) {
-            c = c + __longlong_as_double((long long)pk.sum);
-            if(MAX) { const VT o = max_of<VT>(pk.max); m = m > o ? m : o; }
-        }
-#pragma unroll
-        for(int off = 16; off > 0; off >>= 1) {
-            if(off >= nch) continue;  // the tree's other half holds no chunk: +0
-            c = c + __shfl_down_sync(0xffffffffu, c, off);
-            if(MAX) { const VT o = __shfl_down_sync(0xffffffffu, m, off); m = m > o ? m : o; }
-        }
+        double c;
+        VT m;
+        if(!warp_packets<VT, MAX, ACQUIRE>(slots, nch, parity, c, m)) W.bad = 1;
         if(t == 0) { W.sum = c; W.max = m; }
     }
     __syncthreads();
+    sum = W.sum;
+    mx = W.max;
+    if(W.bad == 0) return true;
+    if(t == 0) atomicOr(flags, BNN_FLAG_TIMEOUT);
+    return false;
+}
+
+// packet_wait for one group on its own (a scene of a batch): the group polls its scene's
+// packets, and no other group waits for it
+template<class VT> struct GroupWaitSmem {
+    double lanes[kLanes];
+    VT lanesMax[kLanes];
+    double sum;
+    VT max;
+    int bad;
+};
+template<class VT, bool MAX, bool ACQUIRE>
+__device__ __forceinline__ bool group_wait(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
+                                           GroupWaitSmem<VT>& W, int grp, int t, double& sum, VT& mx) {
+    if(nch > kWarpPackets) {
+        double acc = 0.0;
+        VT m = VT(0);
+        for(int c = t; c < ((nch + 31) & ~31); c += kLanes) {
+            PcgPacket pk;
+            if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad = 1; break; }
+            if(c < nch) {
+                acc = acc + __longlong_as_double((long long)pk.sum);
+                if(MAX) { const VT o = max_of<VT>(pk.max); m = m > o ? m : o; }
+            }
+        }
+        W.lanes[t] = acc;
+        if(MAX) W.lanesMax[t] = m;
+        group_sync(grp);
+        if(t < 32) {
+            double c;
+            VT x;
+            lane_tree<VT, MAX>(W.lanes, W.lanesMax, c, x);
+            if(t == 0) { W.sum = c; W.max = x; }
+        }
+    } else if(t < 32) {
+        double c;
+        VT m;
+        if(!warp_packets<VT, MAX, ACQUIRE>(slots, nch, parity, c, m)) W.bad = 1;
+        if(t == 0) { W.sum = c; W.max = m; }
+    }
+    group_sync(grp);
     sum = W.sum;
     mx = W.max;
     if(W.bad == 0) return true;
@@ -861,7 +921,7 @@ __device__ __forceinline__ unsigned row_code(int dz, int l, int dy, int sign, bo
 // Shared memory of a block: CH chunks.  x and 1/diag are kept there too where they fit (else
 // x stays in global memory and 1/diag is loaded ahead of every iteration's first exchange).
 template<class VT> constexpr int kRoomy = sizeof(VT) == 4 ? 3 : 2;
-template<class VT, bool COEF, int CH> struct ChunkSmem {
+template<class VT, bool COEF, int CH> struct ChunkRowsSmem {
     static constexpr int kX = CH <= kRoomy<VT> ? CH : 1, kXRows = CH <= kRoomy<VT> ? kChunk : 1;
     VT s[CH][kChunk + 16 / sizeof(VT)];  // s[kNoRow] = 0: what a missing neighbour adds
     uint2 nb[CH][kChunk];
@@ -870,28 +930,42 @@ template<class VT, bool COEF, int CH> struct ChunkSmem {
     float co[COEF ? CH : 1][COEF ? 6 : 1][COEF ? kChunk : 1];
     double sum[CH][kLanes];
     VT max[CH][kLanes];
-    WaitSmem<VT, CH> wait;
+};
+template<class VT, bool COEF, int G, int K> struct ChunkSmem : ChunkRowsSmem<VT, COEF, G * K> {
+    WaitSmem<VT, G * K> wait;
+};
+// A batch's block: every group solves for a scene of its own
+template<class VT, int G, int K> struct BatchChunkSmem : ChunkRowsSmem<VT, false, G * K> {
+    GroupWaitSmem<VT> wait[G];
+    ChunkArgs<VT> args[G];
 };
 
-template<class VT, bool COEF, int G, int K>
-__global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
+// The solve of the K chunks c0, c0 + cStep, ... by group grp of a block of G groups.  BATCH:
+// the group is one of a scene's, and waits and returns by itself; else all groups of the block
+// belong to one system and wait together.
+template<class VT, bool COEF, int G, int K, bool BATCH, class Smem>
+__device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, const int grp, const int t, const int c0,
+                                            const int cStep) {
     // rows whose neighbour loads are in flight together
     constexpr int kGroup = sizeof(VT) == 4 ? (G == 1 ? 8 : 4) : (G == 1 ? 4 : 2);
     constexpr int R = K * kPerLane;
     constexpr bool kHere = G * K <= kRoomy<VT>;  // x and 1/diag in shared memory
-    extern __shared__ __align__(16) unsigned char dynSm[];
-    ChunkSmem<VT, COEF, G * K>& S = *reinterpret_cast<ChunkSmem<VT, COEF, G * K>*>(dynSm);
-    const int n = a.n, nch = a.nch, grp = (int)threadIdx.x / kLanes, t = (int)threadIdx.x % kLanes;
+    const int n = a.n, nch = a.nch;
     unsigned* flags = &a.st->flags;
     RowPair<VT>* __restrict__ pair = a.pair;
     const VT negoff = a.negoff;
-    // this group's chunks: slots grp * K + k of the block, striped over the grid so that the
-    // blocks' counts differ by one at most
-    auto chunk_of = [&](int k) { return (int)blockIdx.x + (grp * K + k) * (int)gridDim.x; };
+    auto chunk_of = [&](int k) { return c0 + k * cStep; };
     auto rows_of = [&](int k) { return max(min(n - chunk_of(k) * kChunk, kChunk), 0); };
+    auto wait = [&](auto withMax, auto acquire, const PcgPacket* slots, unsigned parity, double& sum, VT& mx) {
+        constexpr bool MAX = decltype(withMax)::value, ACQUIRE = decltype(acquire)::value;
+        if constexpr(BATCH) return group_wait<VT, MAX, ACQUIRE>(slots, nch, parity, flags, S.wait[grp], grp, t, sum, mx);
+        else return packet_wait<VT, MAX, ACQUIRE, G * K>(slots, nch, parity, flags, S.wait, sum, mx);
+    };
 
     // ---- init: r = rhs, x = 0, z = D^-1 r; partial z.r and max|r| (PCGSolver.cpp:151-168)
-    if(threadIdx.x == 0) S.wait.bad = 0;
+    if constexpr(BATCH) {
+        if(t == 0) S.wait[grp].bad = 0;
+    } else if(threadIdx.x == 0) S.wait.bad = 0;
     VT r[R], q[R];  // q holds z from phase B to the next phase A
 #pragma unroll
     for(int k = 0; k < K; ++k) {
@@ -942,7 +1016,8 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
         S.sum[slot][t] = acc;
         S.max[slot][t] = m;
     }
-    __syncthreads();
+    if constexpr(BATCH) group_sync(grp);
+    else __syncthreads();
     double rho;
     VT resid;
     unsigned parity = 1;  // of this iteration's exchanges
@@ -956,7 +1031,7 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
         }
     };
     publish(Yes(), Yes(), a.pkB);
-    if(!packet_wait<VT, true, true>(a.pkB, nch, parity, flags, S.wait, rho, resid)) return;
+    if(!wait(Yes(), Yes(), a.pkB, parity, rho, resid)) return;
     const VT tolFactor = fmax(a.tolFactor, VT(1e-30));
     unsigned iter = 0, success = 0;
     bool done = false;
@@ -1067,7 +1142,7 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
                 }
         double tmp;
         VT unused;
-        if(!packet_wait<VT, false, false>(a.pkA, nch, parity, flags, S.wait, tmp, unused)) return;
+        if(!wait(No(), No(), a.pkA, parity, tmp, unused)) return;
         if(tmp < (double)FLT_MIN) {
             ++iter;
             success = 1;
@@ -1119,7 +1194,7 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
             }
         }
         double rhoNew;
-        if(!packet_wait<VT, true, true>(a.pkB, nch, parity, flags, S.wait, rhoNew, resid)) return;
+        if(!wait(Yes(), Yes(), a.pkB, parity, rhoNew, resid)) return;
         ++iter;
         if(resid < tol) {
             success = 1;
@@ -1128,7 +1203,7 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
         beta = (VT)(rhoNew / rho);
         rho = rhoNew;
         if(iter >= a.maxIter) {
-            if(blockIdx.x == 0 && threadIdx.x == 0) atomicOr(flags, BNN_FLAG_PCG_MAXITER);
+            if(chunk_of(0) == 0 && t == 0) atomicOr(flags, BNN_FLAG_PCG_MAXITER);
             break;
         }
     }
@@ -1140,12 +1215,43 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
                 const int l = t + j * kLanes;
                 if(l < rows_of(k)) a.x[(size_t)chunk_of(k) * kChunk + l] = S.x[grp * K + k][l];
             }
-    if(blockIdx.x == 0 && threadIdx.x == 0) {
+    if(chunk_of(0) == 0 && t == 0) {
         a.st->iter = iter;
         a.st->success = success;
         a.st->done = 1;
         Sc<VT>::set_resid(a.st, resid);
     }
+}
+
+// A lone system: the chunks are striped over the grid's groups, so that the blocks' counts
+// differ by one at most
+template<class VT, bool COEF, int G, int K>
+__global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
+    extern __shared__ __align__(16) unsigned char dynSm[];
+    auto& S = *reinterpret_cast<ChunkSmem<VT, COEF, G, K>*>(dynSm);
+    const int grp = (int)threadIdx.x / kLanes, t = (int)threadIdx.x % kLanes;
+    chunk_solve<VT, COEF, G, K, false>(a, S, grp, t, (int)(blockIdx.x + grp * K * gridDim.x), (int)gridDim.x);
+}
+
+// The FP32 systems of many scenes in one launch (BatchGroup: which chunks a group of 256
+// threads owns).  A scene's groups exchange with one another alone, so a scene iterates at the
+// pace of its own chunks and its groups end when it has converged; all groups of the launch
+// are resident.  Every scene gets the scalars, iterates and iteration count of a lone solve.
+struct BatchGroup {
+    int scene;   // -1: no work
+    int chunk0;  // its first chunk; the K of a group follow one another
+};
+template<int G, int K>
+__global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk_batch(const ChunkArgs<float>* __restrict__ scenes,
+                                                                   const BatchGroup* __restrict__ groups) {
+    extern __shared__ __align__(16) unsigned char dynSm[];
+    auto& S = *reinterpret_cast<BatchChunkSmem<float, G, K>*>(dynSm);
+    const int grp = (int)threadIdx.x / kLanes, t = (int)threadIdx.x % kLanes;
+    const BatchGroup g = groups[blockIdx.x * G + grp];
+    if(g.scene < 0) return;
+    if(t == 0) S.args[grp] = scenes[g.scene];
+    group_sync(grp);
+    chunk_solve<float, false, G, K, true>(S.args[grp], S, grp, t, g.chunk0, 1);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1544,424 +1650,6 @@ __global__ void __launch_bounds__(kLanes, cg1_min_blocks<VT>()) k_pcg_cg1(Cg1Arg
     }
 }
 
-// ---------------------------------------------------------------------------------
-// Batched persistent PCG: the Jacobi systems of many scenes (FP32 vectors, grid rows in
-// packed records, face weights 1) in one cooperative launch.  A scene's rows are cut into
-// the same 2048-row chunks as in a lone solve, and the chunks of all scenes are numbered
-// one after another and striped over the blocks (block b takes chunks b, b + grid, ...),
-// so as scenes finish the chunks of those still iterating stay spread over the whole grid
-// and every block keeps its share of the remaining work.  After each grid barrier a block
-// reduces the partials of each scene it works on, a warp per scene
-// (warp_reduce_partials: the canonical order over that scene's chunks alone), so every
-// scene gets exactly the scalars, iterates and iteration count of a lone
-// k_pcg_persistent solve.  Scenes that have finished skip their chunks; the loop ends, for
-// all blocks at the same barrier, when a counter of unfinished scenes (decremented by the
-// block owning a scene's first chunk) reads 0 right after the first barrier of an
-// iteration -- no scene can finish between the last decrement before that barrier and the
-// read.
-// Yield: a second counter holds the chunks of the unfinished scenes.  When it has fallen to
-// yieldBelow (read at the same point), every block leaves at the end of that iteration and
-// the owner of each unfinished scene saves its scalars (iterations, rho, beta, tol, last
-// residual) to the scene's DevState; the host launches the unfinished scenes again with
-// resume set, spread over the whole grid, and they carry on with exactly the iterates they
-// had.  Which of the s buffers is the new one follows from the iteration count (even: s0).
-// ---------------------------------------------------------------------------------
-constexpr int kBatchSlots = 64;  // scenes a block's chunks may belong to
-
-// reduce_partials_bcast's result (the canonical sum over nch chunk partials and their max)
-// formed by one warp: lane t stands for the block's threads t, t + 32, ..., t + 224 (the
-// threads of block_sum_max_256's first level that lane t of warp 0 combines), each summing
-// its partials t', t' + 256, ... in order, then the same association and shuffle tree.
-// The result is valid in lane 0.
-__device__ __forceinline__ void warp_reduce_partials(const double* part, const float* pmax, int nch, double& sum,
-                                                     float& mx) {
-    const int lane = threadIdx.x & 31;
-    double acc[8];
-    float m[8];
-#pragma unroll
-    for(int v = 0; v < 8; ++v) {
-        acc[v] = 0.0;
-        m[v] = 0.f;
-        for(int c = lane + 32 * v; c < nch; c += kLanes) {
-            acc[v] = acc[v] + __ldcg(part + c);
-            if(pmax) {
-                const float o = __ldcg(pmax + c);
-                m[v] = m[v] > o ? m[v] : o;
-            }
-        }
-    }
-    // virtual threads lane + 32 v: level 128 pairs v with v + 4, level 64 v = 0/2 with 4/6 ...
-    const double a0 = acc[0] + acc[4];
-    const double a1 = acc[2] + acc[6];
-    const double a2 = acc[1] + acc[5];
-    const double a3 = acc[3] + acc[7];
-    double c = (a0 + a1) + (a2 + a3);
-#pragma unroll
-    for(int off = 16; off > 0; off >>= 1) c = c + __shfl_down_sync(0xffffffffu, c, off);
-    float x = 0.f;
-    if(pmax) {
-        x = m[0];
-#pragma unroll
-        for(int q = 1; q < 8; ++q) { const float o = m[q]; x = x > o ? x : o; }
-#pragma unroll
-        for(int off = 16; off > 0; off >>= 1) { const float o = __shfl_down_sync(0xffffffffu, x, off); x = x > o ? x : o; }
-    }
-    sum = c;
-    mx = x;
-}
-struct BatchPcgScene {
-    int n;                     // rows
-    int resume;                // carry on from the scalars saved at a yield
-    const float* rhsF;
-    const float* invd;
-    const int4* rec;
-    float negoff;              // -(1 * dt)
-    float tolFactor;
-    unsigned maxIter;
-    float *x, *r, *z, *s0, *s1, *q;
-    double *part0, *part1, *part2;
-    float* partMax;
-    DevState* dst;             // iterations, success and residual go here
-};
-struct BatchPcgArgs {
-    const BatchPcgScene* sc;
-    const unsigned* cp;        // chunk prefix over scenes (ns + 1)
-    int ns;
-    unsigned total;            // chunks of all scenes
-    unsigned perBlock;         // chunks per block
-    GridSync* gs;
-    unsigned* remaining;       // unfinished scenes
-    unsigned* active;          // chunks of the unfinished scenes
-    unsigned yieldBelow;       // leave when active has fallen to this (0: never)
-    unsigned* flags;           // BNN_FLAG_TIMEOUT
-};
-
-__global__ void __launch_bounds__(kLanes, pcg_min_blocks<float, false>()) k_pcg_batch(BatchPcgArgs a) {
-    constexpr int kRowGroup = pcg_row_group<float, false>();
-    constexpr int kWarps = kLanes / 32;
-    __shared__ double smd[kLanes];
-    __shared__ float smv[kLanes];
-    __shared__ double sRho[kBatchSlots];
-    __shared__ float sTol[kBatchSlots], sResid[kBatchSlots], sAlpha[kBatchSlots], sBeta[kBatchSlots];
-    __shared__ unsigned sIter[kBatchSlots];
-    // 0 iterating, 1 finished, 2 no solve, 3 finished in this iteration's first half
-    // (counted off after the second barrier)
-    __shared__ int sState[kBatchSlots];
-    __shared__ int sScene[kBatchSlots];
-    __shared__ unsigned char sSlotOf[kBatchSlots];  // slot of the block's k-th chunk
-    __shared__ int sNslots;
-    const unsigned nb = gridDim.x;
-    unsigned sense = 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // The block's chunks are blockIdx.x + k nb (k < nmine): striped over the grid, so the
-    // chunks of the scenes still iterating stay spread over all blocks as others finish.
-    // Its slots are the scenes those chunks belong to, in order.
-    const unsigned nmine = blockIdx.x < a.total ? (a.total - 1 - blockIdx.x) / nb + 1 : 0u;
-    if(nmine > (unsigned)kBatchSlots) {  // the host keeps chunks per block within the slot table
-        if(threadIdx.x == 0) atomicOr(a.flags, BNN_FLAG_TIMEOUT);
-        return;
-    }
-    if(threadIdx.x == 0) {
-        int m = 0, last = -1;
-        for(unsigned k = 0; k < nmine; ++k) {
-            const int sc = seg_of(a.cp, a.ns, blockIdx.x + k * nb);
-            if(sc != last) { sScene[m++] = sc; last = sc; }
-            sSlotOf[k] = (unsigned char)(m - 1);
-        }
-        sNslots = m;
-    }
-    __syncthreads();
-    const int nslots = sNslots;
-    // the block owning a scene's first chunk reports its result and counts it off
-    auto owner = [&](int sc) { return __ldg(a.cp + sc) % nb == blockIdx.x; };
-    auto count_off = [&](int sc) {
-        atomicSub(a.remaining, 1u);
-        atomicSub(a.active, __ldg(a.cp + sc + 1) - __ldg(a.cp + sc));
-    };
-    // one thread: the scene of slot j is done (deferred: counted off after the second barrier)
-    auto finish1 = [&](int j, unsigned success, bool deferred) {
-        const int sc = sScene[j];
-        sState[j] = deferred ? 3 : 1;
-        if(owner(sc)) {
-            DevState* d = a.sc[sc].dst;
-            d->iter = sIter[j];
-            d->success = success;
-            d->done = 1;
-            d->resid = sResid[j];
-            d->resid64 = sResid[j];
-            if(!deferred) count_off(sc);
-        }
-    };
-    auto chunks_of = [&](int sc) { return (int)(__ldg(a.cp + sc + 1) - __ldg(a.cp + sc)); };
-
-    // ---- init: r = rhs, x = 0, z = D^-1 r; partial z.r and max|r| (not for a resumed scene)
-    for(unsigned k = 0; k < nmine; ++k) {
-        const unsigned c = blockIdx.x + k * nb;
-        const int sc = sScene[sSlotOf[k]];
-        const BatchPcgScene& S = a.sc[sc];
-        if(S.resume) continue;
-        const int n = S.n;
-        const unsigned lc = c - __ldg(a.cp + sc);
-        double acc = 0.0;
-        float m = 0.f;
-        const size_t base = (size_t)lc * kChunk + threadIdx.x;
-#pragma unroll
-        for(int j = 0; j < kPerLane; ++j) {
-            const size_t e = base + (size_t)j * kLanes;
-            if(e < (size_t)n) {
-                const float rv = S.rhsF[e];
-                S.r[e] = rv;
-                S.x[e] = 0.f;
-                const float ab = vabs(rv);
-                m = m > ab ? m : ab;
-                const float zv = __ldg(S.invd + e) * rv;
-                S.z[e] = zv;
-                acc = acc + (double)zv * (double)rv;
-            }
-        }
-        double bs;
-        float bm;
-        block_sum_max_256<float>(acc, m, smd, smv, bs, bm, true);
-        if(threadIdx.x == 0) { S.part0[lc] = bs; S.partMax[lc] = bm; }
-    }
-    if(!grid_barrier(a.gs, nb, sense, a.flags, solve_barrier_limit())) return;
-    // the scenes' first scalars, a warp per slot
-    for(int j = warp; j < nslots; j += kWarps) {
-        const int sc = sScene[j];
-        const BatchPcgScene& S = a.sc[sc];
-        const int nch = chunks_of(sc);
-        if(S.resume) {
-            // the scalars saved at the yield
-            if(lane == 0) {
-                const DevState* d = S.dst;
-                sIter[j] = d->iter; sRho[j] = d->rho; sBeta[j] = d->beta; sTol[j] = d->tol; sResid[j] = d->resid;
-                sState[j] = 0;
-            }
-            continue;
-        }
-        double rho = 0.0;
-        float resid = 0.f;
-        if(nch > 0) warp_reduce_partials(S.part0, S.partMax, nch, rho, resid);
-        if(lane == 0) {
-            sIter[j] = 0;
-            sState[j] = nch > 0 ? 0 : 2;
-            sBeta[j] = 0.f;
-            if(nch > 0) {
-                sRho[j] = rho;
-                sResid[j] = resid;
-                const float tolFactor = fmaxf(S.tolFactor, 1e-30f);
-                if(resid < FLT_MIN) {
-                    finish1(j, 1u, false);
-                } else {
-                    sTol[j] = tolFactor * resid;
-                    if(rho < (double)FLT_MIN || isnan(rho) || S.maxIter == 0) finish1(j, 0u, false);
-                }
-            }
-        }
-    }
-    __syncthreads();
-
-    // a scene's new s is s0 after an even number of iterations, as the lone solve's swap;
-    // its first iteration (no s yet) is the one with 0 iterations done
-    for(;;) {
-        // ---- phase A: s = z + beta s_old, q = A s, partial s.q
-        for(unsigned k = 0; k < nmine; ++k) {
-            const int jslot = sSlotOf[k];
-            if(sState[jslot] != 0) continue;
-            const unsigned c = blockIdx.x + k * nb;
-            const int sc = sScene[jslot];
-            const BatchPcgScene& S = a.sc[sc];
-            const int n = S.n;
-            const unsigned lc = c - __ldg(a.cp + sc);
-            const float beta = sBeta[jslot];
-            const float negoff = S.negoff;
-            const float* __restrict__ zR = S.z;
-            const bool parity = (sIter[jslot] & 1u) != 0;
-            const bool first = sIter[jslot] == 0;
-            const float* __restrict__ sOld = parity ? S.s0 : S.s1;
-            float* __restrict__ sNew = parity ? S.s1 : S.s0;
-            const size_t base = (size_t)lc * kChunk + threadIdx.x;
-            float sOut[kPerLane], qOut[kPerLane];
-            int4 recAll[kPerLane];
-#pragma unroll
-            for(int j = 0; j < kPerLane; ++j) {
-                const size_t e = base + (size_t)j * kLanes;
-                recAll[j] = __ldg(S.rec + (e < (size_t)n ? e : 0));
-            }
-#pragma unroll
-            for(int g0 = 0; g0 < kPerLane; g0 += kRowGroup) {
-                int32_t id[kRowGroup][7];
-                bool has[kRowGroup][7];
-                float dg[kRowGroup];
-#pragma unroll
-                for(int u = 0; u < kRowGroup; ++u) {
-                    const size_t e = base + (size_t)(g0 + u) * kLanes;
-                    const size_t ee = e < (size_t)n ? e : 0;
-                    const int4 rr = recAll[g0 + u];
-                    const int dyM = rr.x & 0xffff, dyP = (int)((unsigned)rr.x >> 16);
-                    const int dzM = rr.y & 0x7fffffff, dzP = rr.z & 0x7fffffff;
-                    const int32_t r0 = (int32_t)ee;
-                    has[u][0] = dzM != 0; id[u][0] = r0 - dzM;
-                    has[u][1] = dyM != 0; id[u][1] = r0 - dyM;
-                    has[u][2] = rr.y < 0; id[u][2] = (lane == 0 && rr.y < 0) ? r0 - 1 : r0;
-                    has[u][3] = true; id[u][3] = r0;
-                    has[u][4] = rr.z < 0; id[u][4] = (lane == 31 && rr.z < 0) ? r0 + 1 : r0;
-                    has[u][5] = dyP != 0; id[u][5] = r0 + dyP;
-                    has[u][6] = dzP != 0; id[u][6] = r0 + dzP;
-                    dg[u] = __int_as_float(rr.w);
-                }
-                float zv[kRowGroup][7], sv[kRowGroup][7];
-#pragma unroll
-                for(int u = 0; u < kRowGroup; ++u)
-#pragma unroll
-                    for(int q = 0; q < 7; ++q) {
-                        const bool load = (q != 2 && q != 4) || (q == 2 && lane == 0) || (q == 4 && lane == 31);
-                        zv[u][q] = load ? __ldcg(zR + id[u][q]) : 0.f;
-                        sv[u][q] = (first || !load) ? 0.f : __ldcg(sOld + id[u][q]);
-                    }
-#pragma unroll
-                for(int u = 0; u < kRowGroup; ++u) {
-                    float s7[7];
-#pragma unroll
-                    for(int q = 0; q < 7; ++q) s7[q] = first ? zv[u][q] : zv[u][q] + beta * sv[u][q];
-                    const float up = __shfl_up_sync(0xffffffffu, s7[3], 1);
-                    const float dn = __shfl_down_sync(0xffffffffu, s7[3], 1);
-                    if(lane != 0) s7[2] = up;
-                    if(lane != 31) s7[4] = dn;
-                    float t = 0.f;
-#pragma unroll
-                    for(int q = 0; q < 3; ++q) if(has[u][q]) t += negoff * s7[q];
-                    if(dg[u] != 0.f) t += dg[u] * s7[3];
-#pragma unroll
-                    for(int q = 4; q < 7; ++q) if(has[u][q]) t += negoff * s7[q];
-                    sOut[g0 + u] = s7[3];
-                    qOut[g0 + u] = t;
-                }
-            }
-            double acc = 0.0;
-#pragma unroll
-            for(int j = 0; j < kPerLane; ++j) {
-                const size_t e = base + (size_t)j * kLanes;
-                if(e < (size_t)n) {
-                    sNew[e] = sOut[j];
-                    S.q[e] = qOut[j];
-                    acc = acc + (double)sOut[j] * (double)qOut[j];
-                }
-            }
-            double bs;
-            float unused;
-            block_sum_max_256<float>(acc, 0.f, smd, smv, bs, unused, false);
-            if(threadIdx.x == 0) S.part1[lc] = bs;
-        }
-        if(!grid_barrier(a.gs, nb, sense, a.flags, solve_barrier_limit())) return;
-        if(ld_acquire_u32(a.remaining) == 0u) break;
-        const bool yieldNow = a.yieldBelow != 0u && ld_acquire_u32(a.active) <= a.yieldBelow;
-        // alpha of every scene this block works on, a warp per slot
-        for(int j = warp; j < nslots; j += kWarps) {
-            if(sState[j] != 0) continue;
-            const int sc = sScene[j];
-            double tmp;
-            float unused2;
-            warp_reduce_partials(a.sc[sc].part1, nullptr, chunks_of(sc), tmp, unused2);
-            if(lane == 0) {
-                if(tmp < (double)FLT_MIN) {
-                    ++sIter[j];
-                    finish1(j, 1u, true);
-                } else {
-                    sAlpha[j] = (float)(sRho[j] / tmp);
-                }
-            }
-        }
-        __syncthreads();
-        // ---- phase B: x += alpha s, r -= alpha q, max|r|, z = D^-1 r, partial z.r
-        for(unsigned k = 0; k < nmine; ++k) {
-            const int jslot = sSlotOf[k];
-            if(sState[jslot] != 0) continue;
-            const unsigned c = blockIdx.x + k * nb;
-            const int sc = sScene[jslot];
-            const BatchPcgScene& S = a.sc[sc];
-            const int n = S.n;
-            const unsigned lc = c - __ldg(a.cp + sc);
-            const float alpha = sAlpha[jslot];
-            const float* __restrict__ sNew = (sIter[jslot] & 1u) ? S.s1 : S.s0;
-            const size_t base = (size_t)lc * kChunk + threadIdx.x;
-            float xs[kPerLane], ss[kPerLane], rs[kPerLane], qs[kPerLane], is[kPerLane];
-#pragma unroll
-            for(int j = 0; j < kPerLane; ++j) {
-                const size_t e = base + (size_t)j * kLanes;
-                const size_t ee = e < (size_t)n ? e : 0;
-                xs[j] = __ldcg(S.x + ee);
-                ss[j] = __ldcg(sNew + ee);
-                rs[j] = __ldcg(S.r + ee);
-                qs[j] = __ldcg(S.q + ee);
-                is[j] = __ldg(S.invd + ee);
-            }
-            double acc = 0.0;
-            float m = 0.f;
-#pragma unroll
-            for(int j = 0; j < kPerLane; ++j) {
-                const size_t e = base + (size_t)j * kLanes;
-                if(e < (size_t)n) {
-                    S.x[e] = xs[j] + alpha * ss[j];
-                    const float rv = rs[j] + (-alpha) * qs[j];
-                    S.r[e] = rv;
-                    const float ab = vabs(rv);
-                    m = m > ab ? m : ab;
-                    const float zv = is[j] * rv;
-                    S.z[e] = zv;
-                    acc = acc + (double)zv * (double)rv;
-                }
-            }
-            double bs;
-            float bm;
-            block_sum_max_256<float>(acc, m, smd, smv, bs, bm, true);
-            if(threadIdx.x == 0) { S.part2[lc] = bs; S.partMax[lc] = bm; }
-        }
-        if(!grid_barrier(a.gs, nb, sense, a.flags, solve_barrier_limit())) return;
-        for(int j = warp; j < nslots; j += kWarps) {
-            if(sState[j] == 3) {
-                if(lane == 0) {
-                    if(owner(sScene[j])) count_off(sScene[j]);
-                    sState[j] = 1;
-                }
-                continue;
-            }
-            if(sState[j] != 0) continue;
-            const int sc = sScene[j];
-            const BatchPcgScene& S = a.sc[sc];
-            double rhoNew;
-            float resid;
-            warp_reduce_partials(S.part2, S.partMax, chunks_of(sc), rhoNew, resid);
-            if(lane == 0) {
-                ++sIter[j];
-                sResid[j] = resid;
-                if(resid < sTol[j]) {
-                    finish1(j, 1u, false);
-                } else {
-                    sBeta[j] = (float)(rhoNew / sRho[j]);
-                    sRho[j] = rhoNew;
-                    if(sIter[j] >= S.maxIter) {
-                        if(owner(sc)) atomicOr(&S.dst->flags, BNN_FLAG_PCG_MAXITER);
-                        finish1(j, 0u, false);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        if(yieldNow) {
-            // every block leaves here; each unfinished scene's owner saves its scalars
-            for(int j = 0; j < nslots; ++j) {
-                const int sc = sScene[j];
-                if(sState[j] != 0 || threadIdx.x != 0 || !owner(sc)) continue;
-                DevState* d = a.sc[sc].dst;
-                d->iter = sIter[j]; d->rho = sRho[j]; d->beta = sBeta[j]; d->tol = sTol[j]; d->resid = sResid[j];
-                d->done = 0;
-            }
-            return;
-        }
-    }
-}
-
 // ---- iterative refinement helpers -------------------------------------------------
 // Last-block-done over a block's share `blk` of a launch (the batched launches give every
 // scene its own share, so the count to reach is the share's, not gridDim.x)
@@ -2217,7 +1905,7 @@ struct ChunkKernel {
     size_t smem = 0;
 };
 template<class VT, bool COEF, int G, int K> static ChunkKernel chunk_kernel_of() {
-    return {(const void*)k_pcg_chunk<VT, COEF, G, K>, sizeof(ChunkSmem<VT, COEF, G * K>)};
+    return {(const void*)k_pcg_chunk<VT, COEF, G, K>, sizeof(ChunkSmem<VT, COEF, G, K>)};
 }
 template<class VT> static ChunkKernel chunk_kernel(bool coef, ChunkShape c) {
     if(coef) {
@@ -2427,9 +2115,11 @@ int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const floa
 // ---------------------------------------------------------------------------------
 // Batched refinement: pcg_solve's BNN_PCG_REFINED loop for many scenes at once.  Every
 // stage is one launch over the scenes still refining (each scene's blocks found through a
-// per-scene block prefix, as the batched step kernels do); the inner FP32 solves of all of
-// them are one k_pcg_batch launch.  The host keeps each scene's outer loop state and
-// takes exactly the decisions the lone loop takes, from the same device values.
+// per-scene block prefix, as the batched step kernels do); their inner FP32 solves are
+// k_pcg_chunk_batch launches of as many scenes as are resident together.  A scene that does
+// not fit the chunk-resident solve is solved alone, between them.  The host keeps each scene's
+// outer loop state and takes exactly the decisions the lone loop takes, from the same device
+// values.
 // ---------------------------------------------------------------------------------
 struct IrScene {
     int n;
@@ -2438,36 +2128,17 @@ struct IrScene {
     float *r32, *d32;
     const float* diag;
     const int32_t* nbr;
-    int4* rec;                 // packed rows
     double negoff;             // (double)(-(1 * dt))
     double* partMax;
     DevState* st;
     float* pressure;
+    PcgPacket *pkA, *pkB;      // of the chunk-resident solve, zeroed before it
 };
 struct IrReport {
     double res, bmax;
     unsigned iter, flags, done, pad;
 };
-// Uploaded with every launch's tables: the barrier word and the unfinished-scene counters
-struct BatchHeader {
-    GridSync gs;
-    unsigned remaining;
-    unsigned flags;
-    unsigned active;
-};
 
-__global__ void kb_pack_rows(const IrScene* __restrict__ S, const unsigned* __restrict__ P, int ns) {
-    int q;
-    const Blk b = seg_blk(P, ns, q);
-    const IrScene& c = S[q];
-    const int n = c.n;
-    const int r = b.x * blockDim.x + threadIdx.x;
-    if(r >= n) return;
-    int32_t nb[6];
-#pragma unroll
-    for(int k = 0; k < 6; ++k) nb[k] = c.nbr[(size_t)k * n + r];
-    c.rec[r] = pack_row(r, nb, c.diag[r]);
-}
 __global__ void __launch_bounds__(kLanes) kb_ir_init(const IrScene* __restrict__ S, const unsigned* __restrict__ P,
                                                      int ns) {
     int q;
@@ -2475,12 +2146,18 @@ __global__ void __launch_bounds__(kLanes) kb_ir_init(const IrScene* __restrict__
     const IrScene& c = S[q];
     ir_init_body(b, c.n, c.b, c.x64, c.r64, c.partMax, c.st);
 }
+// r32 = (float) r64, and the packets of the solve that follows zeroed (a block of 256 rows in
+// every chunk does its chunk's)
 __global__ void kb_ir_to_f32(const IrScene* __restrict__ S, const unsigned* __restrict__ P, int ns) {
     int q;
     const Blk b = seg_blk(P, ns, q);
     const IrScene& c = S[q];
     const size_t e = (size_t)b.x * blockDim.x + threadIdx.x;
     if(e < (size_t)c.n) c.r32[e] = (float)c.r64[e];
+    if(b.x % kPerLane == 0 && threadIdx.x < 2) {
+        PcgPacket* p = threadIdx.x == 0 ? c.pkA : c.pkB;
+        p[(size_t)(b.x / kPerLane) * kPacketStride] = PcgPacket{0ull, 0ull};
+    }
 }
 __global__ void kb_ir_accumulate(const IrScene* __restrict__ S, const unsigned* __restrict__ P, int ns) {
     int q;
@@ -2503,50 +2180,90 @@ __global__ void kb_ir_finish(const IrScene* __restrict__ S, const unsigned* __re
     const size_t e = (size_t)b.x * blockDim.x + threadIdx.x;
     if(e < (size_t)c.n) c.pressure[e] = (float)c.x64[e];
 }
-// one thread per scene: what the host's outer loop reads, plus the barrier's flags
-__global__ void kb_ir_report(const IrScene* __restrict__ S, int ns, const BatchHeader* hdr,
-                             IrReport* __restrict__ out) {
+// one thread per scene: what the host's outer loop reads
+__global__ void kb_ir_report(const IrScene* __restrict__ S, int ns, IrReport* __restrict__ out) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if(q < ns) {
         const DevState* st = S[q].st;
         out[q] = IrReport{st->outer_res, st->outer_bmax, st->iter, st->flags, st->done, 0u};
     }
-    if(q == 0) out[ns] = IrReport{0.0, 0.0, 0u, hdr->flags, 0u, 0u};
 }
 
 namespace {
 // Layout of the context's device blob (the same offsets in the pinned host mirror):
-// header, IrScene[cap], BatchPcgScene[cap], the prefixes of 256-row blocks and of 2048-row
-// chunks (cap + 1 each), then IrReport[cap + 1] (read back, not uploaded).
+// IrScene[cap], ChunkArgs[cap], the prefixes of 256-row blocks and of 2048-row chunks (cap + 1
+// each), BatchGroup[capGroups], then IrReport[cap] (read back, not uploaded).
 struct BatchLayout {
-    size_t hdr, irs, bps, p256, pch, rep, up, total;
-    explicit BatchLayout(int cap) {
+    size_t irs, args, p256, pch, grp, rep, up, total;
+    BatchLayout(int cap, int capGroups) {
         auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
         const size_t pre = (size_t)(cap + 1) * sizeof(unsigned);
-        hdr = 0;
-        irs = al(sizeof(BatchHeader));
-        bps = irs + al((size_t)cap * sizeof(IrScene));
-        p256 = bps + al((size_t)cap * sizeof(BatchPcgScene));
+        irs = 0;
+        args = irs + al((size_t)cap * sizeof(IrScene));
+        p256 = args + al((size_t)cap * sizeof(ChunkArgs<float>));
         pch = p256 + al(pre);
-        up = pch + al(pre);
+        grp = pch + al(pre);
+        up = grp + al((size_t)capGroups * sizeof(BatchGroup));
         rep = up;
-        total = rep + al((size_t)(cap + 1) * sizeof(IrReport));
+        total = rep + al((size_t)cap * sizeof(IrReport));
     }
 };
+// One launch of a round's inner solves: its shape, first group and blocks
+struct BatchLaunch {
+    ChunkShape shape;
+    int group0 = 0, blocks = 0;
+};
+ChunkKernel batch_chunk_kernel(ChunkShape c) {
+    if(c.K == 2) return {(const void*)k_pcg_chunk_batch<3, 2>, sizeof(BatchChunkSmem<float, 3, 2>)};
+    if(c.G == 3) return {(const void*)k_pcg_chunk_batch<3, 1>, sizeof(BatchChunkSmem<float, 3, 1>)};
+    if(c.G == 2) return {(const void*)k_pcg_chunk_batch<2, 1>, sizeof(BatchChunkSmem<float, 2, 1>)};
+    return {(const void*)k_pcg_chunk_batch<1, 1>, sizeof(BatchChunkSmem<float, 1, 1>)};
+}
+// The groups of the scenes with these chunk counts, cut into launches whose groups are all
+// resident.  Scenes go in descending size: those of a launch then take about as many
+// iterations.  K = 1 while one launch holds all chunks that way, else 2 chunks per group.
+// No scene may have more chunks than a launch holds (batch_most_chunks).
+int batch_most_chunks(int numSM) { return numSM * 3 * 2; }
+void batch_groups(const std::vector<int>& nch, int numSM, std::vector<BatchGroup>& groups, std::vector<BatchLaunch>& launches) {
+    groups.clear();
+    launches.clear();
+    std::vector<int> order(nch.size());
+    long long total = 0;
+    for(size_t i = 0; i < nch.size(); ++i) { order[i] = (int)i; total += nch[i]; }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return nch[a] > nch[b]; });
+    ChunkShape shape{3, 2};
+    if(total <= (long long)numSM * 3) shape = ChunkShape{(int)((total + numSM - 1) / numSM), 1};
+    const int most = numSM * shape.G;  // groups of a launch
+    for(size_t i = 0; i < order.size();) {
+        BatchLaunch l;
+        l.shape = shape;
+        l.group0 = (int)groups.size();
+        int used = 0;
+        for(; i < order.size(); ++i) {
+            const int need = (nch[order[i]] + shape.K - 1) / shape.K;
+            if(used + need > most) break;
+            for(int c = 0; c < nch[order[i]]; c += shape.K) groups.push_back(BatchGroup{order[i], c});
+            used += need;
+        }
+        l.blocks = (used + shape.G - 1) / shape.G;
+        groups.resize((size_t)l.group0 + (size_t)l.blocks * shape.G, BatchGroup{-1, 0});
+        launches.push_back(l);
+    }
+}
 } // namespace
 
-static int batch_reserve(BatchPcgCtx& ctx, int count) {
-    if(count <= ctx.cap && ctx.dev) return BNN_OK;
+static int batch_reserve(BatchPcgCtx& ctx, int count, int groups) {
+    if(count <= ctx.cap && groups <= ctx.capGroups && ctx.dev) return BNN_OK;
+    const int cap = std::max(ctx.cap, count < 64 ? 64 : count + count / 4);
+    const int capGroups = std::max(ctx.capGroups, groups + groups / 4 + 256);
     pcg_batch_release(ctx);
-    const int cap = count < 64 ? 64 : count + count / 4;
-    const BatchLayout L(cap);
+    const BatchLayout L(cap, capGroups);
     BNN_CUDA_CHECK(cudaMalloc(&ctx.dev, L.total));
     BNN_CUDA_CHECK(cudaMallocHost(&ctx.host, L.total));
     std::memset(ctx.host, 0, L.total);
     for(auto& e : ctx.ev) BNN_CUDA_CHECK(cudaEventCreate(&e));
     ctx.cap = cap;
-    ctx.upBytes = L.up;
-    ctx.blobBytes = L.total;
+    ctx.capGroups = capGroups;
     return BNN_OK;
 }
 
@@ -2566,68 +2283,89 @@ int pcg_solve_batch_refined(BatchPcgCtx& ctx, BatchSolveItem* items, int count, 
         bool ok = false, stopped = false;
         float kernelMs = 0.f;
     };
+    int numSM = 0;
+    int rc = coop_sm_count(numSM);
+    if(rc != BNN_OK) return rc;
+    const int chunkSM = numSM < kMostSM ? numSM : kMostSM;
+    auto chunks_of = [&](int i) { return (items[i].n + kChunk - 1) / kChunk; };
+    std::vector<char> alone(count, 0);  // scenes the chunk-resident solve does not take
     std::vector<int> live;
+    int groupsMost = 0;
     for(int i = 0; i < count; ++i) {
         items[i].out = PcgOutcome();
         if(items[i].n == 0) { items[i].out.success = 1; continue; }
-        const int rc = pcg_reserve(*items[i].w, items[i].n, true);
+        rc = pcg_reserve(*items[i].w, items[i].n, true);
         if(rc != BNN_OK) return rc;
+        alone[i] = items[i].layout != kRowsCompact || chunks_of(i) > batch_most_chunks(chunkSM);
         live.push_back(i);
+        groupsMost += chunks_of(i) + 1;
     }
     if(live.empty()) return BNN_OK;
-    int rc = batch_reserve(ctx, (int)live.size());
+    // a launch's last block may hold up to 2 empty groups, and there are no more launches than scenes
+    rc = batch_reserve(ctx, (int)live.size(), groupsMost + 2 * (int)live.size());
     if(rc != BNN_OK) return rc;
-    const BatchLayout L(ctx.cap);
+    const BatchLayout L(ctx.cap, ctx.capGroups);
     char* H = (char*)ctx.host;
     char* D = (char*)ctx.dev;
-    BatchHeader* hh = (BatchHeader*)(H + L.hdr);
     IrScene* hirs = (IrScene*)(H + L.irs);
-    BatchPcgScene* hbps = (BatchPcgScene*)(H + L.bps);
+    ChunkArgs<float>* hargs = (ChunkArgs<float>*)(H + L.args);
     unsigned* hp256 = (unsigned*)(H + L.p256);
     unsigned* hpch = (unsigned*)(H + L.pch);
     const IrReport* hrep = (const IrReport*)(H + L.rep);
     const IrScene* dirs = (const IrScene*)(D + L.irs);
     const unsigned* dp256 = (const unsigned*)(D + L.p256);
     const unsigned* dpch = (const unsigned*)(D + L.pch);
-    BatchHeader* dh = (BatchHeader*)(D + L.hdr);
     IrReport* drep = (IrReport*)(D + L.rep);
+    std::vector<BatchGroup> groups;
+    std::vector<BatchLaunch> launches;
 
-    // tables for the scenes `set` (positions in items), uploaded in one copy; resume: the
-    // inner solves carry on from a yield
-    auto upload = [&](const std::vector<int>& set, bool resume = false) -> cudaError_t {
+    // tables for the scenes `set` (positions in items), uploaded in one copy; solve: with the
+    // groups of their inner solves
+    auto upload = [&](const std::vector<int>& set, bool solve) -> cudaError_t {
         hp256[0] = hpch[0] = 0;
+        std::vector<int> nch, at;
         for(size_t k = 0; k < set.size(); ++k) {
             const BatchSolveItem& it = items[set[k]];
             PcgWork& w = *it.w;
             const int n = it.n;
-            hirs[k] = IrScene{n, it.rhs, w.x64, w.r64, w.r32, w.d32, it.diag, it.nbr, w.rec,
-                              (double)(-(1.0f * it.dt)), w.partMaxD, it.dst, it.pressure};
-            BatchPcgScene& b = hbps[k];
-            b.n = n; b.rhsF = w.r32; b.invd = it.invd; b.rec = w.rec; b.negoff = -(1.0f * it.dt);
-            b.tolFactor = it.innerTol; b.maxIter = it.maxIter; b.x = w.d32; b.r = w.r; b.z = w.z; b.s0 = w.s0;
-            b.s1 = w.s1; b.q = w.q; b.part0 = w.part; b.part1 = w.part + w.nchCap;
-            b.part2 = w.part + 2 * (size_t)w.nchCap; b.partMax = w.partMaxF; b.dst = it.dst;
-            b.resume = resume ? 1 : 0;
+            PcgPacket *pkA = w.packets, *pkB = w.packets + (size_t)w.nchCap * kPacketStride;
+            hirs[k] = IrScene{n, it.rhs, w.x64, w.r64, w.r32, w.d32, it.diag, it.nbr, (double)(-(1.0f * it.dt)),
+                              w.partMaxD, it.dst, it.pressure, pkA, pkB};
             hp256[k + 1] = hp256[k] + (unsigned)((n + 255) / 256);
             hpch[k + 1] = hpch[k] + (unsigned)((n + kChunk - 1) / kChunk);
+            ChunkArgs<float>& c = hargs[k];
+            c.n = n; c.nch = chunks_of(set[k]); c.rhsF = w.r32; c.diag = it.diag; c.invd = it.invd; c.nbr = it.nbr;
+            c.coef = nullptr; c.negoff = -(1.0f * it.dt); c.tolFactor = it.innerTol; c.maxIter = it.maxIter; c.x = w.d32;
+            c.pair = (RowPair<float>*)(void*)w.st32[0]; c.pkA = pkA; c.pkB = pkB; c.st = it.dst;
+            if(!alone[set[k]]) { nch.push_back(c.nch); at.push_back((int)k); }
         }
-        *hh = BatchHeader{GridSync{0u}, (unsigned)set.size(), 0u, hpch[set.size()]};
-        return cudaMemcpyAsync(D, H, L.up, cudaMemcpyHostToDevice, s);
+        if(solve) {
+            batch_groups(nch, chunkSM, groups, launches);
+            BatchGroup* hg = (BatchGroup*)(H + L.grp);
+            for(size_t q = 0; q < groups.size(); ++q)
+                hg[q] = BatchGroup{groups[q].scene < 0 ? -1 : at[groups[q].scene], groups[q].chunk0};
+        }
+        return cudaMemcpyAsync(D, H, solve ? L.up : L.grp, cudaMemcpyHostToDevice, s);
     };
     auto report = [&](int ns) -> int {
-        { kb_ir_report<<<(ns + 128) / 128, 128, 0, s>>>(dirs, ns, dh, drep); bnn_note_launch(); }
-        BNN_CUDA_CHECK(cudaMemcpyAsync(H + L.rep, drep, (size_t)(ns + 1) * sizeof(IrReport), cudaMemcpyDeviceToHost, s));
+        { kb_ir_report<<<(ns + 127) / 128, 128, 0, s>>>(dirs, ns, drep); bnn_note_launch(); }
+        BNN_CUDA_CHECK(cudaMemcpyAsync(H + L.rep, drep, (size_t)ns * sizeof(IrReport), cudaMemcpyDeviceToHost, s));
         BNN_CUDA_CHECK(cudaStreamSynchronize(s));
-        if(hrep[ns].flags & BNN_FLAG_TIMEOUT) { bnn_set_error("batched PCG grid barrier timed out"); return BNN_ERR_TIMEOUT; }
+        for(int k = 0; k < ns; ++k)
+            if(hrep[k].flags & BNN_FLAG_TIMEOUT) { bnn_set_error("batched PCG grid barrier timed out"); return BNN_ERR_TIMEOUT; }
         return BNN_OK;
     };
 
     // outer loop start of every scene: x64 = 0, r64 = b, bmax
     std::vector<Outer> o(count);
     const int nl = (int)live.size();
-    BNN_CUDA_CHECK(upload(live));
-    { kb_pack_rows<<<hp256[nl], 256, 0, s>>>(dirs, dp256, nl); bnn_note_launch(); }
+    BNN_CUDA_CHECK(upload(live, false));
     { kb_ir_init<<<hpch[nl], kLanes, 0, s>>>(dirs, dpch, nl); bnn_note_launch(); }
+    for(int i : live)
+        if(alone[i]) {
+            k_pack_rows<<<(items[i].n + 255) / 256, 256, 0, s>>>(items[i].n, items[i].diag, items[i].nbr, items[i].w->rec);
+            bnn_note_launch();
+        }
     rc = report(nl);
     if(rc != BNN_OK) return rc;
     for(int k = 0; k < nl; ++k) {
@@ -2635,19 +2373,6 @@ int pcg_solve_batch_refined(BatchPcgCtx& ctx, BatchSolveItem* items, int count, 
         e.bmax = hrep[k].bmax;
         e.res = hrep[k].res;
         e.ok = e.bmax < (double)FLT_MIN;
-    }
-
-    // cooperative grid of the inner solves
-    int numSM = 0, perSMv = 0;
-    rc = coop_sm_count(numSM);
-    if(rc != BNN_OK) return rc;
-    {
-        std::lock_guard<std::mutex> lk(g_coop.mu);
-        if(!g_coop.perSM[15]) {
-            BNN_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_coop.perSM[15], k_pcg_batch, kLanes, 0));
-            if(g_coop.perSM[15] < 1) { bnn_set_error("batched PCG kernel cannot be resident"); return BNN_ERR_CUDA; }
-        }
-        perSMv = g_coop.perSM[15];
     }
 
     std::vector<int> set;
@@ -2662,60 +2387,38 @@ int pcg_solve_batch_refined(BatchPcgCtx& ctx, BatchSolveItem* items, int count, 
         }
         if(set.empty()) break;
         const int ns = (int)set.size();
-        BNN_CUDA_CHECK(upload(set));
+        BNN_CUDA_CHECK(upload(set, true));
         { kb_ir_to_f32<<<hp256[ns], 256, 0, s>>>(dirs, dp256, ns); bnn_note_launch(); }
-        // the inner solves: launched over the whole grid, again for the scenes still
-        // iterating whenever their chunks have fallen to half of a launch's
         float ms = 0.f;
-        {
-            std::vector<int> part = set;
-            bool resume = false;
-            for(;;) {
-                const int np = (int)part.size();
-                const unsigned total = hpch[np];
-                const unsigned capB = (unsigned)(numSM * perSMv);
-                // chunks striped over every resident block; a block's chunks (and so the
-                // scenes it meets) must fit its slot table
-                const unsigned grid = std::min(total, capB);
-                const unsigned perBlock = (total + grid - 1) / grid;
-                if(perBlock > (unsigned)kBatchSlots) {
-                    bnn_set_error("batched PCG: too many chunks per block");
-                    return BNN_ERR_CAPACITY;
-                }
-                BatchPcgArgs a;
-                a.sc = (const BatchPcgScene*)(D + L.bps);
-                a.cp = dpch;
-                a.ns = np;
-                a.total = total;
-                a.perBlock = perBlock;
-                a.gs = &dh->gs;
-                a.remaining = &dh->remaining;
-                a.active = &dh->active;
-                a.yieldBelow = 0u;  // striped chunks stay balanced: no relaunch
-                a.flags = &dh->flags;
-                void* args[] = {(void*)&a};
-                {
-                    CoopShare share(grid * (kShareUnits / perSMv), numSM * kShareUnits);
-                    BNN_CUDA_CHECK(cudaEventRecord(ctx.ev[0], s));
-                    BNN_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)k_pcg_batch, dim3(grid), dim3(kLanes), args, 0, s));
-                    bnn_note_launch();
-                    BNN_CUDA_CHECK(cudaEventRecord(ctx.ev[1], s));
-                    rc = report(np);
-                    if(rc != BNN_OK) return rc;
-                }
-                float lm = 0.f;
-                cudaEventElapsedTime(&lm, ctx.ev[0], ctx.ev[1]);
-                ms += lm;
-                std::vector<int> left;
-                for(int k = 0; k < np; ++k)
-                    if(!hrep[k].done) left.push_back(part[k]);
-                if(left.empty()) break;
-                part.swap(left);
-                resume = true;
-                BNN_CUDA_CHECK(upload(part, resume));
-            }
+        for(const BatchLaunch& l : launches) {
+            const ChunkKernel kern = batch_chunk_kernel(l.shape);
+            BNN_CUDA_CHECK(cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kern.smem));
+            const ChunkArgs<float>* dargs = (const ChunkArgs<float>*)(D + L.args);
+            const BatchGroup* dgrp = (const BatchGroup*)(D + L.grp) + l.group0;
+            void* args[] = {(void*)&dargs, (void*)&dgrp};
+            // the share is held until the launch has ended
+            CoopShare share((long long)l.blocks * kShareUnits, (long long)numSM * kShareUnits);
+            BNN_CUDA_CHECK(cudaEventRecord(ctx.ev[0], s));
+            BNN_CUDA_CHECK(cudaLaunchCooperativeKernel(kern.fn, dim3(l.blocks), dim3(l.shape.G * kLanes), args, kern.smem, s));
+            bnn_note_launch();
+            BNN_CUDA_CHECK(cudaEventRecord(ctx.ev[1], s));
+            BNN_CUDA_CHECK(cudaEventSynchronize(ctx.ev[1]));
+            float lm = 0.f;
+            cudaEventElapsedTime(&lm, ctx.ev[0], ctx.ev[1]);
+            ms += lm;
         }
-        BNN_CUDA_CHECK(upload(set));
+        for(int i : set) {
+            if(!alone[i]) continue;
+            const BatchSolveItem& it = items[i];
+            PcgWork& w = *it.w;
+            const bool grid = it.layout != kRowsAny;
+            PcgOutcome inner;
+            rc = pcg_solve_t<float>(w, it.n, ChunkShape{}, numSM, w.r32, it.diag, it.invd, it.nbr, grid ? w.rec : nullptr, nullptr,
+                                    nullptr, -(1.0f * it.dt), it.innerTol, it.maxIter, w.d32, w.r, w.z, w.s0, w.s1, w.q,
+                                    w.partMaxF, true, it.dst, it.hst, s, inner);
+            if(rc != BNN_OK) return rc;
+            ms += inner.kernelMs;
+        }
         { kb_ir_accumulate<<<hp256[ns], 256, 0, s>>>(dirs, dp256, ns); bnn_note_launch(); }
         { kb_ir_residual<<<hpch[ns], kLanes, 0, s>>>(dirs, dpch, ns); bnn_note_launch(); }
         rc = report(ns);
@@ -2740,7 +2443,7 @@ int pcg_solve_batch_refined(BatchPcgCtx& ctx, BatchSolveItem* items, int count, 
         out.success = e.ok ? 1 : 0;
     }
     // pressure = (float) x64
-    BNN_CUDA_CHECK(upload(live));
+    BNN_CUDA_CHECK(upload(live, false));
     { kb_ir_finish<<<hp256[nl], 256, 0, s>>>(dirs, dp256, nl); bnn_note_launch(); }
     BNN_CUDA_CHECK(cudaGetLastError());
     BNN_CUDA_CHECK(cudaStreamSynchronize(s));

@@ -110,3 +110,25 @@ def test_staged_batch_mixed_sizes_and_kinds(bnn):
         info = b.scene_info(sid)
         assert info["steps"] == steps and info["pcg_success"] == 1
     b.close()
+
+
+# Pressure chunks (2048 rows) of a batch against what one launch of the chunk-resident solve
+# holds on 148 SMs: below 148 and 296, two chunks per group (above 444), two launches (above
+# 888), and a scene whose lines are too long for it beside one that it takes.
+@pytest.mark.parametrize("res,frac,count,wide", [((64, 64, 64), 0.6, 4, False), ((128, 96, 96), 0.55, 3, False),
+                                                 ((128, 128, 128), 0.6, 3, False), ((128, 128, 128), 0.6, 5, False),
+                                                 ((40, 32, 24), 0.5, 1, True)])
+def test_batch_pressure_launches_equal_lone_solvers(bnn, res, frac, count, wide):
+    specs = [{"res": res, "block_frac": (frac, frac, frac), "seed": 40 + q} for q in range(count)]
+    if wide:
+        specs.append({"res": (600, 12, 12), "block_frac": (0.98, 0.5, 0.6), "seed": 50})
+    b = bnn.FlipBatch()
+    sids = [b.add_scene(*scenes.batch_scene(s, ppc=2)) for s in specs]
+    for _ in range(2):
+        st = b.step()
+        assert st["failed"] == 0 and st["staged_scenes"] == len(specs)
+    for sid, spec in zip(sids, specs):
+        pg, vg = b.get_scene(sid)
+        pl, vl = _lone(bnn, spec, 2, ppc=2)
+        assert np.array_equal(pg, pl) and np.array_equal(vg, vl), spec
+    b.close()
