@@ -398,6 +398,16 @@ constexpr int kCompactDy = 512, kCompactDz = (1 << 18) - 1;
 inline RowLayout row_layout(long long maxDy, long long maxDz) {
     return maxDy <= kCompactDy && maxDz <= kCompactDz ? kRowsCompact : kRowsGrid;
 }
+// What a caller's neighbour table says about its rows (zeroed before launch_rows_from_table)
+struct RowsInfo {
+    unsigned bad;      // an index outside [-1, n)
+    unsigned notGrid;  // not kRowsGrid
+    int maxDy, maxDz;  // the largest y and z distances
+};
+// A table of 6 neighbours per row (-z, -y, -x, +x, +y, +z; -1 = none) as planes, 1/diag (0 for
+// a zero diagonal) and its RowsInfo
+void launch_rows_from_table(int n, const int32_t* table, const float* diag, int32_t* planes, float* invd, RowsInfo* info,
+                            cudaStream_t s);
 // coef (optional): six planes of off-diagonal values in the order of nbr (face weights
 // != 1); without it every off-diagonal is -dt.
 int pcg_solve(PcgWork& w, int n, const float* rhs, const float* diag, const float* invd, const int32_t* nbr,

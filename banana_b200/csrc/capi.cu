@@ -940,75 +940,76 @@ extern "C" int bnn_pcg_solve_7pt(uint32_t n, const float* diag, const int32_t* n
        (mode & BNN_PCG_MODE_MASK) > 2)
         return BNN_ERR_INVALID_ARGUMENT;
     if(!(offdiag <= 0.f)) return BNN_ERR_INVALID_ARGUMENT;
+    if(n > 0x7fffffffu) return BNN_ERR_INVALID_ARGUMENT;
     cudaStream_t s;
     BNN_CUDA_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    float *dDiag = nullptr, *dInv = nullptr, *dRhs = nullptr, *dP = nullptr;
-    int32_t* dNbr = nullptr;
-    double* dX = nullptr;
-    DevState *dst = nullptr, *hst = nullptr;
+    const size_t nn = n ? n : 1;
+    // one allocation: the caller's arrays as they come, the planes and inverses made of them,
+    // the solution, the records
+    struct Slab {
+        size_t diag, inv, rhs, p, nbr, planes, x, dst, info, total;
+    } L;
+    {
+        size_t at = 0;
+        auto take = [&](size_t bytes) { const size_t r = at; at += (bytes + 255) & ~(size_t)255; return r; };
+        L.diag = take(nn * 4); L.inv = take(nn * 4); L.rhs = take(nn * 4); L.p = take(nn * 4);
+        L.nbr = take(24 * nn); L.planes = take(24 * nn); L.x = take(8 * nn);
+        L.dst = take(sizeof(DevState)); L.info = take(sizeof(RowsInfo));
+        L.total = at;
+    }
+    char* D = nullptr;
+    DevState* hst = nullptr;
     PcgWork w;
     int rc = BNN_OK;
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    std::vector<float> inv(n);
-    std::vector<int32_t> planes(6 * (size_t)n);
-    // rows of a grid in cell order (x neighbours r-1 / r+1, y neighbours within 65535 rows,
-    // z neighbours on their side) take the packed-record solve
-    bool gridRows = true;
-    int64_t maxDy = 0, maxDz = 0;
-    for(uint32_t r = 0; r < n; ++r) {
-        inv[r] = diag[r] != 0.f ? 1.0f / diag[r] : 0.f;
-        for(int q = 0; q < 6; ++q) {
-            const int32_t v = nbr[6 * (size_t)r + q];
-            if(v < -1 || (v >= 0 && (uint32_t)v >= n)) {
-                bnn_set_error("bnn_pcg_solve_7pt: neighbour index outside [-1, n)");
-                cudaEventDestroy(e0);
-                cudaEventDestroy(e1);
-                cudaStreamDestroy(s);
-                return BNN_ERR_INVALID_ARGUMENT;
-            }
-            planes[(size_t)q * n + r] = v;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    auto chk = [&](cudaError_t e) {
+        if(e != cudaSuccess && rc == BNN_OK) {
+            bnn_set_error(cudaGetErrorString(e));
+            rc = e == cudaErrorMemoryAllocation ? BNN_ERR_OUT_OF_MEMORY : BNN_ERR_CUDA;
         }
-        const int64_t R = r;
-        const int32_t* nb = nbr + 6 * (size_t)r;
-        if(nb[2] >= 0 && nb[2] != R - 1) gridRows = false;
-        if(nb[3] >= 0 && nb[3] != R + 1) gridRows = false;
-        if(nb[1] >= 0 && !(nb[1] < R && R - nb[1] <= 65535)) gridRows = false;
-        if(nb[4] >= 0 && !(nb[4] > R && nb[4] - R <= 65535)) gridRows = false;
-        if(nb[0] >= 0 && !(nb[0] < R)) gridRows = false;
-        if(nb[5] >= 0 && !(nb[5] > R)) gridRows = false;
-        if(nb[1] >= 0) maxDy = std::max(maxDy, R - nb[1]);
-        if(nb[4] >= 0) maxDy = std::max(maxDy, nb[4] - R);
-        if(nb[0] >= 0) maxDz = std::max(maxDz, R - nb[0]);
-        if(nb[5] >= 0) maxDz = std::max(maxDz, nb[5] - R);
+    };
+    chk(cudaEventCreate(&e0));
+    chk(cudaEventCreate(&e1));
+    chk(dev_alloc(&D, L.total));
+    chk(pinned_state_alloc(&hst));
+    float *dDiag = (float*)(D + L.diag), *dInv = (float*)(D + L.inv), *dRhs = (float*)(D + L.rhs), *dP = (float*)(D + L.p);
+    int32_t* dNbr = (int32_t*)(D + L.planes);
+    double* dX = (double*)(D + L.x);
+    DevState* dst = (DevState*)(D + L.dst);
+    // rows of a grid in cell order (x neighbours r-1 / r+1, y neighbours within 65535 rows,
+    // z neighbours on their side) take the packed-record solves
+    RowsInfo info{};
+    if(rc == BNN_OK) chk(cudaMemsetAsync(dst, 0, sizeof(DevState), s));
+    if(rc == BNN_OK && n) {
+        chk(cudaMemcpyAsync(D + L.nbr, nbr, 24 * (size_t)n, cudaMemcpyHostToDevice, s));
+        chk(cudaMemcpyAsync(dDiag, diag, n * 4, cudaMemcpyHostToDevice, s));
+        chk(cudaMemcpyAsync(dRhs, rhs, n * 4, cudaMemcpyHostToDevice, s));
+        chk(cudaMemsetAsync(D + L.info, 0, sizeof(RowsInfo), s));
+        if(rc == BNN_OK) {
+            launch_rows_from_table((int)n, (const int32_t*)(D + L.nbr), dDiag, dNbr, dInv, (RowsInfo*)(D + L.info), s);
+            chk(cudaGetLastError());
+        }
+        chk(cudaMemcpyAsync(&info, D + L.info, sizeof(RowsInfo), cudaMemcpyDeviceToHost, s));
     }
+    if(rc == BNN_OK) chk(cudaStreamSynchronize(s));
+    if(rc == BNN_OK && info.bad) {
+        bnn_set_error("bnn_pcg_solve_7pt: neighbour index outside [-1, n)");
+        rc = BNN_ERR_INVALID_ARGUMENT;
+    }
+    const RowLayout layout = info.notGrid ? kRowsAny : row_layout(info.maxDy, info.maxDz);
     // the system stores -dt as the off-diagonal; recover dt so the kernels form -(1*dt)
     const float dt = -offdiag;
-    size_t nn = n ? n : 1;
-    auto chk = [&](cudaError_t e) { if(e != cudaSuccess && rc == BNN_OK) { bnn_set_error(cudaGetErrorString(e)); rc = BNN_ERR_CUDA; } };
-    chk(cudaMalloc(&dDiag, nn * 4)); chk(cudaMalloc(&dInv, nn * 4)); chk(cudaMalloc(&dRhs, nn * 4));
-    chk(cudaMalloc(&dP, nn * 4)); chk(cudaMalloc(&dNbr, 6 * nn * 4)); chk(cudaMalloc(&dX, nn * 8));
-    chk(cudaMalloc(&dst, sizeof(DevState))); chk(cudaHostAlloc(&hst, sizeof(DevState), cudaHostAllocDefault));
-    if(rc == BNN_OK && n) {
-        chk(cudaMemcpyAsync(dDiag, diag, n * 4, cudaMemcpyHostToDevice, s));
-        chk(cudaMemcpyAsync(dInv, inv.data(), n * 4, cudaMemcpyHostToDevice, s));
-        chk(cudaMemcpyAsync(dRhs, rhs, n * 4, cudaMemcpyHostToDevice, s));
-        chk(cudaMemcpyAsync(dNbr, planes.data(), 6 * (size_t)n * 4, cudaMemcpyHostToDevice, s));
-    }
-    if(rc == BNN_OK) chk(cudaMemsetAsync(dst, 0, sizeof(DevState), s));
-    if(rc == BNN_OK) chk(cudaStreamSynchronize(s));
     PcgOutcome po;
     if(rc == BNN_OK) rc = pcg_reserve(w, (int)n, (mode & BNN_PCG_MODE_MASK) != BNN_PCG_FP32);  // outside the timed region
     if(rc == BNN_OK) {
         cudaEventRecord(e0, s);
-        rc = pcg_solve(w, (int)n, dRhs, dDiag, dInv, dNbr, nullptr, gridRows ? row_layout(maxDy, maxDz) : kRowsAny, dt, mode, tol, max_iter, inner_tol, tol, dP, dX,
+        rc = pcg_solve(w, (int)n, dRhs, dDiag, dInv, dNbr, nullptr, layout, dt, mode, tol, max_iter, inner_tol, tol, dP, dX,
                        dst, hst, s, po);
         cudaEventRecord(e1, s);
     }
     if(rc == BNN_OK && n) chk(cudaMemcpyAsync(x_out, dX, n * 8, cudaMemcpyDeviceToHost, s));
     if(rc == BNN_OK) chk(cudaStreamSynchronize(s));
-    if(stats) {
+    if(stats && !info.bad) {
         std::memset(stats, 0, sizeof(*stats));
         stats->iterations = po.iterations;
         stats->outer_iterations = po.outer;
@@ -1018,10 +1019,13 @@ extern "C" int bnn_pcg_solve_7pt(uint32_t n, const float* diag, const int32_t* n
         if(rc == BNN_OK) cudaEventElapsedTime(&ms, e0, e1);
         stats->ms = ms;
     }
+    // the memory goes back with nothing pending on it, whatever failed before
+    cudaStreamSynchronize(s);
     pcg_release(w);
-    cudaFree(dDiag); cudaFree(dInv); cudaFree(dRhs); cudaFree(dP); cudaFree(dNbr); cudaFree(dX); cudaFree(dst);
-    if(hst) cudaFreeHost(hst);
-    cudaEventDestroy(e0); cudaEventDestroy(e1);
+    dev_free(D);
+    pinned_state_free(hst);
+    if(e0) cudaEventDestroy(e0);
+    if(e1) cudaEventDestroy(e1);
     cudaStreamDestroy(s);
     if(rc == BNN_OK && !po.success) return BNN_ERR_PCG_NOT_CONVERGED;
     return rc;
