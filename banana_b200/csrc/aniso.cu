@@ -15,7 +15,9 @@
 // One thread per particle in cell-sorted order.  Both passes walk the cell rows around the
 // particle (z outer, y inner) and, in each row, the sorted particles of the cells its
 // kernel sphere can reach, so every thread sums its neighbours in the canonical order
-// (rows, then cell-sorted order).  Rows and cells that provably hold no neighbour are
+// (rows, then cell-sorted order).  Candidates are taken two at a time: coordinates lie in
+// planes, so a pair is one 8-byte load per axis, and distances, weights and products are
+// formed in packed FP32 (each half rounded as the scalar operation); the sums stay serial.  Rows and cells that provably hold no neighbour are
 // skipped; the margins cover the float rounding of the cell index (see row_range).  The
 // accumulation is branch-free: a candidate outside the sphere adds a weight of 0, which
 // leaves every sum unchanged (none of them can be -0), except the weighted mean, which is
@@ -25,6 +27,7 @@
 // operations and matches the CPU restatement bit for bit.
 #include "bnn_internal.cuh"
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -43,9 +46,56 @@ struct AnisoArgs {
     float margin;     // 0.01 cell: bound on how far a point's cell index can be off its position
 };
 
-__device__ __forceinline__ float kernel_w(float d2, float rinv) {
-    const float t = sqrtf(d2) * rinv;
-    return 1.0f - t * t * t;
+// Packed FP32 pairs.  A packed product followed by a packed sum would be fused by the assembler
+// and round once, so products are a * b + (-0) with the -0 pair a kernel argument, unknown to it.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+    return (F2)__float_as_uint(lo) | (F2)__float_as_uint(hi) << 32;
+}
+__device__ __forceinline__ float lo2(F2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(F2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+struct Packed {
+    F2 minus0, minus1, one;
+};
+__device__ __forceinline__ F2 mul2(F2 a, F2 b, const Packed& k) { return fma2(a, b, k.minus0); }
+// (a a + b b) + c c
+__device__ __forceinline__ F2 len2(F2 a, F2 b, F2 c, const Packed& k) {
+    return add2(add2(mul2(a, a, k), mul2(b, b, k)), mul2(c, c, k));
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// Correctly rounded square roots of a pair: g = x y with y near x^(-1/2), then one Newton step
+// on the residual, g + (x - g g) y / 2 with the residual fused (P. Markstein, IBM J. Res. Dev.
+// 34, 1990); y / 2 is y with its exponent lowered.  Equal to sqrtf for every float in [2^-100,
+// 2^100] (all of them tried).  x is raised to 2^-100 first, which keeps 0 out of the
+// reciprocal: below 2^-75 kernel_w2 gives 1 either way while r >= 2^-24.
+__device__ __forceinline__ F2 sqrt2(F2 v, const Packed& k) {
+    const float x0 = fmaxf(lo2(v), 0x1p-100f), x1 = fmaxf(hi2(v), 0x1p-100f);
+    const float y0 = rsqrt_approx(x0), y1 = rsqrt_approx(x1);
+    const F2 g = mul2(pack2(x0, x1), pack2(y0, y1), k);
+    const F2 e = pack2(fmaf(-lo2(g), lo2(g), x0), fmaf(-hi2(g), hi2(g), x1));
+    const F2 h = pack2(__uint_as_float(__float_as_uint(y0) - 0x00800000u), __uint_as_float(__float_as_uint(y1) - 0x00800000u));
+    return fma2(e, h, g);
+}
+// W = 1 - (|d| / r)^3 of a pair of squared distances.  FAST: 2^-24 <= r <= 2^24, the range in
+// which sqrt2 is exact (or the weight does not depend on it)
+template<bool FAST> __device__ __forceinline__ F2 kernel_w2(F2 d2, F2 rinv, const Packed& k) {
+    const F2 root = FAST ? sqrt2(d2, k) : pack2(sqrtf(lo2(d2)), sqrtf(hi2(d2)));
+    const F2 t = mul2(root, rinv, k);
+    return fma2(mul2(mul2(t, t, k), t, k), k.minus1, k.one);
 }
 
 // The sorted-index range [s, e) of cell row (j, k) that may hold neighbours of p.  A
@@ -165,16 +215,25 @@ __device__ __forceinline__ void kernel_matrix(float a[3][3], float axisRatio, fl
             out[c * 3 + r] = v[r][0] * S[0] * v[c][0] + v[r][1] * S[1] * v[c][1] + v[r][2] * S[2] * v[c][2];
 }
 
-__global__ void __launch_bounds__(128) k_aniso(int n, const float4* __restrict__ pos, const uint32_t* __restrict__ ids,
-                                               const uint32_t* __restrict__ cellStart, AnisoGrid g, AnisoArgs a,
+// Bound by the FP32 pipe (a packed operation takes it for two cycles, so packing saves issue
+// slots, not pipe cycles: 22 and 39 a candidate in the two passes) and, below a few hundred
+// thousand points, by the serial chain of a particle's candidates.  ms against one candidate at a
+// time with sqrtf: 5,000 points 0.480 (0.946), 50,000 0.824 (1.278), 200,003 2.63 (2.74),
+// 1,000,000 12.57 (12.41).  Whole bnn_anisotropic_kernels call, with its temporaries from the
+// pool: 200,003 points 2.87 ms (4.20).  Nine blocks per SM: 200,003 points 2.63 ms against 2.73
+// at eight, 2.68 at ten.
+template<bool FAST>
+__global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict__ px, const float* __restrict__ py,
+                                               const float* __restrict__ pz, const uint32_t* __restrict__ ids,
+                                               const uint32_t* __restrict__ cellStart, AnisoGrid g, AnisoArgs a, Packed k2,
                                                float* __restrict__ outC, float* __restrict__ outM,
                                                unsigned* __restrict__ counters) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = p < n;
-    const float4 P = active ? pos[p] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float Px = active ? px[p] : 0.f, Py = active ? py[p] : 0.f, Pz = active ? pz[p] : 0.f;
     int cj, ck;
     {
-        int c[3] = {(int)((P.x - g.bmin[0]) / g.dx), (int)((P.y - g.bmin[1]) / g.dx), (int)((P.z - g.bmin[2]) / g.dx)};
+        int c[3] = {(int)((Px - g.bmin[0]) / g.dx), (int)((Py - g.bmin[1]) / g.dx), (int)((Pz - g.bmin[2]) / g.dx)};
         bool out = false;
 #pragma unroll
         for(int d = 0; d < 3; ++d) {
@@ -188,37 +247,49 @@ __global__ void __launch_bounds__(128) k_aniso(int n, const float4* __restrict__
     }
     const int R = a.R;
     const uint32_t self = (uint32_t)p;
+    const F2 Px2 = pack2(Px, Px), Py2 = pack2(Py, Py), Pz2 = pack2(Pz, Pz), rinv = pack2(a.rinv, a.rinv);
+    auto at2 = [](const float* __restrict__ v, uint32_t q) { return __ldg(reinterpret_cast<const F2*>(v + q)); };
 
-    // pass 1: neighbour count and weighted mean (AniKernelGenerator.cpp:65-75)
-    float sw = 1.0f, mx = P.x, my = P.y, mz = P.z;
+    // pass 1: neighbour count and weighted mean (AniKernelGenerator.cpp:65-75).  A candidate
+    // that is no neighbour adds 0 w = 0.
+    float sw = 1.0f, mx = Px, my = Py, mz = Pz;
     uint32_t cnt = 0;
     for(int dz = -R; dz <= R; ++dz)
         for(int dy = -R; dy <= R; ++dy) {
             uint32_t s = 0, e = 0;
-            if(active) row_range(g, a, cellStart, P.x, P.y, P.z, cj + dy, ck + dz, s, e);
+            if(active) row_range(g, a, cellStart, Px, Py, Pz, cj + dy, ck + dz, s, e);
+            const uint32_t len = e - s;
 #pragma unroll 2
-            for(uint32_t q = s; q < e; ++q) {
-                const float4 Q = __ldg(pos + q);
-                const float ex = P.x - Q.x, ey = P.y - Q.y, ez = P.z - Q.z;
-                const float d2 = ex * ex + ey * ey + ez * ez;
-                const bool hit = d2 < a.r2 && q != self;
-                const float w = hit ? kernel_w(d2, a.rinv) : 0.0f;
-                sw = sw + w;
-                cnt += hit ? 1u : 0u;
-                const float ax = mx + w * Q.x, ay = my + w * Q.y, az = mz + w * Q.z;
-                mx = hit ? ax : mx;
-                my = hit ? ay : my;
-                mz = hit ? az : mz;
+            for(uint32_t q = s & ~1u; q < e; q += 2) {
+                const F2 Qx = at2(px, q), Qy = at2(py, q), Qz = at2(pz, q);
+                const F2 ex = fma2(Qx, k2.minus1, Px2), ey = fma2(Qy, k2.minus1, Py2), ez = fma2(Qz, k2.minus1, Pz2);
+                const F2 d2 = len2(ex, ey, ez, k2);
+                const bool h0 = lo2(d2) < a.r2 && q - s < len && q != self;
+                const bool h1 = hi2(d2) < a.r2 && q + 1 - s < len && q + 1 != self;
+                const F2 w = kernel_w2<FAST>(d2, rinv, k2);
+                const float w0 = h0 ? lo2(w) : 0.0f, w1 = h1 ? hi2(w) : 0.0f;
+                sw = (sw + w0) + w1;
+                cnt += (h0 ? 1u : 0u) + (h1 ? 1u : 0u);
+                const F2 ww = pack2(w0, w1);
+                const F2 ax = mul2(ww, Qx, k2), ay = mul2(ww, Qy, k2), az = mul2(ww, Qz, k2);
+                mx = (mx + lo2(ax)) + hi2(ax);
+                my = (my + lo2(ay)) + hi2(ay);
+                mz = (mz + lo2(az)) + hi2(az);
             }
         }
+    if(cnt == 0) {  // the mean of the particle alone, a coordinate -0 included
+        mx = Px;
+        my = Py;
+        mz = Pz;
+    }
     const float wx = mx / sw, wy = my / sw, wz = mz / sw;
     const uint32_t id = active ? ids[p] : 0u;
     if(active) {
         // MathHelpers::lerp (MathHelpers.h:549-551)
         const float f = a.blend, omf = 1.0f - f;
-        outC[3 * (size_t)id] = omf * P.x + f * wx;
-        outC[3 * (size_t)id + 1] = omf * P.y + f * wy;
-        outC[3 * (size_t)id + 2] = omf * P.z + f * wz;
+        outC[3 * (size_t)id] = omf * Px + f * wx;
+        outC[3 * (size_t)id + 1] = omf * Py + f * wy;
+        outC[3 * (size_t)id + 2] = omf * Pz + f * wz;
     }
     const bool need = active && cnt >= a.threshold;
     const unsigned sprayMask = __ballot_sync(0xffffffffu, active && !need);
@@ -232,26 +303,36 @@ __global__ void __launch_bounds__(128) k_aniso(int n, const float4* __restrict__
 
     // pass 2: covariance about the weighted mean (AniKernelGenerator.cpp:80-89)
     float sw2 = 1.0f, c00 = 0.f, c01 = 0.f, c02 = 0.f, c11 = 0.f, c12 = 0.f, c22 = 0.f;
+    const F2 Wx2 = pack2(-wx, -wx), Wy2 = pack2(-wy, -wy), Wz2 = pack2(-wz, -wz);
     for(int dz = -R; dz <= R; ++dz)
         for(int dy = -R; dy <= R; ++dy) {
             uint32_t s = 0, e = 0;
-            if(need) row_range(g, a, cellStart, P.x, P.y, P.z, cj + dy, ck + dz, s, e);
+            if(need) row_range(g, a, cellStart, Px, Py, Pz, cj + dy, ck + dz, s, e);
+            const uint32_t len = e - s;
 #pragma unroll 2
-            for(uint32_t q = s; q < e; ++q) {
-                const float4 Q = __ldg(pos + q);
-                const float ex = P.x - Q.x, ey = P.y - Q.y, ez = P.z - Q.z;
-                const float d2 = ex * ex + ey * ey + ez * ez;
-                const float x0 = Q.x - wx, x1 = Q.y - wy, x2 = Q.z - wz;
-                const float dm = x0 * x0 + x1 * x1 + x2 * x2;
-                const bool hit = d2 < a.r2 && q != self && dm < a.r2;
-                const float w = hit ? kernel_w(dm, a.rinv) : 0.0f;
-                sw2 = sw2 + w;
-                c00 = c00 + w * (x0 * x0);
-                c01 = c01 + w * (x0 * x1);
-                c02 = c02 + w * (x0 * x2);
-                c11 = c11 + w * (x1 * x1);
-                c12 = c12 + w * (x1 * x2);
-                c22 = c22 + w * (x2 * x2);
+            for(uint32_t q = s & ~1u; q < e; q += 2) {
+                const F2 Qx = at2(px, q), Qy = at2(py, q), Qz = at2(pz, q);
+                const F2 ex = fma2(Qx, k2.minus1, Px2), ey = fma2(Qy, k2.minus1, Py2), ez = fma2(Qz, k2.minus1, Pz2);
+                const F2 d2 = len2(ex, ey, ez, k2);
+                const F2 x0 = add2(Qx, Wx2), x1 = add2(Qy, Wy2), x2 = add2(Qz, Wz2);
+                const F2 q00 = mul2(x0, x0, k2), q11 = mul2(x1, x1, k2), q22 = mul2(x2, x2, k2);
+                const F2 dm = add2(add2(q00, q11), q22);
+                const bool h0 = lo2(d2) < a.r2 && q - s < len && q != self && lo2(dm) < a.r2;
+                const bool h1 = hi2(d2) < a.r2 && q + 1 - s < len && q + 1 != self && hi2(dm) < a.r2;
+                const F2 w = kernel_w2<FAST>(dm, rinv, k2);
+                const float w0 = h0 ? lo2(w) : 0.0f, w1 = h1 ? hi2(w) : 0.0f;
+                sw2 = (sw2 + w0) + w1;
+                const F2 ww = pack2(w0, w1);
+                auto acc = [&](float c, F2 v) {
+                    const F2 t = mul2(ww, v, k2);
+                    return (c + lo2(t)) + hi2(t);
+                };
+                c00 = acc(c00, q00);
+                c01 = acc(c01, mul2(x0, x1, k2));
+                c02 = acc(c02, mul2(x0, x2, k2));
+                c11 = acc(c11, q11);
+                c12 = acc(c12, mul2(x1, x2, k2));
+                c22 = acc(c22, q22);
             }
         }
     if(!need) return;
@@ -266,12 +347,14 @@ __global__ void __launch_bounds__(128) k_aniso(int n, const float4* __restrict__
     for(int e = 0; e < 9; ++e) out[e] = M[e];
 }
 
+// Positions in sorted order as planes of stride `stride`
 __global__ void k_pack_sorted(const float* __restrict__ pos, const uint32_t* __restrict__ order, uint32_t n,
-                              float4* __restrict__ out) {
+                              float* __restrict__ out, size_t stride) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     const uint32_t p = order[i];
-    out[i] = make_float4(pos[3 * (size_t)p], pos[3 * (size_t)p + 1], pos[3 * (size_t)p + 2], 0.0f);
+#pragma unroll
+    for(int d = 0; d < 3; ++d) out[d * stride + i] = pos[3 * (size_t)p + d];
 }
 
 // order-preserving float <-> uint keys for atomic min / max
@@ -348,14 +431,29 @@ int aniso_check_params(const bnn_aniso_params& p) {
     return BNN_OK;
 }
 
-// The pass over cell-sorted points pos (float4 x, y, z, -), ids = input index of each
-// sorted point, cellStart = C + 1 offsets of grid g.  counters[0] receives the spray
-// points, counters[1] the points outside g (both must be zeroed by the caller).
-void launch_aniso(int n, const float4* pos, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
-                  const bnn_aniso_params& prm, float* outC, float* outM, unsigned* counters, cudaStream_t s) {
-    if(n <= 0) return;
+// The pass over cell-sorted points: coordinate planes pos, pos + stride, pos + 2 stride (8-byte
+// aligned, stride > n when n is odd: element n of each is set to 0, the pair mate of the last
+// point), ids = input index of each sorted point, cellStart = C + 1 offsets of grid g.
+// counters[0] receives the spray points, counters[1] the points outside g (both must be zeroed
+// by the caller).
+cudaError_t launch_aniso(int n, float* pos, size_t stride, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
+                         const bnn_aniso_params& prm, float* outC, float* outM, unsigned* counters, cudaStream_t s) {
+    if(n <= 0) return cudaSuccess;
+    if(n & 1)
+        for(int d = 0; d < 3; ++d) {
+            const cudaError_t e = cudaMemsetAsync(pos + d * stride + n, 0, sizeof(float), s);
+            if(e != cudaSuccess) return e;
+        }
     const AnisoArgs a = make_args(prm, g.dx);
-    { k_aniso<<<(n + 127) / 128, 128, 0, s>>>(n, pos, ids, cellStart, g, a, outC, outM, counters); bnn_note_launch(); }
+    auto both = [](unsigned bits) { return (F2)bits << 32 | bits; };
+    const Packed k{both(0x80000000u), both(0xbf800000u), both(0x3f800000u)};
+    const float r = prm.kernel_ratio * prm.particle_radius;
+    const bool fast = r >= 0x1p-24f && r <= 0x1p24f;
+    const unsigned blocks = (unsigned)((n + 127) / 128);
+    if(fast) k_aniso<true><<<blocks, 128, 0, s>>>(n, pos, pos + stride, pos + 2 * stride, ids, cellStart, g, a, k, outC, outM, counters);
+    else k_aniso<false><<<blocks, 128, 0, s>>>(n, pos, pos + stride, pos + 2 * stride, ids, cellStart, g, a, k, outC, outM, counters);
+    bnn_note_launch();
+    return cudaGetLastError();
 }
 
 } // namespace bnn
@@ -363,10 +461,17 @@ void launch_aniso(int n, const float4* pos, const uint32_t* ids, const uint32_t*
 using namespace bnn;
 
 namespace {
+// Temporary memory of the device's pool, in order on the caller's stream
 struct DevMem {
     void* p = nullptr;
-    ~DevMem() { if(p) cudaFree(p); }
-    cudaError_t alloc(size_t b) { return cudaMalloc(&p, b ? b : 1); }
+    cudaStream_t s = nullptr;
+    ~DevMem() { if(p) cudaFreeAsync(p, s); }
+    cudaError_t alloc(size_t b, cudaStream_t st) {
+        const cudaError_t e = mem_pool_setup();
+        if(e != cudaSuccess) return e;
+        s = st;
+        return cudaMallocAsync(&p, b ? b : 1, st);
+    }
     template<class T> T* as() { return (T*)p; }
 };
 } // namespace
@@ -387,10 +492,10 @@ extern "C" int bnn_anisotropic_kernels(const float* pos_dev, uint32_t n, const b
     cudaStream_t s = (cudaStream_t)stream;
     // bounding box of the points -> the cell grid (cells of a quarter kernel radius)
     DevMem keys;
-    BNN_CUDA_CHECK(keys.alloc(8 * sizeof(unsigned)));
+    BNN_CUDA_CHECK(keys.alloc(8 * sizeof(unsigned), s));
     const unsigned init[8] = {~0u, ~0u, ~0u, 0u, 0u, 0u, 0u, 0u};
     BNN_CUDA_CHECK(cudaMemcpyAsync(keys.p, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    { k_bounds<<<4 * 148, 256, 0, s>>>(pos_dev, n, keys.as<unsigned>()); bnn_note_launch(); }
+    { k_bounds<<<(unsigned)std::min<size_t>(((size_t)n + 255) / 256, 4 * 148), 256, 0, s>>>(pos_dev, n, keys.as<unsigned>()); bnn_note_launch(); }
     unsigned hk[8];
     BNN_CUDA_CHECK(cudaMemcpyAsync(hk, keys.p, sizeof(hk), cudaMemcpyDeviceToHost, s));
     BNN_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -415,24 +520,25 @@ extern "C" int bnn_anisotropic_kernels(const float* pos_dev, uint32_t n, const b
     }
     g.dx = cell;
     const size_t C = (size_t)g.G[0] * g.G[1] * g.G[2];
-    DevMem cid, order, start, pos4, cnt;
-    BNN_CUDA_CHECK(cid.alloc((size_t)n * 4));
-    BNN_CUDA_CHECK(order.alloc((size_t)n * 4));
-    BNN_CUDA_CHECK(start.alloc((C + 1) * 4));
-    BNN_CUDA_CHECK(pos4.alloc((size_t)n * sizeof(float4)));
-    BNN_CUDA_CHECK(cnt.alloc(2 * sizeof(unsigned)));
+    DevMem cid, order, start, planes, cnt;
+    BNN_CUDA_CHECK(cid.alloc((size_t)n * 4, s));
+    BNN_CUDA_CHECK(order.alloc((size_t)n * 4, s));
+    BNN_CUDA_CHECK(start.alloc((C + 1) * 4, s));
+    const size_t stride = ((size_t)n + 64) / 64 * 64;  // room for the last point's pair mate
+    BNN_CUDA_CHECK(planes.alloc(3 * stride * sizeof(float), s));
+    BNN_CUDA_CHECK(cnt.alloc(2 * sizeof(unsigned), s));
     uint32_t oor = 0;
     rc = bnn_cell_sort(pos_dev, n, g.bmin, g.dx, g.G, cid.as<uint32_t>(), order.as<uint32_t>(), start.as<uint32_t>(),
                        &oor, stream);
     if(rc != BNN_OK) return rc;
-    { k_pack_sorted<<<(n + 255) / 256, 256, 0, s>>>(pos_dev, order.as<uint32_t>(), n, pos4.as<float4>()); bnn_note_launch(); }
+    { k_pack_sorted<<<(n + 255) / 256, 256, 0, s>>>(pos_dev, order.as<uint32_t>(), n, planes.as<float>(), stride); bnn_note_launch(); }
     BNN_CUDA_CHECK(cudaMemsetAsync(cnt.p, 0, 2 * sizeof(unsigned), s));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    launch_aniso((int)n, pos4.as<float4>(), order.as<uint32_t>(), start.as<uint32_t>(), g, *params, centers_dev,
-                 matrices_dev, cnt.as<unsigned>(), s);
+    BNN_CUDA_CHECK(launch_aniso((int)n, planes.as<float>(), stride, order.as<uint32_t>(), start.as<uint32_t>(), g, *params,
+                                centers_dev, matrices_dev, cnt.as<unsigned>(), s));
     cudaEventRecord(e1, s);
     unsigned hc[2];
     BNN_CUDA_CHECK(cudaMemcpyAsync(hc, cnt.p, sizeof(hc), cudaMemcpyDeviceToHost, s));

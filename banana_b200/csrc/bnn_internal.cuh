@@ -451,8 +451,8 @@ struct AnisoGrid {
 };
 bnn_aniso_params aniso_defaults(float particleRadius);
 int aniso_check_params(const bnn_aniso_params& p);
-void launch_aniso(int n, const float4* pos, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
-                  const bnn_aniso_params& prm, float* outC, float* outM, unsigned* counters, cudaStream_t s);
+cudaError_t launch_aniso(int n, float* pos, size_t stride, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
+                         const bnn_aniso_params& prm, float* outC, float* outM, unsigned* counters, cudaStream_t s);
 
 void pcg_release(PcgWork& w);
 

@@ -141,3 +141,22 @@ def test_dam_break_128_properties(bnn):
     w = np.linalg.eigvalsh(0.5 * (Kn + Kn.transpose(0, 2, 1)))
     assert (w[:, 2] / w[:, 0]).max() < 8.0 * (1 + 1e-4)
     assert w.min() > 0
+
+
+@pytest.mark.parametrize("n,radius,scale", [(2, 0.05, 1.0), (127, 0.02, 1.0), (257, 0.02, 1.0), (2_001, 0.02, 1.0),
+                                            (600, 0.02, 2.0 ** -23), (600, 0.02, 2.0 ** -26), (600, 0.02, 2.0 ** 26)])
+def test_standalone_candidate_pairs_bitexact(bnn, oracle_mod, n, radius, scale):
+    """Odd counts (the last point's pair mate), coincident points (distance 0) and the ends of
+    the radii for which the packed square root is used."""
+    rng = np.random.default_rng(n)
+    pos = (rng.random((n, 3)) * np.array([0.3, 0.1, 0.2])).astype(np.float32)
+    pos[n // 2:n // 2 + 3] = pos[0]
+    pos = (pos * np.float32(scale)).astype(np.float32)
+    prm = capi.aniso_params(radius * scale, neighbor_threshold=2)
+    d = torch.from_numpy(pos).cuda()
+    cen = torch.empty(n, 3, device="cuda")
+    mat = torch.empty(n, 9, device="cuda")
+    st = capi.anisotropic_kernels_dev(d.data_ptr(), n, prm, cen.data_ptr(), mat.data_ptr())
+    oc, om = _oracle_for(oracle_mod, pos, st, radius * scale, neighbor_threshold=2)[:2]
+    _eq(cen.cpu().numpy(), oc, "centres")
+    _eq(mat.cpu().numpy(), om, "matrices")
