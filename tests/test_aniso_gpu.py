@@ -157,6 +157,7 @@ def test_standalone_candidate_pairs_bitexact(bnn, oracle_mod, n, radius, scale):
     cen = torch.empty(n, 3, device="cuda")
     mat = torch.empty(n, 9, device="cuda")
     st = capi.anisotropic_kernels_dev(d.data_ptr(), n, prm, cen.data_ptr(), mat.data_ptr())
-    oc, om = _oracle_for(oracle_mod, pos, st, radius * scale, neighbor_threshold=2)[:2]
-    _eq(cen.cpu().numpy(), oc, "centres")
-    _eq(mat.cpu().numpy(), om, "matrices")
+    oc, om = _oracle_for(oracle_mod, pos, st, radius * scale, threshold=2)[:2]
+    # at the smallest scales the determinant underflows and the matrices are NaN on both sides
+    assert np.array_equal(cen.cpu().numpy(), oc, equal_nan=True)
+    assert np.array_equal(mat.cpu().numpy(), om, equal_nan=True)
