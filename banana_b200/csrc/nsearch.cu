@@ -1,15 +1,15 @@
 // Uniform-grid cell sort, Morton z-sort and neighbour search (BananaCore/Banana/Grid,
 // BananaCore/Banana/NeighborSearch) as standalone device entry points.
 //
-// Sorting is a stable LSD radix sort (8-bit digits, passes only over the key bits that
-// vary): per 2048-item tile a 256-bin histogram, a digit-major exclusive scan over all
-// tiles, then a scatter that ranks equal digits in input order with warp match masks.
-// Stability gives the canonical order of equal keys (input order), which is what the
-// reference's one-thread bucket fill produces.
+// Sorting is a stable LSD radix sort (8-bit digits, passes only over the bits a key can have): per
+// 2048-item tile a 256-bin histogram, per digit an exclusive scan over the tiles, then a scatter
+// that ranks equal digits in input order with warp match masks.  Stability gives the canonical
+// order of equal keys (input order), which is what the reference's one-thread bucket fill
+// produces.
 #include "bnn_internal.cuh"
 
+#include <algorithm>
 #include <mutex>
-#include <vector>
 
 namespace bnn {
 cudaError_t exclusive_scan_u32_to_u64(const uint32_t* in, unsigned long long* out, size_t n, void* ws, cudaStream_t s);
@@ -21,12 +21,14 @@ constexpr int kRPer = 8;           // rounds per tile
 constexpr int kRTile = kRT * kRPer;
 constexpr int kWarps = kRT / 32;
 
+// Tile histograms of one digit: hist[digit * ntiles + tile]
 template<class K> __global__ void __launch_bounds__(kRT) k_radix_hist(const K* __restrict__ keys, size_t n, int shift,
                                                                       uint32_t* __restrict__ hist, unsigned ntiles) {
     __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
     const size_t base = (size_t)blockIdx.x * kRTile;
+#pragma unroll
     for(int r = 0; r < kRPer; ++r) {
         size_t e = base + (size_t)r * kRT + threadIdx.x;
         if(e < n) atomicAdd(&h[(unsigned)((keys[e] >> shift) & 0xFF)], 1u);
@@ -35,48 +37,135 @@ template<class K> __global__ void __launch_bounds__(kRT) k_radix_hist(const K* _
     hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
+// A block per digit: its row of tile counts becomes their exclusive scan, the row's total goes to
+// totals[digit]
+__global__ void __launch_bounds__(kRT) k_radix_rows(uint32_t* __restrict__ hist, unsigned ntiles, uint32_t* __restrict__ totals) {
+    __shared__ uint32_t warpSum[kWarps];
+    uint32_t* row = hist + (size_t)blockIdx.x * ntiles;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t run = 0;
+    for(unsigned t0 = 0; t0 < ntiles; t0 += kRT) {
+        const unsigned i = t0 + threadIdx.x;
+        const uint32_t v = i < ntiles ? row[i] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for(int off = 1; off < 32; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, x, off);
+            if(lane >= off) x += o;
+        }
+        if(lane == 31) warpSum[w] = x;
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for(int q = 0; q < kWarps; ++q) {
+            const uint32_t o = warpSum[q];
+            before += q < w ? o : 0u;
+            all += o;
+        }
+        if(i < ntiles) row[i] = run + before + x - v;
+        run += all;
+        __syncthreads();
+    }
+    if(threadIdx.x == 0) totals[blockIdx.x] = run;
+}
+
+// Each warp owns 256 consecutive items of its tile and ranks them among its own; after a prefix
+// over the tile's warps and digits the tile is sorted in shared memory and written out in order,
+// so that a digit's items leave as a run of consecutive addresses.
 template<class K> __global__ void __launch_bounds__(kRT) k_radix_scatter(const K* __restrict__ kin,
                                                                          const uint32_t* __restrict__ vin,
                                                                          K* __restrict__ kout, uint32_t* __restrict__ vout,
                                                                          size_t n, int shift,
-                                                                         const uint32_t* __restrict__ offs,
+                                                                         const uint32_t* __restrict__ rows,
+                                                                         const uint32_t* __restrict__ totals,
                                                                          unsigned ntiles) {
-    __shared__ uint32_t runBase[256];
     __shared__ uint32_t cnt[kWarps][256];
+    __shared__ uint32_t toOut[256];  // a digit's place in the output minus its place in the tile
+    __shared__ uint32_t warpSum[2][kWarps];
+    __shared__ K sKey[kRTile];
+    __shared__ uint32_t sVal[kRTile];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    runBase[t] = offs[(size_t)t * ntiles + blockIdx.x];
-    const size_t base = (size_t)blockIdx.x * kRTile;
+    const size_t base = (size_t)blockIdx.x * kRTile + (size_t)w * (32 * kRPer) + lane;
     const unsigned lt = (1u << lane) - 1u;
-    for(int r = 0; r < kRPer; ++r) {
+    auto warp_exclusive = [&](uint32_t v, uint32_t* sum) {
+        uint32_t x = v;
 #pragma unroll
-        for(int q = 0; q < kWarps; ++q) cnt[q][t] = 0;
-        __syncthreads();
-        const size_t e = base + (size_t)r * kRT + t;
-        const bool valid = e < n;
-        K key = valid ? kin[e] : K(0);
-        const unsigned d = valid ? (unsigned)((key >> shift) & 0xFF) : 256u;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const unsigned rank = __popc(peers & lt);
-        if(valid && rank == 0) cnt[w][d] = __popc(peers);
-        __syncthreads();
-        if(valid) {
-            uint32_t off = 0;
-            for(int q = 0; q < w; ++q) off += cnt[q][d];
-            const uint32_t dst = runBase[d] + off + rank;
-            kout[dst] = key;
-            vout[dst] = vin ? vin[e] : (uint32_t)e;
+        for(int off = 1; off < 32; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, x, off);
+            if(lane >= off) x += o;
         }
-        __syncthreads();
-        uint32_t tot = 0;
+        if(lane == 31) sum[w] = x;
+        return x - v;
+    };
+    K key[kRPer];
+    uint32_t val[kRPer];
 #pragma unroll
-        for(int q = 0; q < kWarps; ++q) tot += cnt[q][t];
-        runBase[t] += tot;
-        __syncthreads();
+    for(int r = 0; r < kRPer; ++r) {
+        const size_t e = base + 32 * r;
+        key[r] = e < n ? kin[e] : K(0);
+        val[r] = e < n ? (vin ? vin[e] : (uint32_t)e) : 0u;
+    }
+    // where digit t's items of this tile start: the digits before it and the tiles before this one
+    uint32_t start = warp_exclusive(totals[t], warpSum[0]) + rows[(size_t)t * ntiles + blockIdx.x];
+#pragma unroll
+    for(int q = lane; q < 256; q += 32) cnt[w][q] = 0;
+    __syncwarp();
+    // rank of an item among the warp's items of its digit so far
+    uint32_t rank[kRPer];
+#pragma unroll
+    for(int r = 0; r < kRPer; ++r) {
+        const bool valid = base + 32 * r < n;
+        const unsigned d = valid ? (unsigned)((key[r] >> shift) & 0xFF) : 256u;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const unsigned before = __popc(peers & lt);
+        rank[r] = valid ? cnt[w][d] + before : 0u;
+        __syncwarp();
+        if(valid && before == 0) cnt[w][d] += __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    uint32_t mine = 0;  // digit t's items in the tile, then their place in it
+#pragma unroll
+    for(int q = 0; q < kWarps; ++q) mine += cnt[q][t];
+    const uint32_t within = warp_exclusive(mine, warpSum[1]);
+    __syncthreads();
+    {
+        uint32_t run = within;
+        for(int q = 0; q < w; ++q) { start += warpSum[0][q]; run += warpSum[1][q]; }
+        toOut[t] = start - run;
+#pragma unroll
+        for(int q = 0; q < kWarps; ++q) {
+            const uint32_t c = cnt[q][t];
+            cnt[q][t] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for(int r = 0; r < kRPer; ++r)
+        if(base + 32 * r < n) {
+            const uint32_t at = cnt[w][(unsigned)((key[r] >> shift) & 0xFF)] + rank[r];
+            sKey[at] = key[r];
+            sVal[at] = val[r];
+        }
+    __syncthreads();
+    const uint32_t items = (uint32_t)min((size_t)kRTile, n - (size_t)blockIdx.x * kRTile);
+#pragma unroll
+    for(int r = 0; r < kRPer; ++r) {
+        const uint32_t i = r * kRT + t;
+        if(i < items) {
+            const K k = sKey[i];
+            const uint32_t dst = toOut[(unsigned)((k >> shift) & 0xFF)] + i;
+            kout[dst] = k;
+            vout[dst] = sVal[i];
+        }
     }
 }
 
-template<class K> __global__ void k_key_bits(const K* __restrict__ keys, size_t n, unsigned long long* orv,
-                                             unsigned long long* andv) {
+// OR and AND of all keys, reduced over the block before the two atomics
+template<class K> __global__ void __launch_bounds__(256) k_key_bits(const K* __restrict__ keys, size_t n, unsigned long long* orv,
+                                                                    unsigned long long* andv) {
+    __shared__ unsigned long long so[8], sa[8];
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long o = 0, a = ~0ull;
     for(; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -88,7 +177,13 @@ template<class K> __global__ void k_key_bits(const K* __restrict__ keys, size_t 
         o |= __shfl_xor_sync(0xffffffffu, o, off);
         a &= __shfl_xor_sync(0xffffffffu, a, off);
     }
-    if((threadIdx.x & 31) == 0) { atomicOr(orv, o); atomicAnd(andv, a); }
+    if((threadIdx.x & 31) == 0) { so[threadIdx.x >> 5] = o; sa[threadIdx.x >> 5] = a; }
+    __syncthreads();
+    if(threadIdx.x == 0) {
+        for(int q = 1; q < 8; ++q) { o |= so[q]; a &= sa[q]; }
+        atomicOr(orv, o);
+        atomicAnd(andv, a);
+    }
 }
 
 __global__ void k_iota(uint32_t* v, size_t n) {
@@ -96,21 +191,40 @@ __global__ void k_iota(uint32_t* v, size_t n) {
     if(i < n) v[i] = (uint32_t)i;
 }
 
-// Grid::getCellIdx + getCellLinearizedIndex (Grid.h:108-111,156-162), clamped to the grid
-__global__ void k_grid_cell_ids(const float* __restrict__ pos, uint32_t n, float b0, float b1, float b2, float cs,
-                                int n0, int n1, int n2, uint32_t* __restrict__ cid, unsigned* oor) {
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(p >= n) return;
-    int c[3] = {(int)((pos[3 * p] - b0) / cs), (int)((pos[3 * p + 1] - b1) / cs), (int)((pos[3 * p + 2] - b2) / cs)};
+// Grid::getCellIdx + getCellLinearizedIndex (Grid.h:108-111,156-162), clamped to the grid; on
+// the way the tile histogram of the sort's first digit (hist, a block per tile) and the count
+// of every cell (count, optional)
+__global__ void __launch_bounds__(kRT) k_grid_cell_ids(const float* __restrict__ pos, uint32_t n, float b0, float b1, float b2,
+                                                       float cs, int n0, int n1, int n2, uint32_t* __restrict__ cid,
+                                                       unsigned* oor, uint32_t* __restrict__ hist, unsigned ntiles,
+                                                       uint32_t* __restrict__ count) {
+    __shared__ uint32_t h[256];
+    h[threadIdx.x] = 0;
+    __syncthreads();
     const int nn[3] = {n0, n1, n2};
-    bool out = false;
+    const float bb[3] = {b0, b1, b2};
+    int left = 0;  // points outside the grid
+#pragma unroll 4
+    for(int r = 0; r < kRPer; ++r) {
+        const size_t p = (size_t)blockIdx.x * kRTile + (size_t)r * kRT + threadIdx.x;
+        if(p >= n) break;
+        int c[3];
+        bool out = false;
 #pragma unroll
-    for(int d = 0; d < 3; ++d) {
-        if(c[d] < 0) { c[d] = 0; out = true; }
-        if(c[d] >= nn[d]) { c[d] = nn[d] - 1; out = true; }
+        for(int d = 0; d < 3; ++d) {
+            c[d] = (int)((pos[3 * p + d] - bb[d]) / cs);
+            if(c[d] < 0) { c[d] = 0; out = true; }
+            if(c[d] >= nn[d]) { c[d] = nn[d] - 1; out = true; }
+        }
+        left += out ? 1 : 0;
+        const uint32_t id = (uint32_t)(((size_t)c[2] * n1 + c[1]) * n0 + c[0]);
+        cid[p] = id;
+        atomicAdd(&h[id & 0xFF], 1u);
+        if(count) atomicAdd(count + id, 1u);
     }
-    if(out) atomicAdd(oor, 1u);
-    cid[p] = (uint32_t)(((size_t)c[2] * n1 + c[1]) * n0 + c[0]);
+    if(left) atomicAdd(oor, (unsigned)left);
+    __syncthreads();
+    hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
 __global__ void k_histogram(const uint32_t* __restrict__ keys, size_t n, uint32_t* __restrict__ count) {
@@ -368,54 +482,59 @@ struct DevBuf {
     template<class T> T* as() { return (T*)p; }
 };
 
-// stable sort of keys (input order for ties); returns permutation in permOut and sorted
-// keys in keysOut.  Uses only the key bits that vary.
+// uint32 words a sort of n keys needs for its tile histograms and digit totals
+size_t radix_scratch_words(size_t n) { return 256 * ((n + kRTile - 1) / kRTile) + 256; }
+
+// Stable sort (input order for ties) of the key bits [lo, hi): the permutation in permOut, the
+// sorted keys in keysOut; k2 / v2 hold n keys / values, scratch radix_scratch_words(n).  firstHist:
+// scratch already holds the tile histograms of the first digit.
 template<class K>
-int radix_sort(const K* keys, size_t n, K* keysOut, uint32_t* permOut, cudaStream_t s) {
-    if(n == 0) return BNN_OK;
-    DevBuf bits, k2, v2, hist, ws;
-    BNN_CUDA_CHECK(bits.alloc(2 * sizeof(unsigned long long), s));
-    unsigned long long init[2] = {0ull, ~0ull};
-    BNN_CUDA_CHECK(cudaMemcpyAsync(bits.p, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    { k_key_bits<K><<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(keys, n, bits.as<unsigned long long>(),
-                                                                                   bits.as<unsigned long long>() + 1); bnn_note_launch(); }
-    unsigned long long hb[2];
-    BNN_CUDA_CHECK(cudaMemcpyAsync(hb, bits.p, sizeof(hb), cudaMemcpyDeviceToHost, s));
-    BNN_CUDA_CHECK(cudaStreamSynchronize(s));
-    const unsigned long long vary = hb[0] ^ hb[1];
-    int lo = 0, hi = -1;
-    if(vary) {
-        lo = __builtin_ctzll(vary) & ~7;
-        hi = 63 - __builtin_clzll(vary);
-    }
+cudaError_t radix_passes(const K* keys, size_t n, int lo, int hi, K* keysOut, uint32_t* permOut, K* k2, uint32_t* v2,
+                         uint32_t* scratch, bool firstHist, cudaStream_t s) {
     const unsigned ntiles = (unsigned)((n + kRTile - 1) / kRTile);
-    BNN_CUDA_CHECK(k2.alloc(n * sizeof(K), s));
-    BNN_CUDA_CHECK(v2.alloc(n * sizeof(uint32_t), s));
-    BNN_CUDA_CHECK(hist.alloc(((size_t)256 * ntiles + 1) * sizeof(uint32_t), s));
-    size_t wsb = scan_workspace_bytes((size_t)256 * ntiles);
-    if(wsb) BNN_CUDA_CHECK(ws.alloc(wsb, s));
-    std::vector<int> shifts;
-    for(int sh = lo; sh <= hi; sh += 8) shifts.push_back(sh);
-    // ping-pong so that the last pass lands in keysOut / permOut
+    uint32_t* totals = scratch + (size_t)256 * ntiles;
     const K* kin = keys;
     const uint32_t* vin = nullptr;
-    const int np = (int)shifts.size();
-    if(np == 0) {
-        BNN_CUDA_CHECK(cudaMemcpyAsync(keysOut, keys, n * sizeof(K), cudaMemcpyDeviceToDevice, s));
+    const int np = (hi - lo + 7) / 8;
+    if(np <= 0) {
+        if(keysOut) {
+            const cudaError_t e = cudaMemcpyAsync(keysOut, keys, n * sizeof(K), cudaMemcpyDeviceToDevice, s);
+            if(e != cudaSuccess) return e;
+        }
         { k_iota<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(permOut, n); bnn_note_launch(); }
-        return BNN_OK;
+        return cudaGetLastError();
     }
     for(int pi = 0; pi < np; ++pi) {
+        // ping-pong so that the last pass lands in keysOut / permOut
         const bool toOut = ((np - 1 - pi) % 2) == 0;
-        K* kout = toOut ? keysOut : k2.as<K>();
-        uint32_t* vout = toOut ? permOut : v2.as<uint32_t>();
-        { k_radix_hist<K><<<ntiles, kRT, 0, s>>>(kin, n, shifts[pi], hist.as<uint32_t>(), ntiles); bnn_note_launch(); }
-        BNN_CUDA_CHECK(exclusive_scan_u32(hist.as<uint32_t>(), hist.as<uint32_t>(), (size_t)256 * ntiles, ws.p, s));
-        { k_radix_scatter<K><<<ntiles, kRT, 0, s>>>(kin, vin, kout, vout, n, shifts[pi], hist.as<uint32_t>(), ntiles); bnn_note_launch(); }
-        BNN_CUDA_CHECK(cudaGetLastError());
+        K* kout = toOut ? keysOut : k2;
+        uint32_t* vout = toOut ? permOut : v2;
+        const int shift = lo + 8 * pi;
+        if(pi > 0 || !firstHist) { k_radix_hist<K><<<ntiles, kRT, 0, s>>>(kin, n, shift, scratch, ntiles); bnn_note_launch(); }
+        { k_radix_rows<<<256, kRT, 0, s>>>(scratch, ntiles, totals); bnn_note_launch(); }
+        { k_radix_scatter<K><<<ntiles, kRT, 0, s>>>(kin, vin, kout, vout, n, shift, scratch, totals, ntiles); bnn_note_launch(); }
         kin = kout;
         vin = vout;
     }
+    return cudaGetLastError();
+}
+// bits of the values below `bound`
+int bits_below(size_t bound) {
+    int b = 0;
+    while(b < 63 && ((size_t)1 << b) < bound) ++b;
+    return b;
+}
+
+// radix_passes with its temporaries from the pool, in order on s
+template<class K>
+int radix_sort(const K* keys, size_t n, int lo, int hi, K* keysOut, uint32_t* permOut, cudaStream_t s) {
+    if(n == 0) return BNN_OK;
+    DevBuf k2, v2, scratch;
+    BNN_CUDA_CHECK(k2.alloc(n * sizeof(K), s));
+    BNN_CUDA_CHECK(v2.alloc(n * sizeof(uint32_t), s));
+    BNN_CUDA_CHECK(scratch.alloc(radix_scratch_words(n) * sizeof(uint32_t), s));
+    BNN_CUDA_CHECK(radix_passes<K>(keys, n, lo, hi, keysOut, permOut, k2.as<K>(), v2.as<uint32_t>(), scratch.as<uint32_t>(),
+                                   false, s));
     return BNN_OK;
 }
 } // namespace
@@ -432,27 +551,31 @@ extern "C" int bnn_cell_sort(const float* pos_dev, uint32_t n, const float bmin[
     const size_t C = (size_t)ncells[0] * ncells[1] * ncells[2];
     if(C >= 0xffffffffull) return BNN_ERR_NOT_SUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    DevBuf oor, keysSorted;
-    BNN_CUDA_CHECK(oor.alloc(sizeof(unsigned), s));
-    BNN_CUDA_CHECK(cudaMemsetAsync(oor.p, 0, sizeof(unsigned), s));
+    // one allocation: the out-of-grid counter and the cell counts (zeroed together), the sort's
+    // key and value arrays, its histograms, the scan's workspace
+    size_t bytes = 0;
+    auto take = [&](size_t b) { const size_t at = bytes; bytes += (b + 255) & ~(size_t)255; return at; };
+    const size_t aOor = take(sizeof(unsigned)), aCells = take(cell_start_dev ? C * sizeof(uint32_t) : 0), zeroed = bytes;
+    const size_t aKeys = take((size_t)n * 4), aK2 = take((size_t)n * 4), aV2 = take((size_t)n * 4);
+    const size_t aScratch = take(radix_scratch_words(n) * 4), aWs = take(cell_start_dev ? scan_workspace_bytes(C) : 0);
+    DevBuf buf;
+    BNN_CUDA_CHECK(buf.alloc(bytes, s));
+    char* D = buf.as<char>();
+    unsigned* oor = (unsigned*)(D + aOor);
+    uint32_t* count = cell_start_dev ? (uint32_t*)(D + aCells) : nullptr;
+    BNN_CUDA_CHECK(cudaMemsetAsync(D, 0, zeroed, s));
     if(n) {
-        { k_grid_cell_ids<<<(n + 255) / 256, 256, 0, s>>>(pos_dev, n, bmin[0], bmin[1], bmin[2], cell_size, ncells[0],
-                                                         ncells[1], ncells[2], cell_id_dev, oor.as<unsigned>()); bnn_note_launch(); }
-        BNN_CUDA_CHECK(keysSorted.alloc((size_t)n * sizeof(uint32_t), s));
-        int rc = radix_sort<uint32_t>(cell_id_dev, n, keysSorted.as<uint32_t>(), sorted_idx_dev, s);
-        if(rc != BNN_OK) return rc;
+        uint32_t* scratch = (uint32_t*)(D + aScratch);
+        const unsigned ntiles = (n + kRTile - 1) / kRTile;
+        { k_grid_cell_ids<<<ntiles, kRT, 0, s>>>(pos_dev, n, bmin[0], bmin[1], bmin[2], cell_size, ncells[0], ncells[1], ncells[2],
+                                                 cell_id_dev, oor, scratch, ntiles, count); bnn_note_launch(); }
+        // the ids' bits are known from the cell count: no pass over the keys to find them
+        BNN_CUDA_CHECK(radix_passes<uint32_t>(cell_id_dev, n, 0, bits_below(C), (uint32_t*)(D + aKeys), sorted_idx_dev,
+                                              (uint32_t*)(D + aK2), (uint32_t*)(D + aV2), scratch, true, s));
     }
-    if(cell_start_dev) {
-        DevBuf cnt, ws;
-        BNN_CUDA_CHECK(cnt.alloc(C * sizeof(uint32_t), s));
-        BNN_CUDA_CHECK(cudaMemsetAsync(cnt.p, 0, C * sizeof(uint32_t), s));
-        if(n) { k_histogram<<<(n + 255) / 256, 256, 0, s>>>(cell_id_dev, n, cnt.as<uint32_t>()); bnn_note_launch(); }
-        size_t wsb = scan_workspace_bytes(C);
-        if(wsb) BNN_CUDA_CHECK(ws.alloc(wsb, s));
-        BNN_CUDA_CHECK(exclusive_scan_u32(cnt.as<uint32_t>(), cell_start_dev, C, ws.p, s));
-    }
+    if(cell_start_dev) BNN_CUDA_CHECK(exclusive_scan_u32(count, cell_start_dev, C, D + aWs, s));
     unsigned h = 0;
-    BNN_CUDA_CHECK(cudaMemcpyAsync(&h, oor.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    BNN_CUDA_CHECK(cudaMemcpyAsync(&h, oor, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     BNN_CUDA_CHECK(cudaStreamSynchronize(s));
     if(out_of_range) *out_of_range = h;
     return BNN_OK;
@@ -465,9 +588,20 @@ extern "C" int bnn_z_sort(const float* pos_dev, uint32_t n, float radius, uint64
     cudaStream_t s = (cudaStream_t)stream;
     const float inv = (float)(1.0 / (double)radius);
     { k_zvalues<<<(n + 255) / 256, 256, 0, s>>>(pos_dev, n, inv, (unsigned long long*)zvalue_dev); bnn_note_launch(); }
-    DevBuf sorted;
+    // the codes' top bits are the same for all points: sort only the bits that vary
+    DevBuf sorted, bits;
+    BNN_CUDA_CHECK(bits.alloc(2 * sizeof(unsigned long long), s));
+    BNN_CUDA_CHECK(cudaMemsetAsync(bits.p, 0, sizeof(unsigned long long), s));
+    BNN_CUDA_CHECK(cudaMemsetAsync(bits.as<unsigned long long>() + 1, 0xff, sizeof(unsigned long long), s));
+    { k_key_bits<unsigned long long><<<(unsigned)std::min<size_t>(((size_t)n + 255) / 256, 592), 256, 0, s>>>(
+          (const unsigned long long*)zvalue_dev, n, bits.as<unsigned long long>(), bits.as<unsigned long long>() + 1); bnn_note_launch(); }
+    unsigned long long hb[2];
+    BNN_CUDA_CHECK(cudaMemcpyAsync(hb, bits.p, sizeof(hb), cudaMemcpyDeviceToHost, s));
+    BNN_CUDA_CHECK(cudaStreamSynchronize(s));
+    const unsigned long long vary = hb[0] ^ hb[1];
+    const int lo = vary ? __builtin_ctzll(vary) & ~7 : 0, hi = vary ? 64 - __builtin_clzll(vary) : 0;
     BNN_CUDA_CHECK(sorted.alloc((size_t)n * sizeof(unsigned long long), s));
-    int rc = radix_sort<unsigned long long>((const unsigned long long*)zvalue_dev, n, sorted.as<unsigned long long>(),
+    int rc = radix_sort<unsigned long long>((const unsigned long long*)zvalue_dev, n, lo, hi, sorted.as<unsigned long long>(),
                                             perm_dev, s);
     if(rc != BNN_OK) return rc;
     BNN_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -502,7 +636,7 @@ extern "C" int bnn_neighbors(const float* pos_dev, uint32_t n, float radius, uin
     { k_dense_cell<<<(n + 255) / 256, 256, 0, s>>>(keys3.as<int>(), n, kmm.as<int>(), (int)d0, (int)d1, cid.as<uint32_t>()); bnn_note_launch(); }
     BNN_CUDA_CHECK(cidSorted.alloc((size_t)n * sizeof(uint32_t), s));
     BNN_CUDA_CHECK(order.alloc((size_t)n * sizeof(uint32_t), s));
-    int rc = radix_sort<uint32_t>(cid.as<uint32_t>(), n, cidSorted.as<uint32_t>(), order.as<uint32_t>(), s);
+    int rc = radix_sort<uint32_t>(cid.as<uint32_t>(), n, 0, bits_below((size_t)V), cidSorted.as<uint32_t>(), order.as<uint32_t>(), s);
     if(rc != BNN_OK) return rc;
     BNN_CUDA_CHECK(sp.alloc((size_t)n * sizeof(float4), s));
     { k_gather_pos<<<(n + 255) / 256, 256, 0, s>>>(pos_dev, order.as<uint32_t>(), n, sp.as<float4>()); bnn_note_launch(); }
@@ -553,8 +687,8 @@ constexpr size_t kOffCounter = 0;                                               
 constexpr size_t kOffKeys0 = alignUp(kOffCounter + 16);                               // sorted keys
 constexpr size_t kOffKeys1 = alignUp(kOffKeys0 + sizeof(uint32_t) * kNoAllocMaxPoints);  // ping-pong keys
 constexpr size_t kOffVals1 = alignUp(kOffKeys1 + sizeof(uint32_t) * kNoAllocMaxPoints);  // ping-pong payload
-constexpr size_t kOffHist = alignUp(kOffVals1 + sizeof(uint32_t) * kNoAllocMaxPoints);   // radix histogram (+1)
-constexpr size_t kOffCells = alignUp(kOffHist + sizeof(uint32_t) * (256u * kNoAllocTiles + 1));  // cell counts
+constexpr size_t kOffHist = alignUp(kOffVals1 + sizeof(uint32_t) * kNoAllocMaxPoints);   // radix histograms, digit totals
+constexpr size_t kOffCells = alignUp(kOffHist + sizeof(uint32_t) * (256u * kNoAllocTiles + 256));  // cell counts
 constexpr size_t kOffScanWs = alignUp(kOffCells + sizeof(uint32_t) * kNoAllocMaxCells);  // scan workspace
 constexpr size_t kScanWsBytes = 64u * 1024u;  // >= scan_workspace_bytes of either scan, checked at run time
 constexpr size_t kNoAllocScratchBytes = alignUp(kOffScanWs + kScanWsBytes);
@@ -624,8 +758,7 @@ extern "C" int bnn_cell_sort_noalloc(const float* pos_dev, uint32_t n, const flo
                       "fixed scratch array; use bnn_cell_sort");
         return BNN_ERR_CAPACITY;
     }
-    if(scan_workspace_bytes((size_t)256 * kNoAllocTiles) > kScanWsBytes || scan_workspace_bytes(C) > kScanWsBytes)
-        return BNN_ERR_CAPACITY;
+    if(scan_workspace_bytes(C) > kScanWsBytes) return BNN_ERR_CAPACITY;
     unsigned char* scratch = nullptr;
     int rc = noalloc_scratch(&scratch);
     if(rc != BNN_OK) return rc;
@@ -639,36 +772,14 @@ extern "C" int bnn_cell_sort_noalloc(const float* pos_dev, uint32_t n, const flo
     void* scanWs = scratch + kOffScanWs;
     // the array keeps the previous call's contents: zero what is accumulated into
     BNN_CUDA_CHECK(cudaMemsetAsync(oor, 0, sizeof(unsigned), s));
+    if(cell_start_dev) BNN_CUDA_CHECK(cudaMemsetAsync(cells, 0, C * sizeof(uint32_t), s));
     if(n) {
-        { k_grid_cell_ids<<<(n + 255) / 256, 256, 0, s>>>(pos_dev, n, bmin[0], bmin[1], bmin[2], cell_size, ncells[0],
-                                                         ncells[1], ncells[2], cell_id_dev, oor); bnn_note_launch(); }
-        // stable LSD radix sort over the bits a cell id < C can have; ping-pong so the
-        // last pass writes the caller's sorted_idx_dev
-        int bits = 0;
-        while(bits < 32 && ((size_t)1 << bits) < C) ++bits;
-        const int passes = (bits + 7) / 8;
-        const unsigned ntiles = (unsigned)((n + kRTile - 1) / kRTile);
-        if(passes == 0) {
-            { k_iota<<<(n + 255) / 256, 256, 0, s>>>(sorted_idx_dev, n); bnn_note_launch(); }
-        }
-        const uint32_t* kin = cell_id_dev;
-        const uint32_t* vin = nullptr;
-        for(int pi = 0; pi < passes; ++pi) {
-            const bool toOut = ((passes - 1 - pi) % 2) == 0;
-            uint32_t* kout = toOut ? keys0 : keys1;
-            uint32_t* vout = toOut ? sorted_idx_dev : vals1;
-            { k_radix_hist<uint32_t><<<ntiles, kRT, 0, s>>>(kin, n, 8 * pi, hist, ntiles); bnn_note_launch(); }
-            BNN_CUDA_CHECK(exclusive_scan_u32(hist, hist, (size_t)256 * ntiles, scanWs, s));
-            { k_radix_scatter<uint32_t><<<ntiles, kRT, 0, s>>>(kin, vin, kout, vout, n, 8 * pi, hist, ntiles); bnn_note_launch(); }
-            kin = kout;
-            vin = vout;
-        }
+        const unsigned ntiles = (n + kRTile - 1) / kRTile;
+        { k_grid_cell_ids<<<ntiles, kRT, 0, s>>>(pos_dev, n, bmin[0], bmin[1], bmin[2], cell_size, ncells[0], ncells[1], ncells[2],
+                                                 cell_id_dev, oor, hist, ntiles, cell_start_dev ? cells : nullptr); bnn_note_launch(); }
+        BNN_CUDA_CHECK(radix_passes<uint32_t>(cell_id_dev, n, 0, bits_below(C), keys0, sorted_idx_dev, keys1, vals1, hist, true, s));
     }
-    if(cell_start_dev) {
-        BNN_CUDA_CHECK(cudaMemsetAsync(cells, 0, C * sizeof(uint32_t), s));
-        if(n) { k_histogram<<<(n + 255) / 256, 256, 0, s>>>(cell_id_dev, n, cells); bnn_note_launch(); }
-        BNN_CUDA_CHECK(exclusive_scan_u32(cells, cell_start_dev, C, scanWs, s));
-    }
+    if(cell_start_dev) BNN_CUDA_CHECK(exclusive_scan_u32(cells, cell_start_dev, C, scanWs, s));
     BNN_CUDA_CHECK(cudaGetLastError());
     unsigned h = 0;
     BNN_CUDA_CHECK(cudaMemcpyAsync(&h, oor, sizeof(unsigned), cudaMemcpyDeviceToHost, s));

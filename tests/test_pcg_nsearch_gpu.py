@@ -348,6 +348,32 @@ def test_cell_sort_grid_sizes_bitexact(bnn, oracle_mod, nc, cell):
     assert np.array_equal(gst.cpu().numpy().view(np.uint32), start)
 
 
+@pytest.mark.parametrize("n", [1, 31, 2_047, 2_048, 2_049, 6_145, 300_001])
+@pytest.mark.parametrize("nc", [(1, 1, 1), (16, 16, 1), (257, 1, 1), (40, 41, 40), (300, 300, 200)])
+def test_cell_sort_tiles_and_digits(bnn, n, nc):
+    """Around the sort's 2048-item tiles and 8-bit digits (0 to 4 passes), points outside the
+    grid and a crowded cell among them; the allocation-free call gives the same."""
+    rng = np.random.default_rng(n)
+    ncf = np.array(nc, np.float32)
+    p = (rng.random((n, 3)) * 1.02 * ncf - 0.01 * ncf).astype(np.float32)
+    p[n // 2:] = p[n // 2]  # half of the points in one cell
+    c = np.clip(p.astype(np.int32), 0, np.array(nc) - 1)
+    out = ((p.astype(np.int32) < 0) | (p.astype(np.int32) >= np.array(nc))).any(1).sum()
+    cid = (c[:, 2].astype(np.int64) * nc[1] + c[:, 1]) * nc[0] + c[:, 0]
+    cells = nc[0] * nc[1] * nc[2]
+    pos = _dev(p)
+    calls = [bnn.load().bnn_cell_sort] + ([bnn.load().bnn_cell_sort_noalloc] if cells <= 1 << 21 else [])
+    for call in calls:
+        ids, order, start = (torch.zeros(k, dtype=torch.int32, device="cuda") for k in (n, n, cells + 1))
+        oor = C.c_uint32()
+        bnn.capi.check(call(pos.data_ptr(), n, (C.c_float * 3)(), 1.0, (C.c_int32 * 3)(*nc), ids.data_ptr(), order.data_ptr(),
+                            start.data_ptr(), C.byref(oor), None), "bnn_cell_sort")
+        assert oor.value == out
+        assert np.array_equal(ids.cpu().numpy(), cid)
+        assert np.array_equal(order.cpu().numpy(), np.argsort(cid, kind="stable"))
+        assert np.array_equal(start.cpu().numpy(), np.concatenate([[0], np.cumsum(np.bincount(cid, minlength=cells))]))
+
+
 def test_z_sort_bitexact(bnn, oracle_mod):
     pts = scenes.point_cloud(100_000, seed=3)
     z, perm = oracle_mod.z_sort(pts, np.float32(0.01))
