@@ -24,6 +24,7 @@
 #include "bnn_internal.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <cstdio>
 #include <cstring>
@@ -921,8 +922,9 @@ __device__ __forceinline__ unsigned row_code(int dz, int l, int dy, int sign, bo
 // Shared memory of a block: CH chunks.  x and 1/diag are kept there too where they fit (else
 // x stays in global memory and 1/diag is loaded ahead of every iteration's first exchange).
 template<class VT> constexpr int kRoomy = sizeof(VT) == 4 ? 3 : 2;
-template<class VT, bool COEF, int CH> struct ChunkRowsSmem {
-    static constexpr int kX = CH <= kRoomy<VT> ? CH : 1, kXRows = CH <= kRoomy<VT> ? kChunk : 1;
+template<class VT, bool COEF, int CH, bool HERE = (CH <= kRoomy<VT>)> struct ChunkRowsSmem {
+    static constexpr bool kHere = HERE;
+    static constexpr int kX = HERE ? CH : 1, kXRows = HERE ? kChunk : 1;
     VT s[CH][kChunk + 16 / sizeof(VT)];  // s[kNoRow] = 0: what a missing neighbour adds
     uint2 nb[CH][kChunk];
     float diag[CH][kChunk];
@@ -934,38 +936,124 @@ template<class VT, bool COEF, int CH> struct ChunkRowsSmem {
 template<class VT, bool COEF, int G, int K> struct ChunkSmem : ChunkRowsSmem<VT, COEF, G * K> {
     WaitSmem<VT, G * K> wait;
 };
+// A cluster's block: the pairs live in shared memory, and every block holds all packets
+constexpr int kMostCluster = 16;
+template<class VT, bool COEF> struct ClusterSmem : ChunkRowsSmem<VT, COEF, 1, true> {
+    RowPair<VT> pair[kChunk];
+    PcgPacket packets[2][kMostCluster];
+};
 // A batch's block: every group solves for a scene of its own
 template<class VT, int G, int K> struct BatchChunkSmem : ChunkRowsSmem<VT, false, G * K> {
     GroupWaitSmem<VT> wait[G];
     ChunkArgs<VT> args[G];
 };
 
-// The solve of the K chunks c0, c0 + cStep, ... by group grp of a block of G groups.  BATCH:
-// the group is one of a scene's, and waits and returns by itself; else all groups of the block
-// belong to one system and wait together.
-template<class VT, bool COEF, int G, int K, bool BATCH, class Smem>
+// Who waits for whom in chunk_solve.  kGrid: all groups of the launch belong to one system, a
+// block waits as a whole.  kScene: a group is one of a scene's groups, and waits and returns by
+// itself.  kCluster: the launch is one thread-block cluster and holds one system; pairs and
+// packets are exchanged through distributed shared memory, and the waits are cluster barriers.
+enum ChunkMode { kGrid, kScene, kCluster };
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned map_to_rank(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" : : : "memory");
+}
+// ld_pair_if from another block's (or the own) shared memory
+template<class VT> __device__ __forceinline__ RowPair<VT> ld_cluster_pair_if(unsigned addr, bool on) {
+    RowPair<VT> v{VT(0), VT(0)};
+    if constexpr(sizeof(VT) == 4)
+        asm volatile("{ .reg .pred p; setp.ne.s32 p, %3, 0; @p ld.shared::cluster.v2.f32 {%0, %1}, [%2]; }"
+                     : "+f"(v.z), "+f"(v.s) : "r"(addr), "r"((int)on) : "memory");
+    else
+        asm volatile("{ .reg .pred p; setp.ne.s32 p, %3, 0; @p ld.shared::cluster.v2.f64 {%0, %1}, [%2]; }"
+                     : "+d"(v.z), "+d"(v.s) : "r"(addr), "r"((int)on) : "memory");
+    return v;
+}
+
+// One warp: a chunk's packet to every block of the cluster
+template<class VT, bool MAX>
+__device__ __forceinline__ void cluster_publish(const double* smd, const VT* smv, PcgPacket* slot, unsigned blocks) {
+    double c;
+    VT x;
+    lane_tree<VT, MAX>(smd, smv, c, x);
+    c = __shfl_sync(0xffffffffu, c, 0);
+    if(MAX) x = __shfl_sync(0xffffffffu, x, 0);
+    const unsigned lane = threadIdx.x & 31;
+    if(lane < blocks) {
+        const unsigned to = map_to_rank(smem_addr(slot), lane);
+        asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" : : "r"(to), "l"(__double_as_longlong(c)),
+                     "l"((long long)max_bits(x)) : "memory");
+    }
+}
+// After the cluster's barrier every warp forms the sum and max of its block's copy of the
+// packets (canonical tree; the part of it past 16 chunks is 0)
+template<class VT, bool MAX>
+__device__ __forceinline__ void cluster_sum(const PcgPacket* packets, int nch, double& sum, VT& mx) {
+    const int t = threadIdx.x & 31;
+    double c = 0.0;
+    VT m = VT(0);
+    if(t < nch) {
+        c = c + __longlong_as_double((long long)packets[t].sum);
+        if(MAX) { const VT o = max_of<VT>(packets[t].max); m = m > o ? m : o; }
+    }
+#pragma unroll
+    for(int off = kMostCluster / 2; off > 0; off >>= 1) {
+        c = c + __shfl_down_sync(0xffffffffu, c, off);
+        if(MAX) { const VT o = __shfl_down_sync(0xffffffffu, m, off); m = m > o ? m : o; }
+    }
+    sum = __shfl_sync(0xffffffffu, c, 0);
+    mx = MAX ? __shfl_sync(0xffffffffu, m, 0) : m;
+}
+
+// The solve of the K chunks c0, c0 + cStep, ... by group grp of a block of G groups (kCluster:
+// one chunk a block, cStep blocks).
+template<class VT, bool COEF, int G, int K, ChunkMode MODE, class Smem>
 __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, const int grp, const int t, const int c0,
                                             const int cStep) {
     // rows whose neighbour loads are in flight together
     constexpr int kGroup = sizeof(VT) == 4 ? (G == 1 ? 8 : 4) : (G == 1 ? 4 : 2);
     constexpr int R = K * kPerLane;
-    constexpr bool kHere = G * K <= kRoomy<VT>;  // x and 1/diag in shared memory
+    constexpr bool kHere = Smem::kHere;  // x and 1/diag in shared memory
     const int n = a.n, nch = a.nch;
     unsigned* flags = &a.st->flags;
     RowPair<VT>* __restrict__ pair = a.pair;
     const VT negoff = a.negoff;
     auto chunk_of = [&](int k) { return c0 + k * cStep; };
     auto rows_of = [&](int k) { return max(min(n - chunk_of(k) * kChunk, kChunk), 0); };
+    // the pair of another row of the system, and of an own one
+    auto other_pair = [&](int row, bool on) {
+        if constexpr(MODE == kCluster) {
+            const unsigned block = (unsigned)row / kChunk % kMostCluster, l = (unsigned)row % kChunk;
+            return ld_cluster_pair_if<VT>(map_to_rank(smem_addr(S.pair) + l * (unsigned)sizeof(RowPair<VT>), on ? block : 0u), on);
+        } else return ld_pair_if(pair + row, on);
+    };
+    auto own_pair = [&](int k, int l) -> RowPair<VT>& {
+        if constexpr(MODE == kCluster) return S.pair[l];
+        else return pair[(size_t)chunk_of(k) * kChunk + l];
+    };
     auto wait = [&](auto withMax, auto acquire, const PcgPacket* slots, unsigned parity, double& sum, VT& mx) {
-        constexpr bool MAX = decltype(withMax)::value, ACQUIRE = decltype(acquire)::value;
-        if constexpr(BATCH) return group_wait<VT, MAX, ACQUIRE>(slots, nch, parity, flags, S.wait[grp], grp, t, sum, mx);
+        constexpr bool MAX = decltype(withMax)::value;
+        [[maybe_unused]] constexpr bool ACQUIRE = decltype(acquire)::value;
+        if constexpr(MODE == kCluster) {
+            cluster_barrier();
+            cluster_sum<VT, MAX>(S.packets[MAX ? 1 : 0], nch, sum, mx);
+            return true;
+        } else if constexpr(MODE == kScene)
+            return group_wait<VT, MAX, ACQUIRE>(slots, nch, parity, flags, S.wait[grp], grp, t, sum, mx);
         else return packet_wait<VT, MAX, ACQUIRE, G * K>(slots, nch, parity, flags, S.wait, sum, mx);
     };
 
     // ---- init: r = rhs, x = 0, z = D^-1 r; partial z.r and max|r| (PCGSolver.cpp:151-168)
-    if constexpr(BATCH) {
+    if constexpr(MODE == kScene) {
         if(t == 0) S.wait[grp].bad = 0;
-    } else if(threadIdx.x == 0) S.wait.bad = 0;
+    } else if constexpr(MODE == kGrid) {
+        if(threadIdx.x == 0) S.wait.bad = 0;
+    }
     VT r[R], q[R];  // q holds z from phase B to the next phase A
 #pragma unroll
     for(int k = 0; k < K; ++k) {
@@ -995,7 +1083,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
                 m = m > ab ? m : ab;
                 iv = __ldg(a.invd + e);
                 zv = iv * rv;
-                pair[e] = {zv, VT(0)};
+                own_pair(k, l) = {zv, VT(0)};
                 acc = acc + (double)zv * (double)rv;
             }
             if constexpr(kHere) {
@@ -1016,7 +1104,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         S.sum[slot][t] = acc;
         S.max[slot][t] = m;
     }
-    if constexpr(BATCH) group_sync(grp);
+    if constexpr(MODE == kScene) group_sync(grp);
     else __syncthreads();
     double rho;
     VT resid;
@@ -1025,9 +1113,12 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         // a warp of the group for each of its chunks
         if(t < 32 * K) {
             const int k = t >> 5, slot = grp * K + k, c = chunk_of(k);
-            if(c < nch)
-                packet_publish<VT, decltype(withMax)::value, decltype(release)::value>(
-                    S.sum[slot], S.max[slot], slots + (size_t)c * kPacketStride, parity);
+            constexpr bool MAX = decltype(withMax)::value;
+            if(c >= nch) return;
+            if constexpr(MODE == kCluster)
+                cluster_publish<VT, MAX>(S.sum[slot], S.max[slot], &S.packets[MAX ? 1 : 0][c], (unsigned)cStep);
+            else packet_publish<VT, MAX, decltype(release)::value>(S.sum[slot], S.max[slot],
+                                                                   slots + (size_t)c * kPacketStride, parity);
         }
     };
     publish(Yes(), Yes(), a.pkB);
@@ -1055,21 +1146,21 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         // what rows g0 .. of chunk k read from the pairs: their z neighbours, and the y
         // neighbours across the chunk's ends
         auto load_pairs = [&](int k, int g0) {
-            const RowPair<VT>* own = pair + (size_t)chunk_of(k) * kChunk;
+            const int base = chunk_of(k) * kChunk;
 #pragma unroll
             for(int u = 0; u < kGroup; ++u) {
                 const int j = g0 + u, l = t + j * kLanes;
                 nb[u] = S.nb[grp * K + k][l];
                 const int dM = (int)(nb[u].x & 0x3ffffu), dP = (int)(nb[u].y & 0x3ffffu);
-                zn[u][0] = ld_pair_if(own + (l - dM), dM != 0);
-                zn[u][1] = ld_pair_if(own + (l + dP), dP != 0);
+                zn[u][0] = other_pair(base + l - dM, dM != 0);
+                zn[u][1] = other_pair(base + l + dP, dP != 0);
                 if(j < 2) {
                     const unsigned y = nb[u].x >> 18 & 0xfffu;
-                    ye[u] = ld_pair_if(own + (l - (int)(y - kNoRow - 1u)), y > kNoRow);
+                    ye[u] = other_pair(base + l - (int)(y - kNoRow - 1u), y > kNoRow);
                 }
                 if(j >= kPerLane - 2) {
                     const unsigned y = nb[u].y >> 18 & 0xfffu;
-                    ye[u] = ld_pair_if(own + (l + (int)(y - kNoRow - 1u)), y > kNoRow);
+                    ye[u] = other_pair(base + l + (int)(y - kNoRow - 1u), y > kNoRow);
                 }
             }
         };
@@ -1078,7 +1169,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
 #pragma unroll
         for(int k = 0; k < K; ++k) {
             const uint2 e = S.nb[grp * K + k][t == 0 ? 0 : kChunk - 1];
-            xe[k] = ld_pair_if(pair + (t == 0 ? chunk_of(k) * kChunk - 1 : (chunk_of(k) + 1) * kChunk),
+            xe[k] = other_pair(t == 0 ? chunk_of(k) * kChunk - 1 : (chunk_of(k) + 1) * kChunk,
                                (t == 0 && (int)e.x < 0) || (t == kLanes - 1 && (int)e.y < 0));
         }
         load_pairs(0, 0);
@@ -1153,7 +1244,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         // ---- phase B: r -= alpha q, max|r|, z = D^-1 r, partial z.r; then x += alpha s
 #pragma unroll
         for(int k = 0; k < K; ++k) {
-            const int slot = grp * K + k, base = chunk_of(k) * kChunk;
+            const int slot = grp * K + k;
             const bool live = chunk_of(k) < nch;
             double acc = 0.0;
             VT m = VT(0);
@@ -1169,7 +1260,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
                 else iv = inv[i];
                 const VT zv = iv * rv;
                 q[i] = zv;
-                if(live) pair[base + l] = {zv, S.s[slot][l]};
+                if(live) own_pair(k, l) = {zv, S.s[slot][l]};
                 acc = acc + (double)zv * (double)rv;
             }
             S.sum[slot][t] = acc;
@@ -1230,7 +1321,24 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk(ChunkArgs<VT> a) {
     extern __shared__ __align__(16) unsigned char dynSm[];
     auto& S = *reinterpret_cast<ChunkSmem<VT, COEF, G, K>*>(dynSm);
     const int grp = (int)threadIdx.x / kLanes, t = (int)threadIdx.x % kLanes;
-    chunk_solve<VT, COEF, G, K, false>(a, S, grp, t, (int)(blockIdx.x + grp * K * gridDim.x), (int)gridDim.x);
+    chunk_solve<VT, COEF, G, K, kGrid>(a, S, grp, t, (int)(blockIdx.x + grp * K * gridDim.x), (int)gridDim.x);
+}
+
+// A system of up to 16 chunks in one cluster, a chunk per block: an exchange is a write to the
+// other blocks' shared memory and a hardware barrier, a neighbour's pair a load from their
+// shared memory, against a trip through L2 each.  us per iteration with everything around it
+// (k_pcg_chunk): FP32 2,048 rows 3.5 (4.3), 26,652 rows 3.4 (4.9); FP64 26,652 rows 4.0 (5.9);
+// the solve of a 64^3 scene 0.34 ms (0.48).  What is left is the chain of one iteration: two
+// barriers with a reduction before each, two rounds of loads.  Two or three chunks per block,
+// for up to 48, took longer than k_pcg_chunk on as many SMs as there are chunks (solve of a
+// 121 x 77 x 95 scene 0.97 ms against 0.68).
+template<class VT, bool COEF>
+__global__ void __launch_bounds__(kLanes, 1) k_pcg_cluster(ChunkArgs<VT> a) {
+    extern __shared__ __align__(16) unsigned char dynSm[];
+    auto& S = *reinterpret_cast<ClusterSmem<VT, COEF>*>(dynSm);
+    cluster_barrier();  // every block has started: its shared memory may be written
+    chunk_solve<VT, COEF, 1, 1, kCluster>(a, S, 0, (int)threadIdx.x, (int)blockIdx.x, (int)gridDim.x);
+    cluster_barrier();  // no block ends while another may still reach into it
 }
 
 // The FP32 systems of many scenes in one launch (BatchGroup: which chunks a group of 256
@@ -1251,7 +1359,7 @@ __global__ void __launch_bounds__(G * kLanes, 1) k_pcg_chunk_batch(const ChunkAr
     if(g.scene < 0) return;
     if(t == 0) S.args[grp] = scenes[g.scene];
     group_sync(grp);
-    chunk_solve<float, false, G, K, true>(S.args[grp], S, grp, t, g.chunk0, 1);
+    chunk_solve<float, false, G, K, kScene>(S.args[grp], S, grp, t, g.chunk0, 1);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1931,6 +2039,53 @@ void pcg_release(PcgWork& w) {
     w = PcgWork();
 }
 
+struct ChunkKernel {
+    const void* fn = nullptr;
+    size_t smem = 0;
+};
+template<class VT> static ChunkKernel cluster_kernel(bool coef) {
+    if(coef) return {(const void*)k_pcg_cluster<VT, true>, sizeof(ClusterSmem<VT, true>)};
+    return {(const void*)k_pcg_cluster<VT, false>, sizeof(ClusterSmem<VT, false>)};
+}
+static cudaLaunchConfig_t cluster_config(const ChunkKernel& k, int blocks, cudaLaunchAttribute* attr, cudaStream_t s) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)blocks;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)blocks);
+    c.blockDim = dim3(kLanes);
+    c.dynamicSmemBytes = k.smem;
+    c.stream = s;
+    c.attrs = attr;
+    c.numAttrs = 1;
+    return c;
+}
+static cudaError_t cluster_opt_in(const ChunkKernel& k) {
+    const cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+    if(e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+// Whether the current device can hold such a cluster (blocks of a whole SM each within one
+// GPC); asked once per device and size
+template<class VT> static bool cluster_fits(bool coef, int blocks) {
+    static std::atomic<uint32_t> known[64];  // per device: bit 2i asked, 2i + 1 the answer
+    int dev = 0;
+    if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int i = coef ? 5 : 0;  // + log2 of the blocks, 0 .. 4
+    for(int b = 1; b < blocks; b *= 2) ++i;
+    const uint32_t k = known[dev].load(std::memory_order_acquire);
+    if(k >> (2 * i) & 1u) return (k >> (2 * i + 1) & 1u) != 0u;
+    const ChunkKernel kern = cluster_kernel<VT>(coef);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(kern, blocks, &attr, nullptr);
+    int clusters = 0;
+    const bool ok = cluster_opt_in(kern) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, kern.fn, &cfg) == cudaSuccess && clusters > 0;
+    if(!ok) cudaGetLastError();
+    known[dev].fetch_or(1u << (2 * i) | (uint32_t)ok << (2 * i + 1), std::memory_order_acq_rel);
+    return ok;
+}
+
 // The shape of a chunk-resident solve of n rows: groups per block and chunks per group (0:
 // more chunks than it holds, they take turns in k_pcg_persistent).  One block per SM; as few
 // groups as hold the chunks (more registers and loads in flight for each), then two chunks per
@@ -1940,19 +2095,22 @@ void pcg_release(PcgWork& w) {
 // above).
 struct ChunkShape {
     int G = 0, K = 0;
+    int cluster = 0;  // blocks of the one cluster (k_pcg_cluster); 0: k_pcg_chunk over the grid
 };
 template<class VT> static ChunkShape chunk_shape(int n, bool coef, int numSM) {
     const int nch = (n + kChunk - 1) / kChunk;
+    // up to 16 chunks, the most blocks of a cluster: k_pcg_cluster, a power of two of blocks
+    if(nch <= kMostCluster) {
+        int blocks = 1;
+        while(blocks < nch) blocks *= 2;
+        if(cluster_fits<VT>(coef, blocks)) return ChunkShape{1, 1, blocks};
+    }
     const int per = (nch + numSM - 1) / numSM;
     if(coef) return per <= (sizeof(VT) == 4 ? 2 : 1) ? ChunkShape{per, 1} : ChunkShape{};
     const int most = sizeof(VT) == 4 ? 3 : 2;
     if(per <= most) return {per, 1};
     return per <= 2 * most ? ChunkShape{most, 2} : ChunkShape{};
 }
-struct ChunkKernel {
-    const void* fn = nullptr;
-    size_t smem = 0;
-};
 template<class VT, bool COEF, int G, int K> static ChunkKernel chunk_kernel_of() {
     return {(const void*)k_pcg_chunk<VT, COEF, G, K>, sizeof(ChunkSmem<VT, COEF, G, K>)};
 }
@@ -1991,8 +2149,6 @@ static int pcg_solve_chunk(PcgWork& w, int n, ChunkShape shape, int numSM, const
                            const VT* invd, const int32_t* nbr, const float* coef, VT negoff, VT tolFactor,
                            unsigned maxIter, VT* x, DevState* dst, DevState* hst, cudaStream_t s, PcgOutcome& out) {
     out = PcgOutcome();
-    const ChunkKernel kern = chunk_kernel<VT>(coef != nullptr, shape);
-    BNN_CUDA_CHECK(cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kern.smem));
     ChunkArgs<VT> a;
     a.n = n; a.nch = (n + kChunk - 1) / kChunk;
     a.rhsF = rhsF; a.diag = diag; a.invd = invd; a.nbr = nbr; a.coef = coef; a.negoff = negoff;
@@ -2001,8 +2157,22 @@ static int pcg_solve_chunk(PcgWork& w, int n, ChunkShape shape, int numSM, const
     a.pkA = w.packets;
     a.pkB = a.pkA + (size_t)w.nchCap * kPacketStride;
     a.st = dst;
-    BNN_CUDA_CHECK(cudaMemsetAsync(w.packets, 0, 2 * (size_t)w.nchCap * kPacketStride * sizeof(PcgPacket), s));
     void* args[] = {(void*)&a};
+    if(shape.cluster > 0) {
+        // blocks of a cluster start together and wait for no other launch: no share to hold
+        const ChunkKernel kern = cluster_kernel<VT>(coef != nullptr);
+        BNN_CUDA_CHECK(cluster_opt_in(kern));
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = cluster_config(kern, shape.cluster, &attr, s);
+        if(w.ev[0]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[0], s));
+        BNN_CUDA_CHECK(cudaLaunchKernelExC(&cfg, kern.fn, args));
+        bnn_note_launch();
+        if(w.ev[1]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[1], s));
+        return pcg_read_outcome<VT>(w, dst, hst, s, out);
+    }
+    const ChunkKernel kern = chunk_kernel<VT>(coef != nullptr, shape);
+    BNN_CUDA_CHECK(cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kern.smem));
+    BNN_CUDA_CHECK(cudaMemsetAsync(w.packets, 0, 2 * (size_t)w.nchCap * kPacketStride * sizeof(PcgPacket), s));
     const int most = numSM < kMostSM ? numSM : kMostSM, grid = a.nch < most ? a.nch : most;
     CoopShare share((long long)grid * kShareUnits, (long long)numSM * kShareUnits);
     if(w.ev[0]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[0], s));

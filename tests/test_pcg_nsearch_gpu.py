@@ -246,14 +246,16 @@ def _csr_of(nbr, diag, off):
     return start, cols[keep].astype(np.uint32), vals[keep]
 
 
-# Edges of the chunk-resident solve on 148 SMs: of a 2048-row chunk; of one, two, three and six
-# chunks per SM (FP32) and of one, two and four (FP64); of the rows its 8-byte records hold (512
-# cells along x, 2^18 - 1 a plane), past which the other kernels take over.
+# Edges of the chunk-resident solve on 148 SMs: of a 2048-row chunk; of the 16 chunks of one
+# cluster; of one, two, three and six chunks per SM (FP32) and of one, two and four (FP64); of the
+# rows its 8-byte records hold (512 cells along x, 2^18 - 1 a plane), past which the other kernels
+# take over.
 _SM = 148 * 2048
 
 
 @pytest.mark.parametrize("nx,ny,n", [
     (1, 1, 1), (7, 5, 2047), (7, 5, 2048), (7, 5, 2049), (512, 3, 4 * 2048 + 1), (513, 3, 4 * 2048 + 1),
+    (31, 29, 15 * 2048 + 1), (31, 29, 16 * 2048), (31, 29, 16 * 2048 + 1),
     (31, 29, 32 * 2048), (31, 29, 33 * 2048 + 5), (64, 80, _SM), (64, 80, _SM + 1), (101, 90, 2 * _SM), (101, 90, 2 * _SM + 1),
     (102, 154, 3 * _SM + 1), (102, 154, 4 * _SM), (102, 154, 4 * _SM + 1), (260, 260, 6 * _SM), (260, 260, 6 * _SM + 1),
     (512, 511, 600_000), (512, 512, 600_000)])
