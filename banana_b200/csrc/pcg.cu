@@ -605,18 +605,18 @@ __device__ __forceinline__ int4 pack_row(int r, const int32_t nb[6], float diag)
 // in the canonical order; a block has passed when it has seen all of them.  A packet's max
 // carries the parity of its exchange in the top bit (a block is at most one exchange ahead of
 // the slowest, so one bit tells old from new; the packets start zeroed).  Packets lie 128
-// bytes apart so that the polls of all blocks spread over the L2 slices.  The x update
-// overlaps the second wait.
+// bytes apart so that the polls of all blocks spread over the L2 slices; the word behind a
+// packet says that its chunk's pairs can be read (kSplit).  The x update overlaps the second
+// wait.
 //
-// What bounds it: up to a chunk per SM the latency of the two exchanges (about 1.5 us each:
-// the release of the pairs, a packet's way through L2, the FP64 tree) and of one round of
-// neighbour loads; at six chunks per SM the instructions of phase A, the pair stores of phase
-// B and the FP32-to-FP64 conversions of the products (16 a clock and SM).  One block per SM
-// instead of three: one poller per SM, and a group's registers can hold a whole chunk's loads.
-// Measured, us per iteration with everything around it (k_pcg_persistent before): FP32 26,652
-// rows 4.96 (9.41), 161,057 rows 5.51 (9.63), 315,698 6.66 (10.96), 705,846 9.05 (13.81),
-// 1,283,026 14.7 (22.1), 1,736,304 16.9 (22.9); FP64 26,652 rows 5.88 (12.8), 315,698 8.10
-// (15.2), 705,846 14.3 (19.8).
+// What bounds it: up to a chunk per SM the latency of the two exchanges (a packet's way through
+// L2, the FP64 trees on both sides, the pairs' way to L2) and of one round of neighbour loads; at
+// six chunks per SM the instructions of phase A, the pair stores of phase B and the
+// FP32-to-FP64 conversions of the products (16 a clock and SM).  One block per SM instead of
+// three: one poller per SM, and a group's registers can hold a whole chunk's loads.
+// Measured, us per iteration with everything around it (k_pcg_persistent before): FP32 161,057
+// rows 4.86 (9.63), 315,698 6.2 (10.96), 705,846 8.2 (13.81), 1,283,026 15.3 (22.1), 1,736,304
+// 17.5 (22.9); FP64 315,698 7.4 (15.2), 705,846 13.8 (19.8).
 // ---------------------------------------------------------------------------------
 template<class VT> struct alignas(2 * sizeof(VT)) RowPair {
     VT z, s;
@@ -688,6 +688,15 @@ __device__ __forceinline__ PcgPacket ld_acquire_packet(const PcgPacket* p) {
                  : "=l"(v.sum), "=l"(v.max) : "l"(p) : "memory");
     return v;
 }
+// The word behind a packet: its chunk's pairs of an exchange of this parity are visible
+__device__ __forceinline__ void st_ready(PcgPacket* slot, unsigned parity) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" : : "l"(slot + 1), "r"(parity) : "memory");
+}
+__device__ __forceinline__ unsigned ld_acquire_ready(const PcgPacket* slot) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(slot + 1) : "memory");
+    return v;
+}
 
 struct Yes { static constexpr bool value = true; };
 struct No { static constexpr bool value = false; };
@@ -736,25 +745,30 @@ __device__ __forceinline__ void packet_publish(const double* smd, const VT* smv,
     }
 }
 
-// Polls one packet per lane (where `on`) until all of the warp's carry `parity`; false when
-// the bounded wait gave up.
-template<bool ACQUIRE>
-__device__ __forceinline__ bool packet_poll(const PcgPacket* slot, bool on, unsigned parity, PcgPacket& pk) {
+// Tries until `got` is true in every lane of the warp; false when the bounded wait gave up
+template<class F> __device__ __forceinline__ bool warp_poll(F got) {
     const BarrierLimit lim = solve_barrier_limit();
     unsigned spins = 0;
     unsigned long long t0 = 0;
     while(true) {
-        if(on) {
-            pk = ACQUIRE ? ld_acquire_packet(slot) : ld_relaxed_packet(slot);
-            on = (unsigned)(pk.max >> 63) != parity;
-        }
-        if(!__any_sync(0xffffffffu, on)) return true;
+        if(__all_sync(0xffffffffu, got())) return true;
         ++spins;
         if(spins == lim.minSpins) t0 = global_ns();
         const bool late = spins >= lim.maxSpins ||
                           (spins > lim.minSpins && (spins & 255u) == 0u && global_ns() - t0 >= lim.ns);
         if(__any_sync(0xffffffffu, late)) return false;
     }
+}
+// One packet per lane (where `on`), until all carry `parity`
+template<bool ACQUIRE>
+__device__ __forceinline__ bool packet_poll(const PcgPacket* slot, bool on, unsigned parity, PcgPacket& pk) {
+    return warp_poll([&] {
+        if(on) {
+            pk = ACQUIRE ? ld_acquire_packet(slot) : ld_relaxed_packet(slot);
+            on = (unsigned)(pk.max >> 63) != parity;
+        }
+        return !on;
+    });
 }
 
 // One warp: the packets of up to 32 chunks, their canonical sum and max (valid in lane 0);
@@ -834,6 +848,61 @@ __device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, uns
         VT m;
         if(!warp_packets<VT, MAX, ACQUIRE>(slots, nch, parity, c, m)) W.bad = 1;
         if(t == 0) { W.sum = c; W.max = m; }
+    }
+    __syncthreads();
+    sum = W.sum;
+    mx = W.max;
+    if(W.bad == 0) return true;
+    if(t == 0) atomicOr(flags, BNN_FLAG_TIMEOUT);
+    return false;
+}
+
+// packet_wait where the sums come ahead of the pairs (kSplit): the first 256 threads poll the
+// packets, chunk c the lane c mod 256 of the canonical tree; with PAIRS the warps that have no
+// packets wait for the words that say the pairs are visible.  kPer: packets of a lane.
+__device__ __forceinline__ void front_sync(int threads) { asm volatile("bar.sync 15, %0;" : : "r"(threads) : "memory"); }
+template<class VT, bool MAX, bool PAIRS, int kPer, int CH>
+__device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
+                                                  WaitSmem<VT, CH>& W, double& sum, VT& mx) {
+    const int t = threadIdx.x, front = min((nch + 31) & ~31, kLanes);
+    if(t < front) {
+        PcgPacket pk[kPer];
+        unsigned late = (1u << kPer) - 1u;
+#pragma unroll
+        for(int i = 0; i < kPer; ++i)
+            if(t + i * kLanes >= nch) late &= ~(1u << i);
+        if(!warp_poll([&] {
+#pragma unroll
+               for(int i = 0; i < kPer; ++i)
+                   if(late >> i & 1u) pk[i] = ld_relaxed_packet(slots + (size_t)(t + i * kLanes) * kPacketStride);
+#pragma unroll
+               for(int i = 0; i < kPer; ++i)
+                   if((late >> i & 1u) && (unsigned)(pk[i].max >> 63) == parity) late &= ~(1u << i);
+               return late == 0u;
+           })) W.bad = 1;
+        double c = 0.0;
+        VT m = VT(0);
+#pragma unroll
+        for(int i = 0; i < kPer; ++i)
+            if(t + i * kLanes < nch) {
+                c = c + __longlong_as_double((long long)pk[i].sum);
+                if(MAX) { const VT o = max_of<VT>(pk[i].max); m = m > o ? m : o; }
+            }
+        W.lanes[t] = c;
+        if(MAX) W.lanesMax[t] = m;
+        front_sync(front);  // past it the lanes are 0
+        if(t < 32) {
+            lane_tree<VT, MAX>(W.lanes, W.lanesMax, c, m);
+            if(t == 0) { W.sum = c; W.max = m; }
+        }
+    } else if constexpr(PAIRS) {
+        for(int c = t - front; c < ((nch + 31) & ~31); c += (int)blockDim.x - front) {
+            bool on = c < nch;
+            if(!warp_poll([&] {
+                   if(on) on = ld_acquire_ready(slots + (size_t)c * kPacketStride) != parity;
+                   return !on;
+               })) { W.bad = 1; break; }
+        }
     }
     __syncthreads();
     sum = W.sum;
@@ -1036,6 +1105,14 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         if constexpr(MODE == kCluster) return S.pair[l];
         else return pair[(size_t)chunk_of(k) * kChunk + l];
     };
+    // Split: an iteration's second exchange passes sums and pairs.  The sums go out at once, and
+    // another warp waits for the pairs to reach L2 and says so in a word of its own: both ways
+    // are taken at the same time, where a released packet takes them in turn.  Measured, us per
+    // iteration with everything around it (without): FP32 79 chunks 4.86 (5.44), 226 6.6 (7.4),
+    // 345 8.2 (8.8); FP64 79 5.64 (6.30), 226 7.9 (9.0).  With two chunks per group the longer
+    // wait costs registers that spill (627 chunks 18.0 against 15.4): those release the packets.
+    // A scene of a batch shares its SM with others that fill the wait (no difference).
+    constexpr bool kSplit = MODE == kGrid && K == 1;
     auto wait = [&](auto withMax, auto acquire, const PcgPacket* slots, unsigned parity, double& sum, VT& mx) {
         constexpr bool MAX = decltype(withMax)::value;
         [[maybe_unused]] constexpr bool ACQUIRE = decltype(acquire)::value;
@@ -1045,7 +1122,14 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
             return true;
         } else if constexpr(MODE == kScene)
             return group_wait<VT, MAX, ACQUIRE>(slots, nch, parity, flags, S.wait[grp], grp, t, sum, mx);
-        else return packet_wait<VT, MAX, ACQUIRE, G * K>(slots, nch, parity, flags, S.wait, sum, mx);
+        else {
+            if constexpr(kSplit) {
+                static_assert(G * kMostSM <= 2 * kLanes, "packets of a lane");
+                if(G == 1 || (G == 2 && nch <= kLanes))
+                    return packet_wait_split<VT, MAX, ACQUIRE, 1>(slots, nch, parity, flags, S.wait, sum, mx);
+                return packet_wait_split<VT, MAX, ACQUIRE, 2>(slots, nch, parity, flags, S.wait, sum, mx);
+            } else return packet_wait<VT, MAX, ACQUIRE, G * K>(slots, nch, parity, flags, S.wait, sum, mx);
+        }
     };
 
     // ---- init: r = rhs, x = 0, z = D^-1 r; partial z.r and max|r| (PCGSolver.cpp:151-168)
@@ -1053,6 +1137,10 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         if(t == 0) S.wait[grp].bad = 0;
     } else if constexpr(MODE == kGrid) {
         if(threadIdx.x == 0) S.wait.bad = 0;
+        if(threadIdx.x < kLanes) {  // the lanes that no chunk fills
+            S.wait.lanes[threadIdx.x] = 0.0;
+            S.wait.lanesMax[threadIdx.x] = VT(0);
+        }
     }
     VT r[R], q[R];  // q holds z from phase B to the next phase A
 #pragma unroll
@@ -1110,15 +1198,20 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
     VT resid;
     unsigned parity = 1;  // of this iteration's exchanges
     auto publish = [&](auto withMax, auto release, PcgPacket* slots) {
-        // a warp of the group for each of its chunks
+        // a warp of the group for each of its chunks, and one for their pairs (split)
+        constexpr bool MAX = decltype(withMax)::value, RELEASE = decltype(release)::value;
         if(t < 32 * K) {
             const int k = t >> 5, slot = grp * K + k, c = chunk_of(k);
-            constexpr bool MAX = decltype(withMax)::value;
             if(c >= nch) return;
+            [[maybe_unused]] PcgPacket* to = slots + (size_t)c * kPacketStride;
             if constexpr(MODE == kCluster)
                 cluster_publish<VT, MAX>(S.sum[slot], S.max[slot], &S.packets[MAX ? 1 : 0][c], (unsigned)cStep);
-            else packet_publish<VT, MAX, decltype(release)::value>(S.sum[slot], S.max[slot],
-                                                                   slots + (size_t)c * kPacketStride, parity);
+            else packet_publish<VT, MAX, RELEASE && !kSplit>(S.sum[slot], S.max[slot], to, parity);
+        } else if(kSplit && RELEASE && t == 32 * K) {
+            __threadfence();
+#pragma unroll
+            for(int k = 0; k < K; ++k)
+                if(chunk_of(k) < nch) st_ready(slots + (size_t)chunk_of(k) * kPacketStride, parity);
         }
     };
     publish(Yes(), Yes(), a.pkB);
