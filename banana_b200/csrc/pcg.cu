@@ -615,22 +615,13 @@ __device__ __forceinline__ int4 pack_row(int r, const int32_t nb[6], float diag)
 // FP32-to-FP64 conversions of the products (16 a clock and SM).  One block per SM instead of
 // three: one poller per SM, and a group's registers can hold a whole chunk's loads.
 // Measured, us per iteration with everything around it (k_pcg_persistent before): FP32 161,057
-// rows 4.86 (9.63), 315,698 6.2 (10.96), 705,846 8.2 (13.81), 1,283,026 15.3 (22.1), 1,736,304
-// 17.5 (22.9); FP64 315,698 7.4 (15.2), 705,846 13.8 (19.8).
+// rows 4.86 (9.63), 315,698 6.2 (10.96), 705,846 8.2 (13.81), 1,283,026 14.8 (22.1), 1,736,304
+// 17.0 (22.9); FP64 315,698 7.4 (15.2), 705,846 13.8 (19.8).
 // ---------------------------------------------------------------------------------
 template<class VT> struct alignas(2 * sizeof(VT)) RowPair {
     VT z, s;
 };
-template<class VT> __device__ __forceinline__ RowPair<VT> ld_pair(const RowPair<VT>* p) {
-    if constexpr(sizeof(VT) == 4) {
-        const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
-        return {v.x, v.y};
-    } else {
-        const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
-        return {v.x, v.y};
-    }
-}
-// ld_pair where `on`, zeros elsewhere, as one predicated load (a branch around each of a
+// A pair where `on`, zeros elsewhere, as one predicated load (a branch around each of a
 // row's loads costs more than the load)
 template<class VT> __device__ __forceinline__ RowPair<VT> ld_pair_if(const RowPair<VT>* p, bool on) {
     RowPair<VT> v{VT(0), VT(0)};
@@ -796,11 +787,9 @@ __device__ __forceinline__ bool warp_packets(const PcgPacket* slots, int nch, un
 }
 
 // Second half of an exchange: waits for every chunk's packet of this parity and gives the
-// canonical sum and max (as reduce_partials_bcast) to every thread of the block.  Up to 32
-// chunks are polled by warp 0, which then needs no shared memory for their sum; more by all
-// threads, through the W's arrays.  ACQUIRE: what the other blocks released is visible.  False
-// when the bounded wait gave up (the timeout flag is set).
-constexpr int kWarpPackets = 32;
+// canonical sum and max (as reduce_partials_bcast) to every thread of the block: all
+// threads poll, the sums go through the W's arrays.  ACQUIRE: what the other blocks released is
+// visible.  False when the bounded wait gave up (the timeout flag is set).
 constexpr int kMostSM = 160;  // SMs a chunk-resident solve is spread over at most
 template<class VT, int CH> struct WaitSmem {
     double part[CH * kMostSM];  // the chunks' sums and maxima as polled
@@ -815,39 +804,32 @@ template<class VT, bool MAX, bool ACQUIRE, int CH>
 __device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
                                             WaitSmem<VT, CH>& W, double& sum, VT& mx) {
     const int t = threadIdx.x;
-    if(nch > kWarpPackets) {
-        // whole warps stay in the loop (the poll votes)
-        for(int c = t; c < ((nch + 31) & ~31); c += (int)blockDim.x) {
-            PcgPacket pk;
-            if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad = 1; break; }
-            if(c < nch) {
-                W.part[c] = __longlong_as_double((long long)pk.sum);
-                if(MAX) W.partMax[c] = max_of<VT>(pk.max);
-            }
+    // whole warps stay in the loop (the poll votes)
+    for(int c = t; c < ((nch + 31) & ~31); c += (int)blockDim.x) {
+        PcgPacket pk;
+        if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad = 1; break; }
+        if(c < nch) {
+            W.part[c] = __longlong_as_double((long long)pk.sum);
+            if(MAX) W.partMax[c] = max_of<VT>(pk.max);
         }
-        __syncthreads();
-        if(t < kLanes) {
-            double acc = 0.0;
-            VT m = VT(0);
-            for(int c = t; c < nch; c += kLanes) {
-                acc = acc + W.part[c];
-                if(MAX) { const VT o = W.partMax[c]; m = m > o ? m : o; }
-            }
-            W.lanes[t] = acc;
-            if(MAX) W.lanesMax[t] = m;
-            group_sync(0);
+    }
+    __syncthreads();
+    if(t < kLanes) {
+        double acc = 0.0;
+        VT m = VT(0);
+        for(int c = t; c < nch; c += kLanes) {
+            acc = acc + W.part[c];
+            if(MAX) { const VT o = W.partMax[c]; m = m > o ? m : o; }
         }
-        if(t < 32) {
-            double c;
-            VT x;
-            lane_tree<VT, MAX>(W.lanes, W.lanesMax, c, x);
-            if(t == 0) { W.sum = c; W.max = x; }
-        }
-    } else if(t < 32) {
+        W.lanes[t] = acc;
+        if(MAX) W.lanesMax[t] = m;
+        group_sync(0);
+    }
+    if(t < 32) {
         double c;
-        VT m;
-        if(!warp_packets<VT, MAX, ACQUIRE>(slots, nch, parity, c, m)) W.bad = 1;
-        if(t == 0) { W.sum = c; W.max = m; }
+        VT x;
+        lane_tree<VT, MAX>(W.lanes, W.lanesMax, c, x);
+        if(t == 0) { W.sum = c; W.max = x; }
     }
     __syncthreads();
     sum = W.sum;
@@ -913,7 +895,9 @@ __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nc
 }
 
 // packet_wait for one group on its own (a scene of a batch): the group polls its scene's
-// packets, and no other group waits for it
+// packets, and no other group waits for it.  Up to 32 chunks are polled by its first warp, which
+// then needs no shared memory for their sum.
+constexpr int kWarpPackets = 32;
 template<class VT> struct GroupWaitSmem {
     double lanes[kLanes];
     VT lanesMax[kLanes];
