@@ -55,10 +55,10 @@ N_GRID = 256
 METRIC = "particle-steps/s at 256^3 FLIP (1e-6 rel residual)"
 UNIT = "particle-steps/s"
 WORKLOAD = "flip_dam_break_256"
-# DRAM bytes (read + write) per PCG iteration of k_pcg_persistent at 1.59M rows, from an ncu
-# capture of the standalone solve at that row count (`--workload pcg`: 835.7 MB over 300
-# iterations); a launch's traffic is this times its iterations
-PCG_TRAFFIC_PER_ITER = 835.7e6 / 300
+# DRAM bytes (read + write) per PCG iteration at 1.59M rows, from ncu captures of the standalone
+# solve at that row count (`--workload pcg`: 156.5 and 835.7 MB over 300 iterations); a launch's
+# traffic is this times its iterations
+PCG_TRAFFIC_PER_ITER = {"k_pcg_chunk": 156.5e6 / 300, "k_pcg_persistent": 835.7e6 / 300}
 
 
 PCG_MODE = {"fp32": 0, "fp64": 1, "refined": 2}
@@ -70,6 +70,17 @@ def _pcg_flags(args) -> int:
     """BNN_PCG_SINGLE_REDUCTION when the single-reduction form is asked for; the default is
     PCGSolver's step order (two reductions per iteration)"""
     return 0x10 if getattr(args, "pcg_steps", "two") == "single" else 0
+
+
+def _pcg_kernel(args, rows: float) -> str:
+    """The kernel that solves so many rows: up to 16 chunks of 2048 fit in one cluster, up to 6 per
+    SM on the chip in FP32 (also inside the refined solve), 4 in FP64"""
+    if _pcg_flags(args):
+        return "k_pcg_cg1"
+    if rows <= 16 * 2048:
+        return "k_pcg_cluster"
+    most = 4 if args.pcg_mode == "fp64" else 6
+    return "k_pcg_chunk" if rows <= most * 148 * 2048 else "k_pcg_persistent"
 
 
 def _config(pcg_mode: str, cfg: dict | None = None, pcg_text: str | None = None):
@@ -398,20 +409,22 @@ def run_ours(args, ws, rank, local):
                          f"solver in reference arithmetic order, OpenMP {threads} threads, {sec:.1f} s"}
 
     if rank == 0:
+        pcg_kernel = _pcg_kernel(args, max(rows))
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": t_max / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32", "data": "synthetic (seeded dam break, seed 42)",
             "config": dict(_config(pcg_mode, cfg), particles=npart, solver=args.solver.upper(),
                            workload=WORKLOAD if args.solver == "flip" else f"{args.solver}_dam_break_256"),
-            "roofline": {"bound": "hbm", "kernel": "k_pcg_persistent (whole Jacobi PCG solve, one launch per step)",
+            "roofline": {"bound": "hbm", "kernel": f"{pcg_kernel} (whole Jacobi PCG solve, one launch per step)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "algorithmic_bytes": "52 B per active row per PCG iteration (x, r, z, s, q, 1/diag and "
                                               "the row's matrix data once each)",
-                         "traffic": PCG_TRAFFIC_PER_ITER * iters / args.steps,
+                         "traffic": PCG_TRAFFIC_PER_ITER[pcg_kernel] * iters / args.steps
+                         if pcg_kernel in PCG_TRAFFIC_PER_ITER else None,
                          "traffic_note": "ncu DRAM bytes per iteration of the same kernel at the same row count "
-                                         "(standalone capture) x iterations per launch; the solve is L2-resident"},
+                                         "(standalone capture) x iterations per launch; the solve stays on the chip"},
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": int(launches),
             "clocks": clk,
             "detail": {"tile_tuning": capi.tile_tuning(),
@@ -891,8 +904,8 @@ def run_pcg(args, ws, rank, local):
                 "data": "synthetic (box of fluid cells, random rhs, seed 1)",
                 "config": {"workload": "pcg_box_102x153x102", "rows": n,
                            "pcg": f"Jacobi, {args.pcg_mode}, {args.pcg_steps} reduction step order",
-                           "layout": "grid rows (packed 16-byte records)"},
-                "roofline": {"bound": "hbm", "kernel": "k_pcg_persistent", "achieved": achieved, "peak": peak,
+                           "layout": "grid rows"},
+                "roofline": {"bound": "hbm", "kernel": _pcg_kernel(args, n), "achieved": achieved, "peak": peak,
                              "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                              "algorithmic_bytes": "52 B per row per iteration", "traffic": None},
                 "gpu_launches": int(launches)}
