@@ -357,7 +357,7 @@ constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
 // Bound by instruction issue: about 9 per point and 32 candidates, 20 when writing, against 15
 // per point and candidate (and its store through a shared buffer) with a thread per point that
 // walks the candidates alone.  Measured, whole bnn_neighbors call: 4M points and 933 M entries
-// 8.70 ms (11.5 with a thread per point), 20,011 points 0.335 ms (0.617).
+// 8.53 ms (11.5 with a thread per point), 20,011 points 0.293 ms (0.617).
 constexpr int kNsWarps = 4;  // warps per block: they end at different times
 template<int P, bool WRITE>
 __global__ void __launch_bounds__(kNsWarps * 32) k_ns_pairs(const float4* __restrict__ sp, const uint32_t* __restrict__ scid,

@@ -15,7 +15,9 @@
 // shuffles instead of loads.  Record {y, zm, zp, diag}: y = dy- | dy+ << 16 (row distances
 // of the -y / +y neighbours, 0 = none), zm = dz- | (has -x) << 31, zp = dz+ | (has +x) << 31.
 //
-// The solve is one persistent cooperative kernel; every iteration works in the canonical
+// A system whose chunks fit on the chip is solved by k_pcg_cluster or k_pcg_chunk (below), from
+// the compact rows.  Beyond that the solve is k_pcg_persistent, one persistent cooperative
+// kernel on the packed ones.  In all of them every iteration works in the canonical
 // 2048-row chunk layout so the FP64 dot products are bit-reproducible:
 //   phase A: s = z + beta*s_old formed on the fly (double buffered), q = A s, partial s.q;
 //   grid barrier; every block reduces the partials to the same alpha;
