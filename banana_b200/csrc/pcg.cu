@@ -798,18 +798,23 @@ template<class VT, int CH> struct WaitSmem {
     VT partMax[CH * kMostSM];
     double lanes[kLanes];       // ... of the 256 lanes of the canonical tree
     VT lanesMax[kLanes];
-    double sum;                 // the result
-    VT max;
-    int bad;                    // a wait gave up
+    // The result, and whether the wait gave up: a slot for each of an iteration's two exchanges
+    // (MAX: the second).  A group without a chunk publishes nothing, so no packet says that its
+    // warps have read a wait's result before the next wait writes its own; a slot is written again
+    // only after the other exchange's closing barrier, which every reader has reached by then.
+    double sum[2];
+    VT max[2];
+    int bad[2];
 };
 template<class VT, bool MAX, bool ACQUIRE, int CH>
 __device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
                                             WaitSmem<VT, CH>& W, double& sum, VT& mx) {
+    constexpr int X = MAX ? 1 : 0;
     const int t = threadIdx.x;
     // whole warps stay in the loop (the poll votes)
     for(int c = t; c < ((nch + 31) & ~31); c += (int)blockDim.x) {
         PcgPacket pk;
-        if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad = 1; break; }
+        if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad[X] = 1; break; }
         if(c < nch) {
             W.part[c] = __longlong_as_double((long long)pk.sum);
             if(MAX) W.partMax[c] = max_of<VT>(pk.max);
@@ -831,12 +836,12 @@ __device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, uns
         double c;
         VT x;
         lane_tree<VT, MAX>(W.lanes, W.lanesMax, c, x);
-        if(t == 0) { W.sum = c; W.max = x; }
+        if(t == 0) { W.sum[X] = c; W.max[X] = x; }
     }
     __syncthreads();
-    sum = W.sum;
-    mx = W.max;
-    if(W.bad == 0) return true;
+    sum = W.sum[X];
+    mx = W.max[X];
+    if(W.bad[X] == 0) return true;
     if(t == 0) atomicOr(flags, BNN_FLAG_TIMEOUT);
     return false;
 }
@@ -848,6 +853,7 @@ __device__ __forceinline__ void front_sync(int threads) { asm volatile("bar.sync
 template<class VT, bool MAX, bool PAIRS, int kPer, int CH>
 __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
                                                   WaitSmem<VT, CH>& W, double& sum, VT& mx) {
+    constexpr int X = MAX ? 1 : 0;
     const int t = threadIdx.x, front = min((nch + 31) & ~31, kLanes);
     if(t < front) {
         PcgPacket pk[kPer];
@@ -863,7 +869,7 @@ __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nc
                for(int i = 0; i < kPer; ++i)
                    if((late >> i & 1u) && (unsigned)(pk[i].max >> 63) == parity) late &= ~(1u << i);
                return late == 0u;
-           })) W.bad = 1;
+           })) W.bad[X] = 1;
         double c = 0.0;
         VT m = VT(0);
 #pragma unroll
@@ -877,7 +883,7 @@ __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nc
         front_sync(front);  // past it the lanes are 0
         if(t < 32) {
             lane_tree<VT, MAX>(W.lanes, W.lanesMax, c, m);
-            if(t == 0) { W.sum = c; W.max = m; }
+            if(t == 0) { W.sum[X] = c; W.max[X] = m; }
         }
     } else if constexpr(PAIRS) {
         for(int c = t - front; c < ((nch + 31) & ~31); c += (int)blockDim.x - front) {
@@ -885,13 +891,13 @@ __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nc
             if(!warp_poll([&] {
                    if(on) on = ld_acquire_ready(slots + (size_t)c * kPacketStride) != parity;
                    return !on;
-               })) { W.bad = 1; break; }
+               })) { W.bad[X] = 1; break; }
         }
     }
     __syncthreads();
-    sum = W.sum;
-    mx = W.max;
-    if(W.bad == 0) return true;
+    sum = W.sum[X];
+    mx = W.max[X];
+    if(W.bad[X] == 0) return true;
     if(t == 0) atomicOr(flags, BNN_FLAG_TIMEOUT);
     return false;
 }
@@ -1122,7 +1128,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
     if constexpr(MODE == kScene) {
         if(t == 0) S.wait[grp].bad = 0;
     } else if constexpr(MODE == kGrid) {
-        if(threadIdx.x == 0) S.wait.bad = 0;
+        if(threadIdx.x == 0) S.wait.bad[0] = S.wait.bad[1] = 0;
         if(threadIdx.x < kLanes) {  // the lanes that no chunk fills
             S.wait.lanes[threadIdx.x] = 0.0;
             S.wait.lanesMax[threadIdx.x] = VT(0);

@@ -273,6 +273,23 @@ def test_pcg_chunk_edges_match_oracle(bnn, oracle_mod, nx, ny, n, mode, omode):
         assert np.array_equal(x, xo)
 
 
+@pytest.mark.parametrize("chunks", [155, 195, 345])
+@pytest.mark.parametrize("mode,omode", [("fp32", 0), ("fp64", 1)])
+def test_pcg_groups_without_a_chunk_match_oracle(bnn, oracle_mod, chunks, mode, omode):
+    """Chunk counts that leave groups of the last blocks without work (two or three groups a block on
+    148 SMs): they take every wait's result all the same, over many exchanges."""
+    n = chunks * 2048 - 3
+    nbr, diag, rhs = _first_cells(64, 80, n, seed=chunks)
+    off = -float(np.float32(0.004))
+    x, st = bnn.pcg_solve_7pt(diag, nbr, off, rhs, 1e-6, 60, mode=mode)
+    xo, so = oracle_mod.pcg(*_csr_of(nbr, diag, off), rhs, 1e-6, 60, omode)
+    assert st["iterations"] == so["iterations"] == 60
+    if mode == "fp32":
+        assert np.array_equal(x.astype(np.float32), xo.astype(np.float32))
+    else:
+        assert np.array_equal(x, xo)
+
+
 def test_barrier_wait_gives_up_and_device_stays_usable(bnn, oracle_mod):
     """A block waiting at a barrier that nothing completes (sized for two blocks, one
     launched) gives up after its limit and reports a timeout; the device then solves a
