@@ -598,9 +598,10 @@ __device__ __forceinline__ int4 pack_row(int r, const int32_t nb[6], float diag)
 // whole solve and keeps what its own rows need on the chip: r and z / q in registers, s and
 // the row records in shared memory.  Only what other blocks read crosses L2 on the critical
 // path: a pair {z, s} per row, written once per iteration (phase B) and read by its z
-// neighbours and across chunk ends (phase A).  One buffer is enough: all reads lie between
-// the second exchange and the next first one, all writes between the first and the second.
-// The x and y neighbours inside a chunk are read from shared memory.
+// neighbours and across chunk ends (phase A).  The pairs are double-buffered by the exchange's
+// parity: the second exchange, which passes them on, releases and acquires, the first does not,
+// so a buffer is written again only after a second exchange that followed its reads.  The x and
+// y neighbours inside a chunk are read from shared memory.
 //
 // The grid barriers are merged with the reductions: a group publishes a chunk's partial sum
 // and max as one 16-byte packet, and every block polls the packets of all chunks and adds them
@@ -617,8 +618,10 @@ __device__ __forceinline__ int4 pack_row(int r, const int32_t nb[6], float diag)
 // FP32-to-FP64 conversions of the products (16 a clock and SM).  One block per SM instead of
 // three: one poller per SM, and a group's registers can hold a whole chunk's loads.
 // Measured, us per iteration with everything around it (k_pcg_persistent before): FP32 161,057
-// rows 4.86 (9.63), 315,698 6.2 (10.96), 705,846 8.2 (13.81), 1,283,026 14.8 (22.1), 1,736,304
-// 17.0 (22.9); FP64 315,698 7.4 (15.2), 705,846 13.8 (19.8).
+// rows 5.0 (9.63), 315,698 6.25 (10.96), 705,846 8.3 (13.81), 1,283,026 15.1 (22.1), 1,736,304
+// 17.3 (22.9); FP64 315,698 7.4 (15.2), 705,846 13.9 (19.8).  One buffer of pairs, whose rewriting
+// only the order of loads and dependent stores keeps off its readers: 0 to 3 % less (705,846 rows
+// 8.15, 1,736,304 16.8); one buffer and a first exchange that releases and acquires: 8.95, 17.95.
 // ---------------------------------------------------------------------------------
 template<class VT> struct alignas(2 * sizeof(VT)) RowPair {
     VT z, s;
@@ -962,7 +965,8 @@ template<class VT> struct ChunkArgs {
     VT tolFactor;
     unsigned maxIter;
     VT* x;
-    RowPair<VT>* pair;
+    RowPair<VT>* pair;  // two buffers of pairStride rows
+    int pairStride;
     PcgPacket *pkA, *pkB;  // nch packets each, zeroed
     DevState* st;
 };
@@ -1083,6 +1087,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
     const int n = a.n, nch = a.nch;
     unsigned* flags = &a.st->flags;
     RowPair<VT>* __restrict__ pair = a.pair;
+    int buf = 0;  // where the buffer of the last second exchange starts
     const VT negoff = a.negoff;
     auto chunk_of = [&](int k) { return c0 + k * cStep; };
     auto rows_of = [&](int k) { return max(min(n - chunk_of(k) * kChunk, kChunk), 0); };
@@ -1091,17 +1096,17 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         if constexpr(MODE == kCluster) {
             const unsigned block = (unsigned)row / kChunk % kMostCluster, l = (unsigned)row % kChunk;
             return ld_cluster_pair_if<VT>(map_to_rank(smem_addr(S.pair) + l * (unsigned)sizeof(RowPair<VT>), on ? block : 0u), on);
-        } else return ld_pair_if(pair + row, on);
+        } else return ld_pair_if(pair + (row + buf), on);
     };
     auto own_pair = [&](int k, int l) -> RowPair<VT>& {
         if constexpr(MODE == kCluster) return S.pair[l];
-        else return pair[(size_t)chunk_of(k) * kChunk + l];
+        else return pair[chunk_of(k) * kChunk + l + buf];
     };
     // Split: an iteration's second exchange passes sums and pairs.  The sums go out at once, and
     // another warp waits for the pairs to reach L2 and says so in a word of its own: both ways
     // are taken at the same time, where a released packet takes them in turn.  Measured, us per
-    // iteration with everything around it (without): FP32 79 chunks 4.86 (5.44), 226 6.6 (7.4),
-    // 345 8.2 (8.8); FP64 79 5.64 (6.30), 226 7.9 (9.0).  With two chunks per group the longer
+    // iteration with everything around it (without): FP32 79 chunks 5.0 (5.45), 226 6.8 (7.36),
+    // 345 8.3 (8.8); FP64 79 5.86 (6.45), 226 8.2 (8.9).  With two chunks per group the longer
     // wait costs registers that spill (627 chunks 18.0 against 15.4): those release the packets.
     // A scene of a batch shares its SM with others that fill the wait (no difference).
     constexpr bool kSplit = MODE == kGrid && K == 1;
@@ -1304,8 +1309,8 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
             S.sum[slot][t] = acc;
         }
         group_sync(grp);
-        // relaxed: phase A writes nothing that other blocks read, and its reads of the pairs
-        // are over when the sum formed from them is out
+        // relaxed: phase A writes nothing that other blocks read, and the pairs it read are not
+        // written again before the exchange after this one's second
         publish(No(), No(), a.pkA);
         VT inv[kHere ? 1 : R];
         if constexpr(!kHere)
@@ -1326,6 +1331,7 @@ __device__ __forceinline__ void chunk_solve(const ChunkArgs<VT>& a, Smem& S, con
         }
         const VT alpha = (VT)(rho / tmp);
         parity ^= 1u;
+        if constexpr(MODE != kCluster) buf = a.pairStride - buf;
         // ---- phase B: r -= alpha q, max|r|, z = D^-1 r, partial z.r; then x += alpha s
 #pragma unroll
         for(int k = 0; k < K; ++k) {
@@ -2239,6 +2245,7 @@ static int pcg_solve_chunk(PcgWork& w, int n, ChunkShape shape, int numSM, const
     a.rhsF = rhsF; a.diag = diag; a.invd = invd; a.nbr = nbr; a.coef = coef; a.negoff = negoff;
     a.tolFactor = tolFactor; a.maxIter = maxIter; a.x = x;
     a.pair = sizeof(VT) == 8 ? (RowPair<VT>*)(void*)w.st64[0] : (RowPair<VT>*)(void*)w.st32[0];
+    a.pairStride = w.cap;
     a.pkA = w.packets;
     a.pkB = a.pkA + (size_t)w.nchCap * kPacketStride;
     a.st = dst;
@@ -2640,7 +2647,7 @@ int pcg_solve_batch_refined(BatchPcgCtx& ctx, BatchSolveItem* items, int count, 
             ChunkArgs<float>& c = hargs[k];
             c.n = n; c.nch = chunks_of(set[k]); c.rhsF = w.r32; c.diag = it.diag; c.invd = it.invd; c.nbr = it.nbr;
             c.coef = nullptr; c.negoff = -(1.0f * it.dt); c.tolFactor = it.innerTol; c.maxIter = it.maxIter; c.x = w.d32;
-            c.pair = (RowPair<float>*)(void*)w.st32[0]; c.pkA = pkA; c.pkB = pkB; c.st = it.dst;
+            c.pair = (RowPair<float>*)(void*)w.st32[0]; c.pairStride = w.cap; c.pkA = pkA; c.pkB = pkB; c.st = it.dst;
             if(!alone[set[k]]) { nch.push_back(c.nch); at.push_back((int)k); }
         }
         if(solve) {
