@@ -17,11 +17,10 @@
 // kernel sphere can reach, so every thread sums its neighbours in the canonical order
 // (rows, then cell-sorted order).  Candidates are taken two at a time: coordinates lie in
 // planes, so a pair is one 8-byte load per axis, and distances, weights and products are
-// formed in packed FP32 (each half rounded as the scalar operation); the sums stay serial.  Rows and cells that provably hold no neighbour are
+// formed in packed FP32 (each half rounded as the scalar operation); the sums stay serial and
+// take a neighbour's terms alone (add_hits).  Rows and cells that provably hold no neighbour are
 // skipped; the margins cover the float rounding of the cell index (see row_range).  The
-// accumulation is branch-free: a candidate outside the sphere adds a weight of 0, which
-// leaves every sum unchanged (none of them can be -0), except the weighted mean, which is
-// selected.  The covariance is symmetric positive semi-definite, so its SVD is its
+// covariance is symmetric positive semi-definite, so its SVD is its
 // eigen-decomposition; a cyclic Jacobi iteration gives it, and the cube root is Newton's
 // iteration in double precision, so the whole pass uses only correctly rounded
 // operations and matches the CPU restatement bit for bit.
@@ -96,6 +95,15 @@ template<bool FAST> __device__ __forceinline__ F2 kernel_w2(F2 d2, F2 rinv, cons
     const F2 root = FAST ? sqrt2(d2, k) : pack2(sqrtf(lo2(d2)), sqrtf(hi2(d2)));
     const F2 t = mul2(root, rinv, k);
     return fma2(mul2(mul2(t, t, k), t, k), k.minus1, k.one);
+}
+
+// a + v.lo + v.hi, each only where it is a neighbour's, as predicated sums: a candidate that is none
+// leaves a as it is, whatever its coordinates (not finite, the pair mate of another row).  A sum of
+// 0 instead would make a running -0 to 0, and 0 times a NaN coordinate is NaN.
+__device__ __forceinline__ float add_hits(float a, F2 v, bool h0, bool h1) {
+    asm("{ .reg .pred p, q; setp.ne.s32 p, %3, 0; setp.ne.s32 q, %4, 0; @p add.rn.f32 %0, %0, %1; @q add.rn.f32 %0, %0, %2; }"
+        : "+f"(a) : "f"(lo2(v)), "f"(hi2(v)), "r"((int)h0), "r"((int)h1));
+    return a;
 }
 
 // The sorted-index range [s, e) of cell row (j, k) that may hold neighbours of p.  A
@@ -218,10 +226,11 @@ __device__ __forceinline__ void kernel_matrix(float a[3][3], float axisRatio, fl
 // Bound by the FP32 pipe (a packed operation takes it for two cycles, so packing saves issue
 // slots, not pipe cycles: 22 and 39 a candidate in the two passes) and, below a few hundred
 // thousand points, by the serial chain of a particle's candidates.  ms against one candidate at a
-// time with sqrtf: 5,000 points 0.480 (0.946), 50,000 0.824 (1.278), 200,003 2.63 (2.74),
-// 1,000,000 12.57 (12.41).  Whole bnn_anisotropic_kernels call, with its temporaries from the
-// pool: 200,003 points 2.87 ms (4.20).  Nine blocks per SM: 200,003 points 2.63 ms against 2.73
-// at eight, 2.68 at ten.
+// time with sqrtf: 5,000 points 0.456 (0.946), 50,000 0.798 (1.28), 200,003 2.62 (2.75),
+// 1,000,000 12.55 (12.45).  Sums of selected terms instead of predicated ones: 0.498, 0.867, 2.77,
+// 13.2.  Whole bnn_anisotropic_kernels call, with its temporaries from the
+// pool: 200,003 points 2.87 ms (4.20).  Nine blocks per SM: 200,003 points 2.62 ms against 2.75
+// at ten.
 template<bool FAST>
 __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict__ px, const float* __restrict__ py,
                                                const float* __restrict__ pz, const uint32_t* __restrict__ ids,
@@ -250,8 +259,7 @@ __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict
     const F2 Px2 = pack2(Px, Px), Py2 = pack2(Py, Py), Pz2 = pack2(Pz, Pz), rinv = pack2(a.rinv, a.rinv);
     auto at2 = [](const float* __restrict__ v, uint32_t q) { return __ldg(reinterpret_cast<const F2*>(v + q)); };
 
-    // pass 1: neighbour count and weighted mean (AniKernelGenerator.cpp:65-75).  A candidate
-    // that is no neighbour adds 0 w = 0.
+    // pass 1: neighbour count and weighted mean (AniKernelGenerator.cpp:65-75)
     float sw = 1.0f, mx = Px, my = Py, mz = Pz;
     uint32_t cnt = 0;
     for(int dz = -R; dz <= R; ++dz)
@@ -267,21 +275,13 @@ __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict
                 const bool h0 = lo2(d2) < a.r2 && q - s < len && q != self;
                 const bool h1 = hi2(d2) < a.r2 && q + 1 - s < len && q + 1 != self;
                 const F2 w = kernel_w2<FAST>(d2, rinv, k2);
-                const float w0 = h0 ? lo2(w) : 0.0f, w1 = h1 ? hi2(w) : 0.0f;
-                sw = (sw + w0) + w1;
                 cnt += (h0 ? 1u : 0u) + (h1 ? 1u : 0u);
-                const F2 ww = pack2(w0, w1);
-                const F2 ax = mul2(ww, Qx, k2), ay = mul2(ww, Qy, k2), az = mul2(ww, Qz, k2);
-                mx = (mx + lo2(ax)) + hi2(ax);
-                my = (my + lo2(ay)) + hi2(ay);
-                mz = (mz + lo2(az)) + hi2(az);
+                sw = add_hits(sw, w, h0, h1);
+                mx = add_hits(mx, mul2(w, Qx, k2), h0, h1);
+                my = add_hits(my, mul2(w, Qy, k2), h0, h1);
+                mz = add_hits(mz, mul2(w, Qz, k2), h0, h1);
             }
         }
-    if(cnt == 0) {  // the mean of the particle alone, a coordinate -0 included
-        mx = Px;
-        my = Py;
-        mz = Pz;
-    }
     const float wx = mx / sw, wy = my / sw, wz = mz / sw;
     const uint32_t id = active ? ids[p] : 0u;
     if(active) {
@@ -320,13 +320,8 @@ __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict
                 const bool h0 = lo2(d2) < a.r2 && q - s < len && q != self && lo2(dm) < a.r2;
                 const bool h1 = hi2(d2) < a.r2 && q + 1 - s < len && q + 1 != self && hi2(dm) < a.r2;
                 const F2 w = kernel_w2<FAST>(dm, rinv, k2);
-                const float w0 = h0 ? lo2(w) : 0.0f, w1 = h1 ? hi2(w) : 0.0f;
-                sw2 = (sw2 + w0) + w1;
-                const F2 ww = pack2(w0, w1);
-                auto acc = [&](float c, F2 v) {
-                    const F2 t = mul2(ww, v, k2);
-                    return (c + lo2(t)) + hi2(t);
-                };
+                auto acc = [&](float c, F2 v) { return add_hits(c, mul2(w, v, k2), h0, h1); };
+                sw2 = add_hits(sw2, w, h0, h1);
                 c00 = acc(c00, q00);
                 c01 = acc(c01, mul2(x0, x1, k2));
                 c02 = acc(c02, mul2(x0, x2, k2));

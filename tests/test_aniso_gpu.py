@@ -161,3 +161,32 @@ def test_standalone_candidate_pairs_bitexact(bnn, oracle_mod, n, radius, scale):
     # at the smallest scales the determinant underflows and the matrices are NaN on both sides
     assert np.array_equal(cen.cpu().numpy(), oc, equal_nan=True)
     assert np.array_equal(mat.cpu().numpy(), om, equal_nan=True)
+
+
+def test_candidates_that_are_no_neighbours_leave_the_sums_alone(bnn, oracle_mod):
+    """A particle whose x is not a number sorts into the first column and is every near row's
+    candidate, but nobody's neighbour: the others' centres and matrices are those of the scene
+    without it.  And a sheet at x = -0 keeps its sign, as the skipped terms of the oracle do."""
+    cfg = scenes.dam_break_params(24)
+    pos, vel = scenes.dam_break(24)
+    n = len(pos)
+    out = []
+    for extra in ([], [[np.nan, 0.1, 0.1], [np.nan, 0.2, 0.15], [np.nan, 0.02, 0.02]]):
+        s = bnn.FlipSolver(cfg)
+        e = np.array(extra, np.float32).reshape(-1, 3)
+        s.set_particles(np.concatenate([pos, e]), np.concatenate([vel, 0 * e]))
+        out.append(s.anisotropic_kernels()[:2])
+    _eq(out[1][0][:n], out[0][0], "centres")
+    _eq(out[1][1][:n], out[0][1], "kernel matrices")
+
+    rng = np.random.default_rng(5)
+    p = (rng.random((700, 3)) * 0.3).astype(np.float32)
+    p[:, 0] = np.float32(-0.0)
+    d = torch.from_numpy(p).cuda()
+    cen = torch.empty(700, 3, device="cuda")
+    mat = torch.empty(700, 9, device="cuda")
+    st = capi.anisotropic_kernels_dev(d.data_ptr(), 700, capi.aniso_params(0.01, neighbor_threshold=2), cen.data_ptr(),
+                                      mat.data_ptr())
+    oc = _oracle_for(oracle_mod, p, st, 0.01, threshold=2)[0]
+    _eq(cen.cpu().numpy(), oc, "centres")
+    assert np.array_equal(np.signbit(cen.cpu().numpy()), np.signbit(oc))
