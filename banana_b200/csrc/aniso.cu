@@ -15,9 +15,9 @@
 // One thread per particle in cell-sorted order.  Both passes walk the cell rows around the
 // particle (z outer, y inner) and, in each row, the sorted particles of the cells its
 // kernel sphere can reach, so every thread sums its neighbours in the canonical order
-// (rows, then cell-sorted order).  Candidates are taken two at a time: coordinates lie in
-// planes, so a pair is one 8-byte load per axis, and distances, weights and products are
-// formed in packed FP32 (each half rounded as the scalar operation); the sums stay serial and
+// (rows, then cell-sorted order).  Candidates are taken two at a time: of points
+// 2i and 2i + 1, {x pair, y pair} is one 16-byte load and {z pair} one of 8, and distances,
+// weights and products are formed in packed FP32 (each half rounded as the scalar operation); the sums stay serial and
 // take a neighbour's terms alone (add_hits).  Rows and cells that provably hold no neighbour are
 // skipped; the margins cover the float rounding of the cell index (see row_range).  The
 // covariance is symmetric positive semi-definite, so its SVD is its
@@ -226,20 +226,27 @@ __device__ __forceinline__ void kernel_matrix(float a[3][3], float axisRatio, fl
 // Bound by the FP32 pipe (a packed operation takes it for two cycles, so packing saves issue
 // slots, not pipe cycles: 22 and 39 a candidate in the two passes) and, below a few hundred
 // thousand points, by the serial chain of a particle's candidates.  ms against one candidate at a
-// time with sqrtf: 5,000 points 0.456 (0.946), 50,000 0.798 (1.28), 200,003 2.62 (2.75),
-// 1,000,000 12.55 (12.45).  Sums of selected terms instead of predicated ones: 0.498, 0.867, 2.77,
-// 13.2.  Whole bnn_anisotropic_kernels call, with its temporaries from the
-// pool: 200,003 points 2.87 ms (4.20).  Nine blocks per SM: 200,003 points 2.62 ms against 2.75
-// at ten.
+// time with sqrtf and a 16-byte record: 5,000 points 0.467 (0.947), 50,000 0.766 (1.28), 200,003
+// 2.51 (2.75), 600,001 7.18 (7.63), 1,000,000 11.86 (12.45), 3,000,000 36.3 (38.1); the pass over a
+// 256^3 scene with its layout 155.7 (163.5).  Coordinates in three planes, three loads a pair:
+// 0.456, 0.798, 2.62, 7.58, 12.55, 38.5.  Sums of selected terms instead of predicated ones:
+// 0.498, 0.867, 2.77 and 13.2 at a million.  Nine blocks per SM: 200,003 points 2.62 ms against
+// 2.75 at ten (planes).
 template<bool FAST>
-__global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict__ px, const float* __restrict__ py,
-                                               const float* __restrict__ pz, const uint32_t* __restrict__ ids,
+__global__ void __launch_bounds__(128, 9) k_aniso(int n, const ulonglong2* __restrict__ xy, const F2* __restrict__ zz,
+                                               const uint32_t* __restrict__ ids,
                                                const uint32_t* __restrict__ cellStart, AnisoGrid g, AnisoArgs a, Packed k2,
                                                float* __restrict__ outC, float* __restrict__ outM,
                                                unsigned* __restrict__ counters) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = p < n;
-    const float Px = active ? px[p] : 0.f, Py = active ? py[p] : 0.f, Pz = active ? pz[p] : 0.f;
+    float Px = 0.f, Py = 0.f, Pz = 0.f;
+    if(active) {
+        const float* own = reinterpret_cast<const float*>(xy + (p >> 1)) + (p & 1);
+        Px = own[0];
+        Py = own[2];
+        Pz = reinterpret_cast<const float*>(zz)[p];
+    }
     int cj, ck;
     {
         int c[3] = {(int)((Px - g.bmin[0]) / g.dx), (int)((Py - g.bmin[1]) / g.dx), (int)((Pz - g.bmin[2]) / g.dx)};
@@ -257,7 +264,6 @@ __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict
     const int R = a.R;
     const uint32_t self = (uint32_t)p;
     const F2 Px2 = pack2(Px, Px), Py2 = pack2(Py, Py), Pz2 = pack2(Pz, Pz), rinv = pack2(a.rinv, a.rinv);
-    auto at2 = [](const float* __restrict__ v, uint32_t q) { return __ldg(reinterpret_cast<const F2*>(v + q)); };
 
     // pass 1: neighbour count and weighted mean (AniKernelGenerator.cpp:65-75)
     float sw = 1.0f, mx = Px, my = Py, mz = Pz;
@@ -268,8 +274,10 @@ __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict
             if(active) row_range(g, a, cellStart, Px, Py, Pz, cj + dy, ck + dz, s, e);
             const uint32_t len = e - s;
 #pragma unroll 2
-            for(uint32_t q = s & ~1u; q < e; q += 2) {
-                const F2 Qx = at2(px, q), Qy = at2(py, q), Qz = at2(pz, q);
+            for(uint32_t i = s >> 1; 2 * i < e; ++i) {
+                const uint32_t q = 2 * i;
+                const ulonglong2 Qxy = __ldg(xy + i);
+                const F2 Qx = Qxy.x, Qy = Qxy.y, Qz = __ldg(zz + i);
                 const F2 ex = fma2(Qx, k2.minus1, Px2), ey = fma2(Qy, k2.minus1, Py2), ez = fma2(Qz, k2.minus1, Pz2);
                 const F2 d2 = len2(ex, ey, ez, k2);
                 const bool h0 = lo2(d2) < a.r2 && q - s < len && q != self;
@@ -310,8 +318,10 @@ __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict
             if(need) row_range(g, a, cellStart, Px, Py, Pz, cj + dy, ck + dz, s, e);
             const uint32_t len = e - s;
 #pragma unroll 2
-            for(uint32_t q = s & ~1u; q < e; q += 2) {
-                const F2 Qx = at2(px, q), Qy = at2(py, q), Qz = at2(pz, q);
+            for(uint32_t i = s >> 1; 2 * i < e; ++i) {
+                const uint32_t q = 2 * i;
+                const ulonglong2 Qxy = __ldg(xy + i);
+                const F2 Qx = Qxy.x, Qy = Qxy.y, Qz = __ldg(zz + i);
                 const F2 ex = fma2(Qx, k2.minus1, Px2), ey = fma2(Qy, k2.minus1, Py2), ez = fma2(Qz, k2.minus1, Pz2);
                 const F2 d2 = len2(ex, ey, ez, k2);
                 const F2 x0 = add2(Qx, Wx2), x1 = add2(Qy, Wy2), x2 = add2(Qz, Wz2);
@@ -342,14 +352,23 @@ __global__ void __launch_bounds__(128, 9) k_aniso(int n, const float* __restrict
     for(int e = 0; e < 9; ++e) out[e] = M[e];
 }
 
-// Positions in sorted order as planes of stride `stride`
-__global__ void k_pack_sorted(const float* __restrict__ pos, const uint32_t* __restrict__ order, uint32_t n,
-                              float* __restrict__ out, size_t stride) {
+// Sorted points as pairs (PairPoints): point i is order[i] of the AoS positions, or i of the
+// coordinate planes of stride `stride`; the last point of an odd number gets a mate at 0
+template<bool PLANES>
+__global__ void k_pack_pairs(const float* __restrict__ pos, size_t stride, const uint32_t* __restrict__ order, uint32_t n,
+                             float4* __restrict__ xy, float2* __restrict__ z) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= n) return;
-    const uint32_t p = order[i];
+    if(i >= (((size_t)n + 1) & ~(size_t)1)) return;
+    float v[3] = {0.f, 0.f, 0.f};
+    if(i < n) {
+        const size_t p = PLANES ? i : order[i];
 #pragma unroll
-    for(int d = 0; d < 3; ++d) out[d * stride + i] = pos[3 * (size_t)p + d];
+        for(int d = 0; d < 3; ++d) v[d] = PLANES ? pos[d * stride + p] : pos[3 * p + d];
+    }
+    float* at = reinterpret_cast<float*>(xy + (i >> 1)) + (i & 1);
+    at[0] = v[0];
+    at[2] = v[1];
+    reinterpret_cast<float*>(z)[i] = v[2];
 }
 
 // order-preserving float <-> uint keys for atomic min / max
@@ -426,27 +445,39 @@ int aniso_check_params(const bnn_aniso_params& p) {
     return BNN_OK;
 }
 
-// The pass over cell-sorted points: coordinate planes pos, pos + stride, pos + 2 stride (8-byte
-// aligned, stride > n when n is odd: element n of each is set to 0, the pair mate of the last
-// point), ids = input index of each sorted point, cellStart = C + 1 offsets of grid g.
-// counters[0] receives the spray points, counters[1] the points outside g (both must be zeroed
-// by the caller).
-cudaError_t launch_aniso(int n, float* pos, size_t stride, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
+// Lays n sorted points out for launch_aniso
+PairPoints aniso_pairs(void* mem, int n) {
+    PairPoints q;
+    q.xy = (float4*)mem;
+    q.z = (float2*)(q.xy + ((size_t)n + 1) / 2);
+    return q;
+}
+static void launch_pack(const PairPoints& q, const float* pos, size_t stride, const uint32_t* order, int n, cudaStream_t s) {
+    const unsigned blocks = (unsigned)(((size_t)n + 256) / 256);
+    if(order) k_pack_pairs<false><<<blocks, 256, 0, s>>>(pos, stride, order, (uint32_t)n, q.xy, q.z);
+    else k_pack_pairs<true><<<blocks, 256, 0, s>>>(pos, stride, order, (uint32_t)n, q.xy, q.z);
+    bnn_note_launch();
+}
+void launch_aniso_pack(const PairPoints& q, const float* planes, size_t stride, int n, cudaStream_t s) {
+    if(n > 0) launch_pack(q, planes, stride, nullptr, n, s);
+}
+
+// The pass over cell-sorted points q (laid out by launch_aniso_pack), ids = input index of each
+// sorted point, cellStart = C + 1 offsets of grid g.  counters[0] receives the spray points,
+// counters[1] the points outside g (both must be zeroed by the caller).
+cudaError_t launch_aniso(int n, const PairPoints& q, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
                          const bnn_aniso_params& prm, float* outC, float* outM, unsigned* counters, cudaStream_t s) {
     if(n <= 0) return cudaSuccess;
-    if(n & 1)
-        for(int d = 0; d < 3; ++d) {
-            const cudaError_t e = cudaMemsetAsync(pos + d * stride + n, 0, sizeof(float), s);
-            if(e != cudaSuccess) return e;
-        }
     const AnisoArgs a = make_args(prm, g.dx);
     auto both = [](unsigned bits) { return (F2)bits << 32 | bits; };
     const Packed k{both(0x80000000u), both(0xbf800000u), both(0x3f800000u)};
     const float r = prm.kernel_ratio * prm.particle_radius;
     const bool fast = r >= 0x1p-24f && r <= 0x1p24f;
     const unsigned blocks = (unsigned)((n + 127) / 128);
-    if(fast) k_aniso<true><<<blocks, 128, 0, s>>>(n, pos, pos + stride, pos + 2 * stride, ids, cellStart, g, a, k, outC, outM, counters);
-    else k_aniso<false><<<blocks, 128, 0, s>>>(n, pos, pos + stride, pos + 2 * stride, ids, cellStart, g, a, k, outC, outM, counters);
+    const ulonglong2* xy = reinterpret_cast<const ulonglong2*>(q.xy);
+    const F2* zz = reinterpret_cast<const F2*>(q.z);
+    if(fast) k_aniso<true><<<blocks, 128, 0, s>>>(n, xy, zz, ids, cellStart, g, a, k, outC, outM, counters);
+    else k_aniso<false><<<blocks, 128, 0, s>>>(n, xy, zz, ids, cellStart, g, a, k, outC, outM, counters);
     bnn_note_launch();
     return cudaGetLastError();
 }
@@ -515,25 +546,25 @@ extern "C" int bnn_anisotropic_kernels(const float* pos_dev, uint32_t n, const b
     }
     g.dx = cell;
     const size_t C = (size_t)g.G[0] * g.G[1] * g.G[2];
-    DevMem cid, order, start, planes, cnt;
+    DevMem cid, order, start, pairs, cnt;
     BNN_CUDA_CHECK(cid.alloc((size_t)n * 4, s));
     BNN_CUDA_CHECK(order.alloc((size_t)n * 4, s));
     BNN_CUDA_CHECK(start.alloc((C + 1) * 4, s));
-    const size_t stride = ((size_t)n + 64) / 64 * 64;  // room for the last point's pair mate
-    BNN_CUDA_CHECK(planes.alloc(3 * stride * sizeof(float), s));
+    BNN_CUDA_CHECK(pairs.alloc(pair_bytes(n), s));
     BNN_CUDA_CHECK(cnt.alloc(2 * sizeof(unsigned), s));
     uint32_t oor = 0;
     rc = bnn_cell_sort(pos_dev, n, g.bmin, g.dx, g.G, cid.as<uint32_t>(), order.as<uint32_t>(), start.as<uint32_t>(),
                        &oor, stream);
     if(rc != BNN_OK) return rc;
-    { k_pack_sorted<<<(n + 255) / 256, 256, 0, s>>>(pos_dev, order.as<uint32_t>(), n, planes.as<float>(), stride); bnn_note_launch(); }
+    const PairPoints q = aniso_pairs(pairs.p, (int)n);
+    launch_pack(q, pos_dev, 0, order.as<uint32_t>(), (int)n, s);
     BNN_CUDA_CHECK(cudaMemsetAsync(cnt.p, 0, 2 * sizeof(unsigned), s));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    BNN_CUDA_CHECK(launch_aniso((int)n, planes.as<float>(), stride, order.as<uint32_t>(), start.as<uint32_t>(), g, *params,
-                                centers_dev, matrices_dev, cnt.as<unsigned>(), s));
+    BNN_CUDA_CHECK(launch_aniso((int)n, q, order.as<uint32_t>(), start.as<uint32_t>(), g, *params, centers_dev, matrices_dev,
+                                cnt.as<unsigned>(), s));
     cudaEventRecord(e1, s);
     unsigned hc[2];
     BNN_CUDA_CHECK(cudaMemcpyAsync(hc, cnt.p, sizeof(hc), cudaMemcpyDeviceToHost, s));

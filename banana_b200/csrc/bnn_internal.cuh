@@ -451,7 +451,15 @@ struct AnisoGrid {
 };
 bnn_aniso_params aniso_defaults(float particleRadius);
 int aniso_check_params(const bnn_aniso_params& p);
-cudaError_t launch_aniso(int n, float* pos, size_t stride, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
+// Sorted points 2i and 2i + 1: {x, x, y, y} and {z, z}
+struct PairPoints {
+    float4* xy;
+    float2* z;
+};
+inline size_t pair_bytes(size_t n) { return (n + 1) / 2 * (sizeof(float4) + sizeof(float2)); }
+PairPoints aniso_pairs(void* mem, int n);  // in pair_bytes(n) of memory
+void launch_aniso_pack(const PairPoints& q, const float* planes, size_t stride, int n, cudaStream_t s);
+cudaError_t launch_aniso(int n, const PairPoints& q, const uint32_t* ids, const uint32_t* cellStart, const AnisoGrid& g,
                          const bnn_aniso_params& prm, float* outC, float* outM, unsigned* counters, cudaStream_t s);
 
 void pcg_release(PcgWork& w);

@@ -866,7 +866,10 @@ extern "C" int bnn_flip_anisotropic_kernels(bnn_flip* h, const bnn_aniso_params*
     for(int d = 0; d < 3; ++d) { ag.G[d] = g.G[d]; ag.bmin[d] = g.bmin[d]; }
     ag.dx = g.dx;
     cudaEventRecord(h->ev[0], s);
-    BNN_CUDA_CHECK(launch_aniso(n, h->p6[h->cur], cap, h->ids[h->cur], h->cellStart, ag, prm, dC, dM, cnt, s));
+    // the records of the P2G pass are scratch here: the next sub-step's sort writes them anew
+    const PairPoints q = aniso_pairs(h->rec, n);
+    launch_aniso_pack(q, h->p6[h->cur], cap, n, s);
+    BNN_CUDA_CHECK(launch_aniso(n, q, h->ids[h->cur], h->cellStart, ag, prm, dC, dM, cnt, s));
     cudaEventRecord(h->ev[1], s);
     BNN_CUDA_CHECK(cudaMemcpyAsync(centers, dC, 3 * (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, s));
     BNN_CUDA_CHECK(cudaMemcpyAsync(matrices, dM, 9 * (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, s));
