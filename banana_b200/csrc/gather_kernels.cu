@@ -38,9 +38,9 @@
 // and, where cells are crowded, by the serial sum over a cell's particles; one after another in
 // a block they took, with a small scene's few tiles leaving most of the GPU idle, ms per
 // sub-step: 64^3 FLIP 0.128 (now 0.055), 121 x 77 x 95 APIC 0.415 (0.148), 96^3 AFLIP 0.509
-// (0.19), 160 x 192 x 128 FLIP 0.384 (0.275), 256^3 FLIP 0.974 (0.773); a batch of 24 scenes, 30
-// steps, 206 -> 169.
-//
+// (0.19), 160 x 192 x 128 FLIP 0.384 (0.275), 256^3 FLIP 0.974 (0.751); a batch of 24 scenes, 30
+// steps, 206 -> 169.  A batch whose tiles fill the GPU by themselves keeps a tile's passes in one
+// block (batch_tiles_together).
 //
 // Input: one 16-byte record per particle and component, written by the sort's gather
 // (flip_kernels.cu, k_gather_particles): plane D < 3 holds {e_x, e_y, e_z, v_D}, e_a the
@@ -361,12 +361,14 @@ __device__ __forceinline__ void write_phi(const TileArgs& a, int fx, int fy, int
 // out of registers.
 constexpr int kPasses = 4;
 template<bool P2G> struct OwnTile {
+    static constexpr bool kAll = false;
     __device__ __forceinline__ unsigned pass() const { return P2G ? blockIdx.x % kPasses : 3u; }
     __device__ __forceinline__ unsigned x() const { return P2G ? blockIdx.x / kPasses : blockIdx.x; }
     __device__ __forceinline__ unsigned z() const { return blockIdx.y; }
     __device__ __forceinline__ unsigned y() const { return blockIdx.z; }
 };
-struct GivenTile {
+template<bool ALL> struct GivenTile {
+    static constexpr bool kAll = ALL;
     unsigned bp, bx, bz, by;
     __device__ __forceinline__ unsigned pass() const { return bp; }
     __device__ __forceinline__ unsigned x() const { return bx; }
@@ -374,16 +376,56 @@ struct GivenTile {
     __device__ __forceinline__ unsigned y() const { return by; }
 };
 
-// One block of the pass PASS: tile (x, z) of face columns, y-chunk y.  EXACT: some particle
-// left the grid (the same for the whole launch; see sdf_partials).  AFF: APIC / AFLIP
-// momentum (cell_partials).
-template<int PASS, class SH, bool EXACT, bool AFF, class Tile>
-__device__ __forceinline__ void pass_body(const TileArgs& a, const Tile tile) {
-    constexpr int kTZ = SH::kTZ, kYC = SH::kYC;
-    constexpr bool SDF = PASS == 3;
+// What the pass PASS keeps of a face column: layers cy - 1 + j around the walk's cell layer cy (v
+// uses j = 1, 2), momentum and weight, or the minimum
+template<int PASS> struct PassSums {
+    static constexpr bool kSdf = PASS == 3;
     // the cell layer that completes face / cell layer y: y + 1, but y itself for v, whose faces
     // have the walk's axis
-    constexpr int kLag = PASS == 1 ? 0 : 1;
+    static constexpr int kLag = PASS == 1 ? 0 : 1;
+    float s[3], w[3];
+    __device__ __forceinline__ static float none() { return kSdf ? __int_as_float(0x7f800000) : 0.0f; }
+    __device__ __forceinline__ PassSums() {
+#pragma unroll
+        for(int j = 0; j < 3; ++j) { s[j] = none(); w[j] = 0.f; }
+    }
+    __device__ __forceinline__ static void write(const TileArgs& a, int fx, int fy, int fz, float S, float W) {
+        if constexpr(kSdf) write_phi(a, fx, fy, fz, S);
+        else write_face<PASS>(a, fx, fy, fz, S, W);
+    }
+    // cell layer cy: particles [pb, pe) of this thread's cell; [nb, ne) are the next layer's, or none
+    template<class SH, bool EXACT, bool AFF>
+    __device__ __forceinline__ void add(const TileArgs& a, int x0, int z0, int cy, int t, uint32_t pb, uint32_t pe, uint32_t nb,
+                                        uint32_t ne, float* __restrict__ sm, bool owner, int tx, int tz) {
+        if constexpr(kSdf) sdf_partials<SH, EXACT>(a, x0, z0, cy, t, pb, pe, sm);
+        else cell_partials<PASS, SH, AFF>(a, t, pb, pe, sm, x0, z0, cy);
+        // the first line of the next layer's records: the one load the serial sum cannot
+        // issue ahead (256^3 0.81 -> 0.77 ms)
+        if(nb < ne) asm volatile("prefetch.global.L1 [%0];" : : "l"(a.rec + (size_t)PASS * a.stride + nb));
+        __syncthreads();
+        if(owner) {
+            if constexpr(kSdf) pull_sdf<SH>(sm, tx, tz, s);
+            else pull_partials<PASS, SH>(sm, tx, tz, s, w);
+        }
+        __syncthreads();
+    }
+    // the layer that cy completes goes out, the others move down
+    __device__ __forceinline__ void shift(const TileArgs& a, int fx, int cy, int fz, int yA, int yB) {
+        const int fy = cy - kLag;
+        if(fy >= yA && fy < yB) write(a, fx, fy, fz, s[1 - kLag], w[1 - kLag]);
+        s[0] = s[1]; s[1] = s[2]; s[2] = none();
+        w[0] = w[1]; w[1] = w[2]; w[2] = 0.f;
+    }
+};
+
+// One block of the passes PS: tile (x, z) of face columns, y-chunk y.  EXACT: some particle
+// left the grid (the same for the whole launch; see sdf_partials).  AFF: APIC / AFLIP
+// momentum (cell_partials).
+template<class SH, bool EXACT, bool AFF, int... PS, class Tile>
+__device__ __forceinline__ void walk_tile(const TileArgs& a, const Tile tile) {
+    constexpr int kTZ = SH::kTZ, kYC = SH::kYC;
+    constexpr int kMostLag = ((PS != 1) || ...) ? 1 : 0;
+    constexpr bool kOne = sizeof...(PS) == 1;
     extern __shared__ float sm[];
     const GridDesc& g = a.g;
     const int t = threadIdx.y * kHX + threadIdx.x;        // this thread's halo cell
@@ -392,63 +434,47 @@ __device__ __forceinline__ void pass_body(const TileArgs& a, const Tile tile) {
     const int x0 = (int)tile.x() * kTX, z0 = (int)tile.z() * kTZ;
     const int yA = (int)tile.y() * kYC, yB = min(yA + kYC, g.G[1] + 1);  // face layers [yA, yB)
     const int fx = owner ? x0 + tx : INT_MAX, fz = owner ? z0 + tz : INT_MAX;
-    const float inf = __int_as_float(0x7f800000);
     {
         const int lo[3] = {x0 - 1, yA - 1, z0 - 1}, hi[3] = {x0 + kTX, yB, z0 + kTZ};
         if(!meets_particles(a.st, lo, hi)) {
             // no particle reaches the tile: empty faces and cells
-            for(int fy = yA; fy < yB; ++fy) {
-                if constexpr(SDF) write_phi(a, fx, fy, fz, inf);
-                else write_face<PASS>(a, fx, fy, fz, 0.0f, 0.0f);
-            }
+            for(int fy = yA; fy < yB; ++fy) (PassSums<PS>::write(a, fx, fy, fz, PassSums<PS>::none(), 0.0f), ...);
             return;
         }
     }
-    // accumulators of layers cy - 1 + j (v uses j = 1, 2): momentum and weight, or the minimum
-    const float none = SDF ? inf : 0.0f;
-    float aS[3] = {none, none, none}, aW[3] = {0.f, 0.f, 0.f};
-    const int cEnd = min(yB - 1 + kLag, g.G[1] - 1);
+    struct : PassSums<PS>... {} sums;
+    const int last = yB - 1 + kMostLag, cEnd = min(last, g.G[1] - 1);
     uint32_t pb = 0u, pe = 0u;
-    if(yA > 0) cell_range(a, x0, z0, yA - 1, t, pb, pe);
-    for(int cy = yA - 1; cy <= yB - 1 + kLag; ++cy) {
-        // the next layer's particle range, on its way while this layer is summed
+    if(kOne && yA > 0) cell_range(a, x0, z0, yA - 1, t, pb, pe);
+    for(int cy = yA - 1; cy <= last; ++cy) {
+        // the next layer's particle range, on its way while this layer is summed (not with four
+        // passes' sums in registers: 256 scenes 4.59 ms against 4.48)
         uint32_t nb = 0u, ne = 0u;
-        if(cy + 1 <= cEnd) cell_range(a, x0, z0, cy + 1, t, nb, ne);
-        if(cy >= 0 && cy < g.G[1]) {
-            if constexpr(SDF) sdf_partials<SH, EXACT>(a, x0, z0, cy, t, pb, pe, sm);
-            else cell_partials<PASS, SH, AFF>(a, t, pb, pe, sm, x0, z0, cy);
-            // the first line of the next layer's records: the one load the serial sum cannot
-            // issue ahead (256^3 0.81 -> 0.77 ms)
-            if(nb < ne) asm volatile("prefetch.global.L1 [%0];" : : "l"(a.rec + (size_t)PASS * a.stride + nb));
-            __syncthreads();
-            if(owner) {
-                if constexpr(SDF) pull_sdf<SH>(sm, tx, tz, aS);
-                else pull_partials<PASS, SH>(sm, tx, tz, aS, aW);
-            }
-            __syncthreads();
-        }
-        pb = nb;
-        pe = ne;
-        const int fy = cy - kLag;
-        if(fy >= yA) {
-            if constexpr(SDF) write_phi(a, fx, fy, fz, aS[0]);
-            else write_face<PASS>(a, fx, fy, fz, aS[1 - kLag], aW[1 - kLag]);
-        }
-        aS[0] = aS[1]; aS[1] = aS[2]; aS[2] = none;
-        aW[0] = aW[1]; aW[1] = aW[2]; aW[2] = 0.f;
+        if(kOne && cy + 1 <= cEnd) cell_range(a, x0, z0, cy + 1, t, nb, ne);
+        if(!kOne && cy >= 0 && cy <= cEnd) cell_range(a, x0, z0, cy, t, pb, pe);
+        if(cy >= 0 && cy < g.G[1])
+            ((PassSums<PS>::kLag == kMostLag || cy < last
+                  ? sums.PassSums<PS>::template add<SH, EXACT, AFF>(a, x0, z0, cy, t, pb, pe, nb, ne, sm, owner, tx, tz)
+                  : (void)0), ...);
+        if(kOne) { pb = nb; pe = ne; }
+        (sums.PassSums<PS>::shift(a, fx, cy, fz, yA, yB), ...);
     }
 }
+// The block's pass, or all four
 template<bool P2G, class SH, bool EXACT, bool AFF = false, class Tile>
 __device__ __forceinline__ void tile_body(const TileArgs& a, const Tile tile) {
-    if constexpr(P2G) {
-        switch(tile.pass()) {
-        case 0: pass_body<0, SH, EXACT, AFF>(a, tile); return;
-        case 1: pass_body<1, SH, EXACT, AFF>(a, tile); return;
-        case 2: pass_body<2, SH, EXACT, AFF>(a, tile); return;
-        default: break;
+    if constexpr(Tile::kAll) walk_tile<SH, EXACT, AFF, 0, 1, 2, 3>(a, tile);
+    else {
+        if constexpr(P2G) {
+            switch(tile.pass()) {
+            case 0: walk_tile<SH, EXACT, AFF, 0>(a, tile); return;
+            case 1: walk_tile<SH, EXACT, AFF, 1>(a, tile); return;
+            case 2: walk_tile<SH, EXACT, AFF, 2>(a, tile); return;
+            default: break;
+            }
         }
+        walk_tile<SH, EXACT, AFF, 3>(a, tile);
     }
-    pass_body<3, SH, EXACT, AFF>(a, tile);
 }
 // The rare launch in which some particle left the grid, kept out of line so that its
 // per-slot tests do not weigh on the registers of the common path
@@ -462,18 +488,18 @@ __global__ void __launch_bounds__(SH::kThreads, SH::min_blocks(AFF ? 768 : 1024)
     else tile_body<P2G, SH, false, AFF>(a, OwnTile<P2G>{});
 }
 
-// Batched: the tiles of all scenes of a batch in one launch (P: per-scene tile prefix);
-// a block's flat index within its scene maps to (pass, x, z, y) as in tile_grid
-template<class SH>
+// Batched: the tiles of all scenes of a batch in one launch (P: per-scene tile prefix), a block
+// per tile and pass, or per tile (ALL); a tile's flat index within its scene maps to (x, z, y)
+template<class SH, bool ALL>
 __global__ void __launch_bounds__(SH::kThreads, SH::min_blocks(768)) kb_p2g_sdf_tile(const TileArgs* __restrict__ A,
                                                                             const unsigned* __restrict__ P, int ns) {
-    int q;
-    const Blk b = seg_blk(P, ns, q);
+    const unsigned flat = ALL ? blockIdx.x : blockIdx.x / kPasses;
+    const int q = seg_of(P, ns, flat);
+    const unsigned f = flat - __ldg(P + q);
     const TileArgs& a = A[q];
     const unsigned gx = (unsigned)((a.g.G[0] + 1 + kTX - 1) / kTX);
     const unsigned gz = (unsigned)((a.g.G[2] + 1 + SH::kTZ - 1) / SH::kTZ);
-    const unsigned f = b.x / kPasses;
-    const GivenTile tile{b.x % kPasses, f % gx, (f / gx) % gz, f / (gx * gz)};
+    const GivenTile<ALL> tile{blockIdx.x % kPasses, f % gx, (f / gx) % gz, f / (gx * gz)};
     if((a.st->flags & BNN_FLAG_OUT_OF_GRID) != 0u) tile_body_exact<true, SH, false>(a, tile);  // the scene's flag
     else tile_body<true, SH, false, false>(a, tile);
 }
@@ -500,11 +526,22 @@ template<bool P2G, class SH> static void launch_tile_sh(const TileArgs& a, cudaS
     k_p2g_sdf_tile<P2G, SH><<<tile_grid_of<SH, P2G>(a.g), dim3(kHX, SH::kHZ), SH::kSmemBytes, s>>>(a);
     bnn_note_launch();
 }
+template<class SH> static void opt_in_batch() {
+    static std::atomic<uint64_t> one{0}, all{0};
+    opt_in_smem(kb_p2g_sdf_tile<SH, false>, SH::kSmemBytes, one);
+    opt_in_smem(kb_p2g_sdf_tile<SH, true>, SH::kSmemBytes, all);
+}
+// Whether a batch of so many cells keeps a tile's four passes in one block.  Apart they hide one
+// another's loads, at four times the blocks to place and cell ranges to read; past the line the
+// tiles alone fill the GPU.  Scenes of the batch workload, ms per pass apart (together): 24 0.516
+// (0.577), 64 1.41 (1.47), 96 (52 M cells) 2.005 (2.006), 128 2.58 (2.51), 256 4.84 (4.48).
+static bool batch_tiles_together(uint64_t cells) { return cells > 52500000ull; }
 template<class SH>
-static void launch_batch_sh(const TileArgs* A, const unsigned* P, int ns, unsigned tiles, cudaStream_t s) {
-    static std::atomic<uint64_t> configured{0};
-    opt_in_smem(kb_p2g_sdf_tile<SH>, SH::kSmemBytes, configured);
-    kb_p2g_sdf_tile<SH><<<tiles, dim3(kHX, SH::kHZ), SH::kSmemBytes, s>>>(A, P, ns);
+static void launch_batch_sh(const TileArgs* A, const unsigned* P, int ns, unsigned tiles, bool together, cudaStream_t s) {
+    opt_in_batch<SH>();
+    const dim3 threads(kHX, SH::kHZ);
+    if(together) kb_p2g_sdf_tile<SH, true><<<tiles, threads, SH::kSmemBytes, s>>>(A, P, ns);
+    else kb_p2g_sdf_tile<SH, false><<<tiles * kPasses, threads, SH::kSmemBytes, s>>>(A, P, ns);
     bnn_note_launch();
 }
 
@@ -538,15 +575,17 @@ static void launch_p2g_shape(int shape, const TileArgs& a, cudaStream_t s) {
     default: launch_tile_sh<true, S0>(a, s); break;
     }
 }
-static void launch_batch_shape(int shape, const TileArgs* A, const unsigned* P, int ns, unsigned tiles, cudaStream_t s) {
+static void launch_batch_shape(int shape, const TileArgs* A, const unsigned* P, int ns, unsigned tiles, uint64_t cells,
+                               cudaStream_t s) {
     if(tiles == 0) return;
+    const bool together = batch_tiles_together(cells);
     switch(shape) {
-    case 1: launch_batch_sh<S1>(A, P, ns, tiles, s); break;
-    case 2: launch_batch_sh<S2>(A, P, ns, tiles, s); break;
-    case 3: launch_batch_sh<S3>(A, P, ns, tiles, s); break;
-    case 4: launch_batch_sh<S4>(A, P, ns, tiles, s); break;
-    case 5: launch_batch_sh<S5>(A, P, ns, tiles, s); break;
-    default: launch_batch_sh<S0>(A, P, ns, tiles, s); break;
+    case 1: launch_batch_sh<S1>(A, P, ns, tiles, together, s); break;
+    case 2: launch_batch_sh<S2>(A, P, ns, tiles, together, s); break;
+    case 3: launch_batch_sh<S3>(A, P, ns, tiles, together, s); break;
+    case 4: launch_batch_sh<S4>(A, P, ns, tiles, together, s); break;
+    case 5: launch_batch_sh<S5>(A, P, ns, tiles, together, s); break;
+    default: launch_batch_sh<S0>(A, P, ns, tiles, together, s); break;
     }
 }
 
@@ -685,10 +724,10 @@ void launch_p2g_sdf_affine(const GridDesc& g, const DevState* st, const uint32_t
     bnn_note_launch();
 }
 
-// Tiles of one scene's P2G + SDF pass in a shape (the batched launch's share of the scene)
+// Tiles of one scene's P2G + SDF pass in a shape (for the batched launch)
 unsigned p2g_sdf_tiles(const GridDesc& g, int shape) {
     const dim3 d = tile_grid(g, shape);
-    return d.x * d.y * d.z;
+    return d.x / kPasses * d.y * d.z;
 }
 // Size of the per-scene argument record the batched launch reads, and its host-side fill
 size_t p2g_tile_args_bytes() { return sizeof(TileArgs); }
@@ -705,13 +744,12 @@ static uint64_t batch_key(int ns, uint64_t cells) {
     return ((uint64_t)(dev & 0xff) << 56) | (1ull << 48) | (log2_bucket((uint64_t)ns) << 24) | log2_bucket(cells);
 }
 int p2g_batch_shape(int ns, uint64_t cells) {
-    static std::atomic<uint64_t> c0{0}, c1{0}, c2{0}, c3{0}, c4{0}, c5{0};
-    opt_in_smem(kb_p2g_sdf_tile<S0>, S0::kSmemBytes, c0);
-    opt_in_smem(kb_p2g_sdf_tile<S1>, S1::kSmemBytes, c1);
-    opt_in_smem(kb_p2g_sdf_tile<S2>, S2::kSmemBytes, c2);
-    opt_in_smem(kb_p2g_sdf_tile<S3>, S3::kSmemBytes, c3);
-    opt_in_smem(kb_p2g_sdf_tile<S4>, S4::kSmemBytes, c4);
-    opt_in_smem(kb_p2g_sdf_tile<S5>, S5::kSmemBytes, c5);
+    opt_in_batch<S0>();
+    opt_in_batch<S1>();
+    opt_in_batch<S2>();
+    opt_in_batch<S3>();
+    opt_in_batch<S4>();
+    opt_in_batch<S5>();
     return lookup(batch_key(ns, cells));
 }
 void launch_p2g_sdf_batch(const void* args, const unsigned* const* P, const unsigned* tiles, int ns, uint64_t cells,
@@ -719,8 +757,8 @@ void launch_p2g_sdf_batch(const void* args, const unsigned* const* P, const unsi
     const uint64_t key = batch_key(ns, cells);
     const TileArgs* A = (const TileArgs*)args;
     int shape = lookup(key);
-    if(shape < 0) shape = tune(key, s, [&](int v) { launch_batch_shape(v, A, P[v], ns, tiles[v], s); });
-    else launch_batch_shape(shape, A, P[shape], ns, tiles[shape], s);
+    if(shape < 0) shape = tune(key, s, [&](int v) { launch_batch_shape(v, A, P[v], ns, tiles[v], cells, s); });
+    else launch_batch_shape(shape, A, P[shape], ns, tiles[shape], cells, s);
 }
 
 // The fluid SDF alone (APIC / AFLIP / PIC), in the default shape

@@ -64,6 +64,25 @@ def test_every_shape_gives_the_same_batch(bnn, shapes):
             assert np.array_equal(pa, pb) and np.array_equal(va, vb), (shapes[k], q)
 
 
+def test_tiles_with_all_passes_in_one_block(bnn, shapes):
+    """A batch of more than 52.5 million cells keeps a tile's four passes in one block: every shape
+    gives what the scenes give alone"""
+    specs = [{"res": (192, 192, 192), "block_frac": (0.2 + 0.05 * q, 0.3, 0.5 - 0.05 * q), "seed": 60 + q} for q in range(7)]
+    made = [scenes.batch_scene(sp, ppc=1) for sp in specs]
+    steps = len(shapes)
+    b = bnn.FlipBatch(worker_threads=1)
+    ids = [b.add_scene(*m) for m in made]
+    for k in range(steps):
+        bnn.capi.set_tile_shape(k)
+        assert b.step()["staged_scenes"] == len(specs)
+    out = [b.get_scene(i) for i in ids]
+    b.close()
+    bnn.capi.set_tile_shape(0)
+    for (cfg, pos, vel), (pb, vb), sp in zip(made, out, specs):
+        pa, va, _, _ = _run_lone(bnn, cfg, pos, vel, steps)
+        assert np.array_equal(pa, pb) and np.array_equal(va, vb), sp
+
+
 def test_tuner_records_the_fastest_shape(bnn, shapes):
     bnn.capi.set_tile_shape(-1)
     n = 36  # a resolution bucket no other test uses
