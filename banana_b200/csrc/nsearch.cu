@@ -357,8 +357,46 @@ constexpr unsigned long long kMinusZero2 = 0x8000000080000000ull;
 // Bound by instruction issue: about 9 per point and 32 candidates, 20 when writing, against 15
 // per point and candidate (and its store through a shared buffer) with a thread per point that
 // walks the candidates alone.  Measured, whole bnn_neighbors call: 4M points and 933 M entries
-// 8.53 ms (11.5 with a thread per point), 20,011 points 0.293 ms (0.617).
+// 8.45 ms (11.45 with a thread per point), 20,011 points 0.305 ms (0.602).
+//
+// That takes turns over the cells of a warp's points.  In sparse sets a cell holds a few points and
+// a turn is nearly all waiting, so a warp of 32 points whose points lie in many cells has a thread
+// walk each point's rows alone (ns_alone).  Lines at more than 4 cells when counting and 8 when
+// writing, where one thread's short runs of stores cost more.  Whole call, ms, thread per point for
+// all (this warp form for all) -> by the lines: 1M points of 0.5 a cell 0.445 (0.578) -> 0.320, of 5
+// 0.650 (0.655) -> 0.578, of 20 1.247 (1.069) -> 1.080; 4M points of 0.5 a cell 1.04 (1.87) -> 0.89,
+// of 3 1.51 (1.97) -> 1.40, of 6 2.04 (2.22) -> 2.04, of 20 4.30 (3.87) -> 3.91.
 constexpr int kNsWarps = 4;  // warps per block: they end at different times
+template<bool WRITE> constexpr int kNsCells = WRITE ? 8 : 4;
+// One point's hits, counted or written to `to`
+template<bool WRITE>
+__device__ __forceinline__ uint32_t ns_alone(const float4* __restrict__ sp, const float4& a, uint32_t at, uint32_t cell,
+                                             const uint32_t* __restrict__ cellStart, int d0, int d1, float r2,
+                                             uint32_t* __restrict__ to) {
+    uint32_t cnt = 0;
+#pragma unroll 1
+    for(int dz = -1; dz <= 1; ++dz) {
+        uint32_t b[3], e[3];
+#pragma unroll
+        for(int dy = 0; dy < 3; ++dy) {
+            const long long row = (long long)cell + dz * ((long long)d0 * d1) + (dy - 1) * (long long)d0;
+            b[dy] = cellStart[row - 1];
+            e[dy] = cellStart[row + 2];
+        }
+#pragma unroll
+        for(int dy = 0; dy < 3; ++dy)
+            for(uint32_t j = b[dy]; j < e[dy]; ++j) {
+                const float4 q = sp[j];
+                const float t0 = a.x - q.x, t1 = a.y - q.y, t2 = a.z - q.z;
+                const float l2 = t0 * t0 + t1 * t1 + t2 * t2;
+                if(l2 < r2 && j != at) {
+                    if(WRITE) to[cnt] = __float_as_uint(q.w);
+                    ++cnt;
+                }
+            }
+    }
+    return cnt;
+}
 template<int P, bool WRITE>
 __global__ void __launch_bounds__(kNsWarps * 32) k_ns_pairs(const float4* __restrict__ sp, const uint32_t* __restrict__ scid,
                                                             uint32_t n, const uint32_t* __restrict__ cellStart, int d0,
@@ -376,6 +414,17 @@ __global__ void __launch_bounds__(kNsWarps * 32) k_ns_pairs(const float4* __rest
     const float4 a = live ? sp[first + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
     const uint32_t self = __float_as_uint(a.w);
     const uint32_t cell = live ? scid[first + lane] : full;
+    if constexpr(P == 32) {
+        const uint32_t before = __shfl_up_sync(full, cell, 1);
+        if(__popc(__ballot_sync(full, live && (lane == 0 || cell != before))) > kNsCells<WRITE>) {
+            if(live) {
+                const uint32_t cnt = ns_alone<WRITE>(sp, a, first + lane, cell, cellStart, d0, d1, r2,
+                                                     WRITE ? idx + offsets[self] : nullptr);
+                if(!WRITE) counts[self] = cnt;
+            }
+            return;
+        }
+    }
     if(lane < P) {
         float* xy = reinterpret_cast<float*>(&sXY[warp][lane & ~1]);
         xy[lane & 1] = a.x;
@@ -451,7 +500,10 @@ __global__ void __launch_bounds__(kNsWarps * 32) k_ns_pairs(const float4* __rest
     if(!WRITE && live) counts[self] = cnt;
 }
 // Points per warp: 32 share their candidates' loads best; below kNsFew points, 8 give the GPU
-// four times the warps
+// four times the warps.  Whole call, ms with 8 (with 32) on 148 SMs: 20,000 points of 20 a cell 0.190
+// (0.243), of 0.5 0.157 (0.159); 80,000 0.249 (0.259), 0.202 (0.182); 160,000 0.337 (0.324), 0.231
+// (0.187); 400,000 0.612 (0.548), 0.340 (0.226).  The two are within 4 % from 80,000 to 160,000
+// points of 20 a cell.
 constexpr uint32_t kNsFew = 150000;
 template<bool WRITE>
 void launch_ns_pairs(const float4* sp, const uint32_t* scid, uint32_t n, const uint32_t* cellStart, int d0, int d1, float r2,

@@ -485,3 +485,25 @@ def test_neighbors_capacity_error(bnn):
     rc = L.bnn_neighbors(C.c_void_p(p.data_ptr()), len(pts), 0.05, C.c_void_p(goff.data_ptr()),
                          C.c_void_p(gidx.data_ptr()), 4, C.byref(tot), None)
     assert rc == 8 and tot.value > 4
+
+
+@pytest.mark.parametrize("n,r", [(150_000, 0.008), (150_003, 0.03), (400_000, 0.0165), (400_001, 0.021)])
+def test_neighbors_sparse_and_mixed_sets_equal(bnn, oracle_mod, n, r):
+    """Warps whose points lie in many cells walk them a thread per point: sets of less than a point a
+    cell, of about four and eight cells a warp, each with crowded cells beside sparse ones"""
+    rng = np.random.default_rng(n)
+    p = rng.random((n, 3)).astype(np.float32)
+    p[: n // 50] = np.float32(0.3) + np.float32(0.01) * rng.standard_normal((n // 50, 3)).astype(np.float32)
+    pos = _dev(p)
+    off = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    idx = torch.zeros(120_000_000, dtype=torch.int32, device="cuda")
+    tot = C.c_uint64()
+    bnn.capi.check(bnn.load().bnn_neighbors(pos.data_ptr(), n, r, off.data_ptr(), idx.data_ptr(), idx.numel(),
+                                            C.byref(tot), None), "bnn_neighbors")
+    want_off, want = oracle_mod.neighbors(p, np.float32(r))
+    off = off.cpu().numpy()
+    assert np.array_equal(off, want_off.astype(np.int64)) and off[-1] == tot.value
+    idx = idx[: tot.value].cpu().numpy()
+    rows = np.repeat(np.arange(n), np.diff(off))
+    a, b = np.lexsort((idx, rows)), np.lexsort((want, rows))
+    assert np.array_equal(idx[a], want[b])
