@@ -76,7 +76,8 @@ struct Shape {
     static constexpr int kThreads = kNH;
     // resident threads per SM: 1024 of 64 registers (256^3 0.81 ms against 0.84 at 768 of 80,
     // 80^3 0.068 against 0.079); the affine term and the batch's scene lookup want 80 (121 x 77 x
-    // 95 APIC 0.15 ms against 0.27 with the spills of 64)
+    // 95 APIC 0.15 ms against 0.27 with the spills of 64), and so does the SDF alone (64^3 0.045 ms
+    // against 0.054, 128^3 0.066 against 0.072, 256^3 0.166 against 0.179)
     static constexpr int min_blocks(int threads) { return threads / kThreads > 0 ? threads / kThreads : 1; }
     static constexpr size_t kSmemBytes = sizeof(float) * kPartials * kNH;
 };
@@ -483,7 +484,7 @@ __device__ __noinline__ void tile_body_exact(const TileArgs& a, const Tile tile)
     tile_body<P2G, SH, true, AFF>(a, tile);
 }
 template<bool P2G, class SH, bool AFF = false>
-__global__ void __launch_bounds__(SH::kThreads, SH::min_blocks(AFF ? 768 : 1024)) k_p2g_sdf_tile(const __grid_constant__ TileArgs a) {
+__global__ void __launch_bounds__(SH::kThreads, SH::min_blocks(P2G && !AFF ? 1024 : 768)) k_p2g_sdf_tile(const __grid_constant__ TileArgs a) {
     if((a.st->flags & BNN_FLAG_OUT_OF_GRID) != 0u) tile_body_exact<P2G, SH, AFF>(a, OwnTile<P2G>{});
     else tile_body<P2G, SH, false, AFF>(a, OwnTile<P2G>{});
 }
