@@ -392,7 +392,7 @@ struct PcgOutcome {
 // r-1 / r+1 (or none), its y neighbours lie within 65535 rows and on their side, its z
 // neighbours on theirs (rows of a grid in cell order, at most 65535 cells along x); the solve
 // then reads the packed 16-byte row records.  kRowsCompact: also y within kCompactDy rows and
-// z within kCompactDz (the chunk-resident solve's 8-byte records).
+// z within kCompactDz (the chunk-resident solve's 8-byte records), finite off-diagonal values.
 enum RowLayout { kRowsAny, kRowsGrid, kRowsCompact };
 constexpr int kCompactDy = 512, kCompactDz = (1 << 18) - 1;
 inline RowLayout row_layout(long long maxDy, long long maxDz) {

@@ -999,7 +999,9 @@ extern "C" int bnn_pcg_solve_7pt(uint32_t n, const float* diag, const int32_t* n
         bnn_set_error("bnn_pcg_solve_7pt: neighbour index outside [-1, n)");
         rc = BNN_ERR_INVALID_ARGUMENT;
     }
-    const RowLayout layout = info.notGrid ? kRowsAny : row_layout(info.maxDy, info.maxDz);
+    RowLayout layout = info.notGrid ? kRowsAny : row_layout(info.maxDy, info.maxDz);
+    // the chunk-resident solves multiply a missing neighbour's 0 by the off-diagonal value
+    if(layout == kRowsCompact && !std::isfinite(offdiag)) layout = kRowsGrid;
     // the system stores -dt as the off-diagonal; recover dt so the kernels form -(1*dt)
     const float dt = -offdiag;
     PcgOutcome po;

@@ -290,6 +290,17 @@ def test_pcg_groups_without_a_chunk_match_oracle(bnn, oracle_mod, chunks, mode, 
         assert np.array_equal(x, xo)
 
 
+@pytest.mark.parametrize("mode", ["fp32", "fp64", "refined"])
+def test_pcg_unbounded_offdiagonal_without_neighbours(bnn, mode):
+    """Rows without neighbours never meet the off-diagonal value, finite or not"""
+    n = 3000
+    nbr = np.full((n, 6), -1, np.int32)
+    diag = np.full(n, 0.5, np.float32)
+    rhs = np.random.default_rng(2).standard_normal(n).astype(np.float32)
+    x, st = bnn.pcg_solve_7pt(diag, nbr, -np.inf, rhs, 1e-6, 10, mode=mode)
+    assert st["success"] == 1 and np.array_equal(x, (2 * rhs).astype(np.float64))
+
+
 def test_barrier_wait_gives_up_and_device_stays_usable(bnn, oracle_mod):
     """A block waiting at a barrier that nothing completes (sized for two blocks, one
     launched) gives up after its limit and reports a timeout; the device then solves a
