@@ -24,6 +24,7 @@
 //   phase B: x += alpha s, r -= alpha q, max|r|, z = D^-1 r, partial z.r;
 //   grid barrier; every block reduces to the same rho, max|r| and beta.
 #include "bnn_internal.cuh"
+#include "coop_share.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -2031,15 +2032,13 @@ __global__ void k_pack_coef(int n, const float* __restrict__ coef, float4* __res
 // ---------------------------------------------------------------------------------
 
 // Process-wide record of the cooperative PCG kernels: SM count, resident blocks per SM of
-// each variant, and the share of the GPU held by solves in flight.  A share is counted
-// in units of 1/840 SM (840 is divisible by every resident-block count 1..8).
-constexpr int kShareUnits = 840;
+// each variant, and what the solves in flight hold of the GPU (coop_share.cuh).
 struct CoopState {
     std::mutex mu;
     std::condition_variable cv;
     int numSM = 0;
     int perSM[16] = {};
-    long long held = 0;
+    CoopLoad held;
 };
 static CoopState g_coop;
 
@@ -2054,19 +2053,20 @@ static int coop_sm_count(int& numSM) {
     return BNN_OK;
 }
 
-// Holds `units` of the GPU for the lifetime of the object; waits while other solves hold
-// so much that this grid would not fit beside them.
+// Holds a launch's part of the GPU for the lifetime of the object; waits while other solves
+// hold so much that it would not fit beside them.  A launch fits an empty GPU.
 struct CoopShare {
-    long long units;
-    CoopShare(long long u, long long capacity) : units(u < capacity ? u : capacity) {
+    const CoopLoad load;
+    CoopShare(const CoopLoad& l, int numSM) : load(l) {
         std::unique_lock<std::mutex> lk(g_coop.mu);
-        g_coop.cv.wait(lk, [&] { return g_coop.held + units <= capacity; });
-        g_coop.held += units;
+        g_coop.cv.wait(lk, [&] { return coop_fits(g_coop.held + load, numSM); });
+        g_coop.held = g_coop.held + load;
     }
+    CoopShare(const CoopShare&) = delete;
     ~CoopShare() {
         {
             std::lock_guard<std::mutex> lk(g_coop.mu);
-            g_coop.held -= units;
+            g_coop.held = g_coop.held - load;
         }
         g_coop.cv.notify_all();
     }
@@ -2266,7 +2266,7 @@ static int pcg_solve_chunk(PcgWork& w, int n, ChunkShape shape, int numSM, const
     BNN_CUDA_CHECK(cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kern.smem));
     BNN_CUDA_CHECK(cudaMemsetAsync(w.packets, 0, 2 * (size_t)w.nchCap * kPacketStride * sizeof(PcgPacket), s));
     const int most = numSM < kMostSM ? numSM : kMostSM, grid = a.nch < most ? a.nch : most;
-    CoopShare share((long long)grid * kShareUnits, (long long)numSM * kShareUnits);
+    CoopShare share(CoopLoad{grid, 0, 0}, numSM);
     if(w.ev[0]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[0], s));
     BNN_CUDA_CHECK(cudaLaunchCooperativeKernel(kern.fn, dim3(grid), dim3(shape.G * kLanes), args, kern.smem, s));
     bnn_note_launch();
@@ -2324,7 +2324,7 @@ static int pcg_solve_t(PcgWork& w, int n, ChunkShape shape, int numSM, const flo
     void* args[] = {twoReductions ? (void*)&a : (void*)&c};
     // grids of concurrent solves (several solver handles on several host threads) must
     // fit the GPU together, or blocks of one could wait for SMs held by another's barrier
-    CoopShare share(grid * (kShareUnits / perSMv), numSM * kShareUnits);
+    CoopShare share(CoopLoad{0, grid, grid * (kShareUnits / perSMv)}, numSM);
     if(w.ev[0]) BNN_CUDA_CHECK(cudaEventRecord(w.ev[0], s));
     BNN_CUDA_CHECK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kLanes), args, 0, s));
     bnn_note_launch();
@@ -2708,7 +2708,7 @@ int pcg_solve_batch_refined(BatchPcgCtx& ctx, BatchSolveItem* items, int count, 
             const BatchGroup* dgrp = (const BatchGroup*)(D + L.grp) + l.group0;
             void* args[] = {(void*)&dargs, (void*)&dgrp};
             // the share is held until the launch has ended
-            CoopShare share((long long)l.blocks * kShareUnits, (long long)numSM * kShareUnits);
+            CoopShare share(CoopLoad{l.blocks, 0, 0}, numSM);
             BNN_CUDA_CHECK(cudaEventRecord(ctx.ev[0], s));
             BNN_CUDA_CHECK(cudaLaunchCooperativeKernel(kern.fn, dim3(l.blocks), dim3(l.shape.G * kLanes), args, kern.smem, s));
             bnn_note_launch();

@@ -518,3 +518,40 @@ def test_neighbors_sparse_and_mixed_sets_equal(bnn, oracle_mod, n, r):
     rows = np.repeat(np.arange(n), np.diff(off))
     a, b = np.lexsort((idx, rows)), np.lexsort((want, rows))
     assert np.array_equal(idx[a], want[b])
+
+
+def test_pcg_kinds_in_flight_together(bnn):
+    """Solves of every kind from several threads at once (one cluster, chunks on one and two groups an
+    SM, a general row order, one reduction an iteration): each gives what it gives alone"""
+    import threading
+
+    jobs = []
+    for nx, ny, n, mode in [(31, 29, 9 * 2048, "fp32"), (64, 80, 60 * 2048 + 3, "fp64"), (64, 80, 160 * 2048, "fp32"),
+                            (513, 40, 300_000, "fp32"), (101, 90, 250 * 2048 + 1, "refined")]:
+        nbr, diag, rhs = _first_cells(nx, ny, n, seed=n)
+        jobs.append((diag, nbr, rhs, mode))
+    d, nb, b, _ = jobs[1]
+    perm = np.random.default_rng(4).permutation(len(d))
+    inv = np.empty(len(d), np.int64)
+    inv[perm] = np.arange(len(d))
+    jobs.append((d[perm], np.where(nb[perm] >= 0, inv[nb[perm]], -1).astype(np.int32), b[perm], "fp32"))
+
+    def solve(j, form):
+        mode = bnn.capi.PCG_MODE[j[3]] | form
+        return bnn.pcg_solve_7pt(j[0], j[1], -float(np.float32(0.004)), j[2], 1e-5, 40, mode=mode)[0]
+
+    forms = [(j, 0) for j in jobs] + [(jobs[0], SINGLE), (jobs[2], SINGLE)]
+    alone = [solve(*f) for f in forms]
+    got = [[] for _ in forms]
+
+    def run(i):
+        for _ in range(6):
+            got[i].append(solve(*forms[i]))
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(len(forms))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i, a in enumerate(alone):
+        assert len(got[i]) == 6 and all(np.array_equal(a, x) for x in got[i]), i
