@@ -743,8 +743,7 @@ __device__ __forceinline__ void packet_publish(const double* smd, const VT* smv,
 }
 
 // Tries until `got` is true in every lane of the warp; false when the bounded wait gave up
-template<class F> __device__ __forceinline__ bool warp_poll(F got) {
-    const BarrierLimit lim = solve_barrier_limit();
+template<class F> __device__ __forceinline__ bool warp_poll(F got, BarrierLimit lim) {
     unsigned spins = 0;
     unsigned long long t0 = 0;
     while(true) {
@@ -758,23 +757,24 @@ template<class F> __device__ __forceinline__ bool warp_poll(F got) {
 }
 // One packet per lane (where `on`), until all carry `parity`
 template<bool ACQUIRE>
-__device__ __forceinline__ bool packet_poll(const PcgPacket* slot, bool on, unsigned parity, PcgPacket& pk) {
+__device__ __forceinline__ bool packet_poll(const PcgPacket* slot, bool on, unsigned parity, PcgPacket& pk, BarrierLimit lim) {
     return warp_poll([&] {
         if(on) {
             pk = ACQUIRE ? ld_acquire_packet(slot) : ld_relaxed_packet(slot);
             on = (unsigned)(pk.max >> 63) != parity;
         }
         return !on;
-    });
+    }, lim);
 }
 
 // One warp: the packets of up to 32 chunks, their canonical sum and max (valid in lane 0);
 // false when the wait gave up
 template<class VT, bool MAX, bool ACQUIRE>
-__device__ __forceinline__ bool warp_packets(const PcgPacket* slots, int nch, unsigned parity, double& sum, VT& mx) {
+__device__ __forceinline__ bool warp_packets(const PcgPacket* slots, int nch, unsigned parity, double& sum, VT& mx,
+                                             BarrierLimit lim) {
     const int t = threadIdx.x & 31;
     PcgPacket pk;
-    const bool ok = packet_poll<ACQUIRE>(slots + (size_t)t * kPacketStride, t < nch, parity, pk);
+    const bool ok = packet_poll<ACQUIRE>(slots + (size_t)t * kPacketStride, t < nch, parity, pk, lim);
     double c = 0.0;
     VT m = VT(0);
     if(t < nch) {
@@ -812,13 +812,14 @@ template<class VT, int CH> struct WaitSmem {
 };
 template<class VT, bool MAX, bool ACQUIRE, int CH>
 __device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
-                                            WaitSmem<VT, CH>& W, double& sum, VT& mx) {
+                                            WaitSmem<VT, CH>& W, double& sum, VT& mx,
+                                            BarrierLimit lim = solve_barrier_limit()) {
     constexpr int X = MAX ? 1 : 0;
     const int t = threadIdx.x;
     // whole warps stay in the loop (the poll votes)
     for(int c = t; c < ((nch + 31) & ~31); c += (int)blockDim.x) {
         PcgPacket pk;
-        if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad[X] = 1; break; }
+        if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk, lim)) { W.bad[X] = 1; break; }
         if(c < nch) {
             W.part[c] = __longlong_as_double((long long)pk.sum);
             if(MAX) W.partMax[c] = max_of<VT>(pk.max);
@@ -856,7 +857,8 @@ __device__ __forceinline__ bool packet_wait(const PcgPacket* slots, int nch, uns
 __device__ __forceinline__ void front_sync(int threads) { asm volatile("bar.sync 15, %0;" : : "r"(threads) : "memory"); }
 template<class VT, bool MAX, bool PAIRS, int kPer, int CH>
 __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
-                                                  WaitSmem<VT, CH>& W, double& sum, VT& mx) {
+                                                  WaitSmem<VT, CH>& W, double& sum, VT& mx,
+                                                  BarrierLimit lim = solve_barrier_limit()) {
     constexpr int X = MAX ? 1 : 0;
     const int t = threadIdx.x, front = min((nch + 31) & ~31, kLanes);
     if(t < front) {
@@ -873,7 +875,7 @@ __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nc
                for(int i = 0; i < kPer; ++i)
                    if((late >> i & 1u) && (unsigned)(pk[i].max >> 63) == parity) late &= ~(1u << i);
                return late == 0u;
-           })) W.bad[X] = 1;
+           }, lim)) W.bad[X] = 1;
         double c = 0.0;
         VT m = VT(0);
 #pragma unroll
@@ -895,7 +897,7 @@ __device__ __forceinline__ bool packet_wait_split(const PcgPacket* slots, int nc
             if(!warp_poll([&] {
                    if(on) on = ld_acquire_ready(slots + (size_t)c * kPacketStride) != parity;
                    return !on;
-               })) { W.bad[X] = 1; break; }
+               }, lim)) { W.bad[X] = 1; break; }
         }
     }
     __syncthreads();
@@ -919,13 +921,14 @@ template<class VT> struct GroupWaitSmem {
 };
 template<class VT, bool MAX, bool ACQUIRE>
 __device__ __forceinline__ bool group_wait(const PcgPacket* slots, int nch, unsigned parity, unsigned* flags,
-                                           GroupWaitSmem<VT>& W, int grp, int t, double& sum, VT& mx) {
+                                           GroupWaitSmem<VT>& W, int grp, int t, double& sum, VT& mx,
+                                           BarrierLimit lim = solve_barrier_limit()) {
     if(nch > kWarpPackets) {
         double acc = 0.0;
         VT m = VT(0);
         for(int c = t; c < ((nch + 31) & ~31); c += kLanes) {
             PcgPacket pk;
-            if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk)) { W.bad = 1; break; }
+            if(!packet_poll<ACQUIRE>(slots + (size_t)c * kPacketStride, c < nch, parity, pk, lim)) { W.bad = 1; break; }
             if(c < nch) {
                 acc = acc + __longlong_as_double((long long)pk.sum);
                 if(MAX) { const VT o = max_of<VT>(pk.max); m = m > o ? m : o; }
@@ -943,7 +946,7 @@ __device__ __forceinline__ bool group_wait(const PcgPacket* slots, int nch, unsi
     } else if(t < 32) {
         double c;
         VT m;
-        if(!warp_packets<VT, MAX, ACQUIRE>(slots, nch, parity, c, m)) W.bad = 1;
+        if(!warp_packets<VT, MAX, ACQUIRE>(slots, nch, parity, c, m, lim)) W.bad = 1;
         if(t == 0) { W.sum = c; W.max = m; }
     }
     group_sync(grp);
@@ -2774,6 +2777,39 @@ __global__ void k_barrier_probe(GridSync* gs, unsigned* flags, BarrierLimit lim,
     }
 }
 
+// The packet waits in turn, each with a packet that nobody publishes: a block of two groups as one
+// (both forms), then the groups apart, the first of them with all its packets there.  passed[k] and
+// flags[k] of wait k; what is left to do after a wait is what a solve does: return.
+constexpr int kProbeWaits = 7, kProbeChunks = 40;
+__global__ void __launch_bounds__(2 * kLanes) k_wait_probe(PcgPacket* slots, unsigned* passed, unsigned* flags, BarrierLimit lim) {
+    __shared__ WaitSmem<float, 2> split;
+    __shared__ WaitSmem<float, 6> whole;
+    __shared__ GroupWaitSmem<float> group[2];
+    const int grp = (int)threadIdx.x / kLanes, t = (int)threadIdx.x % kLanes;
+    double sum;
+    float mx;
+    if(threadIdx.x == 0) {
+        for(int x = 0; x < 2; ++x) split.bad[x] = whole.bad[x] = 0;
+        // chunk 0 is there, the others are not
+        st_release_packet(slots, PcgPacket{(unsigned long long)__double_as_longlong(2.0), max_bits(3.0f) | 1ull << 63});
+        st_ready(slots, 1u);
+    }
+    if(t == 0) group[grp].bad = 0;
+    __syncthreads();
+    auto note = [&](int k, bool ok, bool writer) { if(writer) passed[k] = ok ? 1u : 0u; };
+    note(0, packet_wait_split<float, false, false, 1, 2>(slots, 2, 1u, flags + 0, split, sum, mx, lim), threadIdx.x == 0);
+    note(1, packet_wait_split<float, true, true, 1, 2>(slots, 2, 1u, flags + 1, split, sum, mx, lim), threadIdx.x == 0);
+    note(2, packet_wait<float, false, false, 6>(slots, 2, 1u, flags + 2, whole, sum, mx, lim), threadIdx.x == 0);
+    note(3, packet_wait<float, true, true, 6>(slots, kProbeChunks, 1u, flags + 3, whole, sum, mx, lim), threadIdx.x == 0);
+    if(grp == 0) {
+        const bool ok = group_wait<float, true, true>(slots, 1, 1u, flags + 4, group[0], 0, t, sum, mx, lim);
+        note(4, ok && sum == 2.0 && mx == 3.0f, t == 0);
+    } else {
+        note(5, group_wait<float, true, true>(slots, 2, 1u, flags + 5, group[1], 1, t, sum, mx, lim), t == 0);
+        note(6, group_wait<float, true, true>(slots, kProbeChunks, 1u, flags + 6, group[1], 1, t, sum, mx, lim), t == 0);
+    }
+}
+
 int pcg_barrier_probe(float limitSeconds, int* barrierStatus, float* elapsedMs) {
     GridSync* gs = nullptr;
     unsigned* flags = nullptr;
@@ -2783,11 +2819,15 @@ int pcg_barrier_probe(float limitSeconds, int* barrierStatus, float* elapsedMs) 
     chk(cudaMalloc(&gs, sizeof(GridSync)));
     chk(cudaMalloc(&flags, sizeof(unsigned)));
     chk(cudaMalloc(&out, 2 * sizeof(unsigned long long)));
+    constexpr size_t slotBytes = (size_t)kProbeChunks * kPacketStride * sizeof(PcgPacket), waitBytes = 2 * kProbeWaits * sizeof(unsigned);
+    PcgPacket* slots = nullptr;
+    chk(cudaMalloc(&slots, slotBytes + waitBytes));
     unsigned long long h[2] = {0, 0};
-    unsigned hf = 0;
+    unsigned hf = 0, hw[2 * kProbeWaits] = {};
     if(rc == BNN_OK) {
         chk(cudaMemset(gs, 0, sizeof(GridSync)));
         chk(cudaMemset(flags, 0, sizeof(unsigned)));
+        chk(cudaMemset(slots, 0, slotBytes + waitBytes));
     }
     if(rc == BNN_OK) {
         // 4096 polls, then limitSeconds of time; 2^26 polls at most whatever the clock says
@@ -2795,15 +2835,26 @@ int pcg_barrier_probe(float limitSeconds, int* barrierStatus, float* elapsedMs) 
         k_barrier_probe<<<1, kLanes>>>(gs, flags, lim, out);
         bnn_note_launch();
         chk(cudaGetLastError());
+        unsigned* waits = (unsigned*)((char*)slots + slotBytes);
+        // six waits in turn: at most 50 ms each
+        const BarrierLimit each = {std::min(lim.ns, 50000000ull), lim.minSpins, lim.maxSpins};
+        k_wait_probe<<<1, 2 * kLanes>>>(slots, waits, waits + kProbeWaits, each);
+        bnn_note_launch();
+        chk(cudaGetLastError());
         chk(cudaDeviceSynchronize());
+        chk(cudaMemcpy(hw, waits, waitBytes, cudaMemcpyDeviceToHost));
         chk(cudaMemcpy(h, out, sizeof(h), cudaMemcpyDeviceToHost));
         chk(cudaMemcpy(&hf, flags, sizeof(hf), cudaMemcpyDeviceToHost));
     }
     cudaFree(gs);
     cudaFree(flags);
     cudaFree(out);
+    cudaFree(slots);
     if(rc != BNN_OK) return rc;
-    *barrierStatus = (h[0] == 1ull && (hf & BNN_FLAG_TIMEOUT)) ? BNN_ERR_TIMEOUT : BNN_OK;
+    bool gaveUp = h[0] == 1ull && (hf & BNN_FLAG_TIMEOUT);
+    for(int k = 0; k < kProbeWaits; ++k)  // wait 4 has its packet
+        gaveUp = gaveUp && hw[k] == (k == 4 ? 1u : 0u) && hw[kProbeWaits + k] == (k == 4 ? 0u : (unsigned)BNN_FLAG_TIMEOUT);
+    *barrierStatus = gaveUp ? BNN_ERR_TIMEOUT : BNN_OK;
     *elapsedMs = (float)((double)h[1] * 1e-6);
     return BNN_OK;
 }

@@ -294,12 +294,13 @@ typedef struct bnn_pcg_stats {
 int bnn_pcg_solve_7pt(uint32_t n, const float* diag, const int32_t* nbr, float offdiag, const float* rhs, float tol,
                       uint32_t max_iter, int32_t mode, float inner_tol, double* x_out, bnn_pcg_stats* stats);
 
-/* Self-test of the bounded wait of the PCG grid barrier (no counterpart in the reference,
+/* Self-test of the bounded waits of the PCG kernels (no counterpart in the reference,
  * whose solver has no device-side waits).  One block waits at a barrier sized for two
  * blocks, so the wait can only end by giving up: after 4096 polls and limit_seconds
- * (0 < limit_seconds <= 10) of wall time, the limit a solve uses being 1 s.
- * *barrier_status receives BNN_ERR_TIMEOUT when the wait gave up as designed, *elapsed_ms
- * how long the block polled.  The device stays usable afterwards.  The probe runs on the
+ * (0 < limit_seconds <= 10) of wall time, the limit a solve uses being 1 s.  Another waits
+ * for partial sums that nobody publishes, at most 50 ms each time.
+ * *barrier_status receives BNN_ERR_TIMEOUT when all of them gave up as designed,
+ * *elapsed_ms how long the first block polled.  The device stays usable afterwards.  The probe runs on the
  * default stream and synchronizes the device, so it is not for use while solves run. */
 int bnn_pcg_barrier_probe(float limit_seconds, int32_t* barrier_status, float* elapsed_ms);
 

@@ -316,6 +316,21 @@ def test_barrier_wait_gives_up_and_device_stays_usable(bnn, oracle_mod):
     assert np.array_equal(x.astype(np.float32), xo.astype(np.float32))
 
 
+@pytest.mark.parametrize("limit", [0.02, 0.2])
+def test_packet_waits_give_up_and_device_stays_usable(bnn, oracle_mod, limit):
+    """The probe's status also covers the waits of the chunk-resident solves, block-wide and per group:
+    each gives up on a packet that nobody publishes, says so in its own flag and returns, a group that
+    has its packets passes beside it; a solve on their kernel then works"""
+    from banana_b200 import capi
+    status, ms = bnn.pcg_barrier_probe(limit)
+    assert status == capi.STATUS_CODE["TIMEOUT"] and ms >= 1000 * limit
+    nbr, diag, rhs = _first_cells(64, 80, 40 * 2048 + 7, seed=8)
+    off = -float(np.float32(0.004))
+    x, st = bnn.pcg_solve_7pt(diag, nbr, off, rhs, 1e-6, 20)
+    xo, so = oracle_mod.pcg(*_csr_of(nbr, diag, off), rhs, 1e-6, 20, 0)
+    assert st["iterations"] == so["iterations"] and np.array_equal(x.astype(np.float32), xo.astype(np.float32))
+
+
 def test_pcg_7pt_rejects_bad_neighbour_index(bnn):
     nbr, _, diag, off, rhs, _ = _box_system(8, 8, 8)
     bad = nbr.copy()
