@@ -107,6 +107,28 @@ def test_dynamic_boundary_fp64_and_refined(bnn, oracle_mod, mode):
     _run_frames(g, o, 1, lambda f: [_moving_sphere(f)])
 
 
+@pytest.mark.parametrize("n,block,mode,chunks", [
+    (80, (0.4, 0.6, 0.4), 0, (17, 148)), (80, (0.4, 0.6, 0.4), 1, (17, 148)), (80, (0.4, 0.6, 0.4), 2, (17, 148)),
+    (100, (0.8, 0.6, 0.8), 0, (149, 296)), (100, (0.8, 0.6, 0.8), 1, (149, 296)), (124, (0.8, 0.65, 0.8), 0, (297, 592))])
+def test_dynamic_boundary_every_weighted_solve(bnn, oracle_mod, n, block, mode, chunks):
+    """Weighted systems of more than 16 chunks of 2048 rows, which the scenes above do not reach: on 148
+    SMs the chunk-resident solve takes up to 2 chunks an SM in FP32 (also inside the refined solve) and 1
+    in FP64, k_pcg_persistent with its packed off-diagonals what is beyond"""
+    cfg = scenes.dam_break_params(n, pcg_mode=mode, cg_relative_tolerance=5e-2, refine_tolerance=1e-3)
+    pos, vel = scenes.dam_break(n, block=block, ppc=2)
+    g = bnn.FlipSolver(cfg)
+    o = oracle_mod.Oracle(cfg)
+    for s in (g, o):
+        s.set_particles(pos, vel)
+        s.set_boundaries([_rotating_box(1)])
+    sg, so = g.step(), o.step()
+    assert chunks[0] <= -(-sg["n_active"] // 2048) <= chunks[1]
+    assert sg["n_active"] == so["n_active"] and sg["pcg_iterations"] == so["pcg_iterations"] and sg["pcg_success"] == 1
+    w = g.grid("weight_u")
+    assert ((w > 0) & (w < 1)).any()
+    _check(g, o, f"{n} mode {mode}")
+
+
 def test_clearing_boundaries_restores_the_box(bnn):
     cfg = scenes.dam_break_params(20)
     pos, vel = scenes.dam_break(20)
