@@ -36,7 +36,7 @@ EXPORTS = [
     "bnn_flip_device_bytes", "bnn_scene_bytes_estimate", "bnn_flip_set_grid",
     "bnn_batch_create", "bnn_batch_destroy", "bnn_batch_add_scene", "bnn_batch_remove_scene", "bnn_batch_step",
     "bnn_batch_scene_info", "bnn_batch_get_scene", "bnn_batch_memory",
-    "bnn_aniso_default_params", "bnn_anisotropic_kernels", "bnn_flip_anisotropic_kernels",
+    "bnn_aniso_default_params", "bnn_anisotropic_kernels", "bnn_flip_anisotropic_kernels", "bnn_aniso_sqrt_probe",
     "bnn_flip_set_boundaries", "bnn_tile_shapes", "bnn_set_tile_shape", "bnn_tile_tuning",
 ]
 
@@ -195,6 +195,7 @@ def load() -> C.CDLL:
     L.bnn_tile_tuning.argtypes = [C.c_char_p, C.c_size_t, C.POINTER(C.c_size_t)]
     L.bnn_aniso_default_params.argtypes = [C.c_float, C.POINTER(AnisoParams)]
     L.bnn_anisotropic_kernels.argtypes = [vp, C.c_uint32, C.POINTER(AnisoParams), vp, vp, C.POINTER(AnisoStats), vp]
+    L.bnn_aniso_sqrt_probe.argtypes = [u64p, u64p]
     L.bnn_flip_anisotropic_kernels.argtypes = [vp, C.POINTER(AnisoParams), fp, fp, C.POINTER(AnisoStats)]
     L.bnn_launch_count.argtypes = []
     L.bnn_launch_count.restype = C.c_uint64

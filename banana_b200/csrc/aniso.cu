@@ -80,7 +80,8 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // on the residual, g + (x - g g) y / 2 with the residual fused (P. Markstein, IBM J. Res. Dev.
 // 34, 1990); y / 2 is y with its exponent lowered.  Equal to sqrtf for every float in [2^-100,
 // 2^100] (all of them tried).  x is raised to 2^-100 first, which keeps 0 out of the
-// reciprocal: below 2^-75 kernel_w2 gives 1 either way while r >= 2^-24.
+// reciprocal: below 2^-75 kernel_w2 gives 1 either way while r >= 2^-24.  bnn_aniso_sqrt_probe tries
+// them again.
 __device__ __forceinline__ F2 sqrt2(F2 v, const Packed& k) {
     const float x0 = fmaxf(lo2(v), 0x1p-100f), x1 = fmaxf(hi2(v), 0x1p-100f);
     const float y0 = rsqrt_approx(x0), y1 = rsqrt_approx(x1);
@@ -425,6 +426,23 @@ AnisoArgs make_args(const bnn_aniso_params& prm, float dx) {
     return a;
 }
 
+// sqrt2 against sqrtf for the floats with bits [first, first + count), each in both halves beside
+// another value of the range
+__global__ void __launch_bounds__(256) k_sqrt_probe(unsigned first, unsigned count, Packed k, unsigned long long* bad) {
+    unsigned wrong = 0;
+    for(size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
+        const float a = __uint_as_float(first + (unsigned)i), b = __uint_as_float(first + (count - 1u - (unsigned)i));
+        const F2 r = sqrt2(pack2(a, b), k);
+        wrong += (__float_as_uint(lo2(r)) != __float_as_uint(sqrtf(a)) ? 1u : 0u) +
+                 (__float_as_uint(hi2(r)) != __float_as_uint(sqrtf(b)) ? 1u : 0u);
+    }
+    if(wrong) atomicAdd(bad, (unsigned long long)wrong);
+}
+Packed packed_constants() {
+    auto both = [](unsigned bits) { return (F2)bits << 32 | bits; };
+    return Packed{both(0x80000000u), both(0xbf800000u), both(0x3f800000u)};
+}
+
 } // namespace
 
 bnn_aniso_params aniso_defaults(float particleRadius) {
@@ -469,8 +487,7 @@ cudaError_t launch_aniso(int n, const PairPoints& q, const uint32_t* ids, const 
                          const bnn_aniso_params& prm, float* outC, float* outM, unsigned* counters, cudaStream_t s) {
     if(n <= 0) return cudaSuccess;
     const AnisoArgs a = make_args(prm, g.dx);
-    auto both = [](unsigned bits) { return (F2)bits << 32 | bits; };
-    const Packed k{both(0x80000000u), both(0xbf800000u), both(0x3f800000u)};
+    const Packed k = packed_constants();
     const float r = prm.kernel_ratio * prm.particle_radius;
     const bool fast = r >= 0x1p-24f && r <= 0x1p24f;
     const unsigned blocks = (unsigned)((n + 127) / 128);
@@ -505,6 +522,23 @@ struct DevMem {
 extern "C" int bnn_aniso_default_params(float particle_radius, bnn_aniso_params* out) {
     if(!out) return BNN_ERR_INVALID_ARGUMENT;
     *out = aniso_defaults(particle_radius);
+    return BNN_OK;
+}
+
+extern "C" int bnn_aniso_sqrt_probe(uint64_t* tested, uint64_t* mismatches) {
+    if(!tested || !mismatches) return BNN_ERR_INVALID_ARGUMENT;
+    constexpr unsigned first = (127u - 100u) << 23, last = (127u + 100u) << 23;  // 2^-100 .. 2^100
+    DevMem bad;
+    BNN_CUDA_CHECK(bad.alloc(sizeof(unsigned long long), cudaStreamPerThread));
+    BNN_CUDA_CHECK(cudaMemsetAsync(bad.p, 0, sizeof(unsigned long long), cudaStreamPerThread));
+    k_sqrt_probe<<<2048, 256, 0, cudaStreamPerThread>>>(first, last - first + 1u, packed_constants(), bad.as<unsigned long long>());
+    bnn_note_launch();
+    BNN_CUDA_CHECK(cudaGetLastError());
+    unsigned long long h = 0;
+    BNN_CUDA_CHECK(cudaMemcpyAsync(&h, bad.p, sizeof(h), cudaMemcpyDeviceToHost, cudaStreamPerThread));
+    BNN_CUDA_CHECK(cudaStreamSynchronize(cudaStreamPerThread));
+    *tested = last - first + 1u;
+    *mismatches = h;
     return BNN_OK;
 }
 

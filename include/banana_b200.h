@@ -376,6 +376,10 @@ int bnn_anisotropic_kernels(const float* pos_dev, uint32_t n, const bnn_aniso_pa
 int bnn_flip_anisotropic_kernels(bnn_flip* h, const bnn_aniso_params* params, float* centers, float* matrices,
                                  bnn_aniso_stats* stats);
 
+/* Self-test: the pass's packed square roots against correctly rounded ones, for every float of
+ * [2^-100, 2^100] (some 20 ms; no counterpart in the reference). */
+int bnn_aniso_sqrt_probe(uint64_t* tested, uint64_t* mismatches);
+
 const char* bnn_version(void);
 const char* bnn_last_error(void);
 uint64_t bnn_launch_count(void);

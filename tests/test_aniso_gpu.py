@@ -6,6 +6,8 @@ Both sum every particle's neighbours in the canonical order of the same cell gri
 only correctly rounded operations, so centres and kernel matrices must agree bit for bit.
 At the 128^3 dam-break size the checks are the size-independent properties of the output.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -190,3 +192,10 @@ def test_candidates_that_are_no_neighbours_leave_the_sums_alone(bnn, oracle_mod)
     oc = _oracle_for(oracle_mod, p, st, 0.01, threshold=2)[0]
     _eq(cen.cpu().numpy(), oc, "centres")
     assert np.array_equal(np.signbit(cen.cpu().numpy()), np.signbit(oc))
+
+
+def test_packed_square_roots_are_correctly_rounded(bnn):
+    """Every float of the range in which the weights' square roots are packed"""
+    tested, bad = C.c_uint64(), C.c_uint64()
+    capi.check(capi.load().bnn_aniso_sqrt_probe(C.byref(tested), C.byref(bad)), "bnn_aniso_sqrt_probe")
+    assert tested.value == 200 * 2 ** 23 + 1 and bad.value == 0
