@@ -618,7 +618,7 @@ extern "C" int bnn_cell_sort(const float* pos_dev, uint32_t n, const float bmin[
     BNN_CUDA_CHECK(cudaMemsetAsync(D, 0, zeroed, s));
     if(n) {
         uint32_t* scratch = (uint32_t*)(D + aScratch);
-        const unsigned ntiles = (n + kRTile - 1) / kRTile;
+        const unsigned ntiles = (unsigned)(((size_t)n + kRTile - 1) / kRTile);
         { k_grid_cell_ids<<<ntiles, kRT, 0, s>>>(pos_dev, n, bmin[0], bmin[1], bmin[2], cell_size, ncells[0], ncells[1], ncells[2],
                                                  cell_id_dev, oor, scratch, ntiles, count); bnn_note_launch(); }
         // the ids' bits are known from the cell count: no pass over the keys to find them
