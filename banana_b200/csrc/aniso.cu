@@ -225,8 +225,8 @@ __device__ __forceinline__ void kernel_matrix(float a[3][3], float axisRatio, fl
 }
 
 // Bound by the FP32 pipe (a packed operation takes it for two cycles, so packing saves issue
-// slots, not pipe cycles: 22 and 39 a candidate in the two passes) and, below a few hundred
-// thousand points, by the serial chain of a particle's candidates.  ms against one candidate at a
+// slots, not pipe cycles; 1.58 M points: pipe busy 67 % of the cycles, ALU 50 %, issue 76 %, 25.5 of 32
+// lanes, stalls math_pipe_throttle 3.6 and not_selected 3.3) and, below a few hundred thousand points, by the serial chain of a particle's candidates.  ms against one candidate at a
 // time with sqrtf and a 16-byte record: 5,000 points 0.467 (0.947), 50,000 0.766 (1.28), 200,003
 // 2.51 (2.75), 600,001 7.18 (7.63), 1,000,000 11.86 (12.45), 3,000,000 36.3 (38.1); the pass over a
 // 256^3 scene with its layout 155.7 (163.5).  Coordinates in three planes, three loads a pair:

@@ -56,9 +56,9 @@ METRIC = "particle-steps/s at 256^3 FLIP (1e-6 rel residual)"
 UNIT = "particle-steps/s"
 WORKLOAD = "flip_dam_break_256"
 # DRAM bytes (read + write) per PCG iteration at 1.59M rows, from ncu captures of the standalone
-# solve at that row count (`--workload pcg`: 156.5 and 835.7 MB over 300 iterations); a launch's
+# solve at that row count (`--workload pcg`: 304.2 and 835.7 MB over 300 iterations); a launch's
 # traffic is this times its iterations
-PCG_TRAFFIC_PER_ITER = {"k_pcg_chunk": 156.5e6 / 300, "k_pcg_persistent": 835.7e6 / 300}
+PCG_TRAFFIC_PER_ITER = {"k_pcg_chunk": 304.2e6 / 300, "k_pcg_persistent": 835.7e6 / 300}
 
 
 PCG_MODE = {"fp32": 0, "fp64": 1, "refined": 2}
@@ -424,7 +424,9 @@ def run_ours(args, ws, rank, local):
                          "traffic": PCG_TRAFFIC_PER_ITER[pcg_kernel] * iters / args.steps
                          if pcg_kernel in PCG_TRAFFIC_PER_ITER else None,
                          "traffic_note": "ncu DRAM bytes per iteration of the same kernel at the same row count "
-                                         "(standalone capture) x iterations per launch; the solve stays on the chip"},
+                                         "(standalone capture) x iterations per launch.  k_pcg_chunk and k_pcg_cluster "
+                                         "keep the rows on the chip: there frac compares with a rate they do not "
+                                         "use, and exchange latency and instruction issue bound them"},
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": int(launches),
             "clocks": clk,
             "detail": {"tile_tuning": capi.tile_tuning(),
