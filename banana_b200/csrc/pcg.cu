@@ -657,8 +657,12 @@ struct alignas(16) PcgPacket {
 };
 constexpr int kPacketStride = 8;  // packets apart
 __device__ __forceinline__ unsigned long long max_bits(float m) { return __float_as_uint(m) & 0x7fffffffu; }
+// The mask is written out: in C it is the absolute value to the compiler, whose result for a NaN may
+// have either sign (abs.f64), and the sign's place is the parity's
 __device__ __forceinline__ unsigned long long max_bits(double m) {
-    return (unsigned long long)__double_as_longlong(m) & 0x7fffffffffffffffull;
+    unsigned long long b = (unsigned long long)__double_as_longlong(m);
+    asm("and.b64 %0, %0, 0x7fffffffffffffff;" : "+l"(b));
+    return b;
 }
 template<class VT> __device__ __forceinline__ VT max_of(unsigned long long b) {
     if constexpr(sizeof(VT) == 4) return __uint_as_float((unsigned)b);

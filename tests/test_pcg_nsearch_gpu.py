@@ -316,6 +316,23 @@ def test_barrier_wait_gives_up_and_device_stays_usable(bnn, oracle_mod):
     assert np.array_equal(x.astype(np.float32), xo.astype(np.float32))
 
 
+@pytest.mark.parametrize("chunks", [3, 17, 60, 200, 420])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_pcg_residual_that_is_not_a_number(bnn, chunks, bad):
+    """A right-hand side with an infinity or a NaN makes every later sum and maximum NaN: on every kernel
+    the waits still see each exchange (the call returns instead of timing out), and FP64 takes the
+    iterations and the outcome of FP32; the refined solve returns too"""
+    n = chunks * 2048 - 11
+    nbr, diag, rhs = _first_cells(64, 80, n, seed=chunks)
+    rhs[n // 2] = bad
+    out = {}
+    for mode in ("fp32", "fp64", "refined"):
+        x, st = bnn.pcg_solve_7pt(diag, nbr, -float(np.float32(0.004)), rhs, 1e-6, 7, mode=mode)
+        out[mode] = (st["iterations"], st["success"], int(np.isnan(x).sum()))
+    assert out["fp32"] == out["fp64"]
+    assert out["fp32"][2] == (n if bad == np.inf else 0)
+
+
 @pytest.mark.parametrize("limit", [0.02, 0.2])
 def test_packet_waits_give_up_and_device_stays_usable(bnn, oracle_mod, limit):
     """The probe's status also covers the waits of the chunk-resident solves, block-wide and per group:
